@@ -295,6 +295,27 @@ bool stage_layout(size_t symm_bytes, uint32_t W, uint32_t M, uint32_t K, StageLa
 // ---------------------------------------------------------------------------------------------
 // launches
 // ---------------------------------------------------------------------------------------------
+// Every kernel of this library that waits for its predecessor with grid_dep_wait() before it touches memory is
+// launched with programmatic stream serialisation: its launch latency and set-up pass while the predecessor drains.
+// Measured (B200, back to back on one stream, a 3 us kernel): 6.2 us per launch without the attribute (a plain
+// dependency is picked up in steps of 2.05 us), 3.6 us with it.
+template <typename... KArgs, typename... Args>
+cudaError_t launch_after(void (*kern)(KArgs...), dim3 grid, uint32_t threads, size_t smem, cudaStream_t st, Args&&... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    g_launches++;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
 int quant_grid(const RankCtx& rc)
 {
     int per_sm = 0;
@@ -343,6 +364,16 @@ void choose_segments(uint32_t M, uint32_t K, int num_sms, QuantPushParams& p, ui
     }
     p.seg_cols = seg_cols;
     p.segs_per_chunk = (K + seg_cols - 1) / seg_cols;
+}
+
+// bf16 [M, K] -> codes and scales in one place, nobody waiting on flags: the flat quantiser.
+int launch_quant_flat(cudaStream_t st, const void* in, uint32_t M, uint32_t K, uint8_t* codes, uint8_t* scales)
+{
+    const uint64_t halves = (uint64_t)M * (K / 16);
+    const dim3 grid((unsigned)((halves + kQuantThreads - 1) / kQuantThreads));
+    CUDA_TRY(launch_after(g.a_dtype == 1 ? mx_quant_flat_kernel<true> : mx_quant_flat_kernel<false>, grid, kQuantThreads, 0, st,
+                          static_cast<const uint8_t*>(in), codes, scales, halves, g.tiny_block_rule != 0 ? 1u : 0u));
+    return 0;
 }
 
 // max_grid (0 = no limit): an upper bound on the CTAs, for a push that has to leave in item order.
@@ -929,8 +960,12 @@ int allgather_matmul(void* stream, const void* a, const void* a_scale, bool preq
     // transfer like everybody's: the tiles then follow the send groups, slice by slice over all ranks.
     p.own_first = g.tile_order >= 0 ? (uint32_t)g.tile_order : ((fuse_mode == 6 || fuse_mode == 7) ? 0u : 1u);
     if (produce && consume && fuse_mode == 3) {
-        q.publish = 0;
-        rcode = launch_quant_push(rc, st, q, prequant, true);
+        if (prequant) {
+            q.publish = 0;
+            rcode = launch_quant_push(rc, st, q, prequant, true);
+        } else {
+            rcode = launch_quant_flat(st, a, M, K, q.dst_codes[0], q.dst_scales[0]);
+        }
         if (rcode != 0) return rcode;
         p.flags = nullptr;  // stream order is the only dependency
         return launch_gemm(rc, st, a_stage, b, p, false, true);
@@ -1334,20 +1369,7 @@ int catccos_b200_mx_quant(void* stream, const void* in_bf16, uint32_t rows, uint
     }
     int rcode = ensure_init();
     if (rcode != 0) return rcode;
-    RankCtx& rc = cur();
-    QuantPushParams q = {};
-    q.in = in_bf16;
-    q.M = rows;
-    q.K = k;
-    q.world = 1;
-    q.num_dst = 1;
-    q.dst_codes[0] = (uint8_t*)codes;
-    q.dst_scales[0] = (uint8_t*)scales;
-    choose_segments(rows, k, rc.num_sms, q);
-    q.publish = 0;
-    q.status = rc.status;
-    q.timeout_ns = g.timeout_ns;
-    return launch_quant_push(rc, (cudaStream_t)stream, q, false, true);
+    return launch_quant_flat((cudaStream_t)stream, in_bf16, rows, k, (uint8_t*)codes, (uint8_t*)scales);
 }
 
 int catccos_b200_mx_quant_fp4(void* stream, const void* in_bf16, uint32_t rows, uint32_t k, void* packed, void* scales)
@@ -1360,16 +1382,10 @@ int catccos_b200_mx_quant_fp4(void* stream, const void* in_bf16, uint32_t rows, 
     }
     int rcode = ensure_init();
     if (rcode != 0) return rcode;
-    RankCtx& rc = cur();
-    const uint32_t rows_per_cta = kQuantThreads / 32;
-    uint32_t grid = (rows + rows_per_cta - 1) / rows_per_cta;
-    const uint32_t cap = (uint32_t)rc.num_sms * 6u;
-    if (grid > cap) grid = cap;
-    mx_quant_e2m1_kernel<<<grid, kQuantThreads, 0, (cudaStream_t)stream>>>(
-        static_cast<const uint16_t*>(in_bf16), rows, k, static_cast<uint8_t*>(packed), static_cast<uint8_t*>(scales),
-        g.tiny_block_rule != 0 ? 1u : 0u);
-    g_launches++;
-    CUDA_TRY(cudaGetLastError());
+    const uint64_t halves = (uint64_t)rows * (k / 16);
+    CUDA_TRY(launch_after(mx_quant_e2m1_kernel, dim3((unsigned)((halves + kQuantThreads - 1) / kQuantThreads)), kQuantThreads, 0,
+                          (cudaStream_t)stream, static_cast<const uint8_t*>(in_bf16), halves, static_cast<uint8_t*>(packed),
+                          static_cast<uint8_t*>(scales), g.tiny_block_rule != 0 ? 1u : 0u));
     return 0;
 }
 
@@ -1410,9 +1426,7 @@ int catccos_b200_mx_quant_allgather(void* stream, const void* in_bf16, void* out
     uint8_t* oc = (uint8_t*)out_codes;
     uint8_t* os = (uint8_t*)out_scales;
     if (W == 1) {
-        q.dst_codes[0] = oc;
-        q.dst_scales[0] = os;
-        return launch_quant_push(rc, (cudaStream_t)stream, q, false, true);
+        return launch_quant_flat((cudaStream_t)stream, in_bf16, M, K, oc, os);
     }
     SymmAlloc* sa = find_symm(symm);
     if (sa == nullptr) {
@@ -1761,15 +1775,11 @@ int catccos_b200_mx_quant_scatter_packed(void* stream, const void* in_bf16, cons
     }
     int rcode = ensure_init();
     if (rcode != 0) return rcode;
-    RankCtx& rc = cur();
-    const uint32_t per_cta = kQuantThreads / 32;
-    uint32_t grid = (tokens + per_cta - 1) / per_cta;
-    grid = std::min(grid, (uint32_t)rc.num_sms * 6u);
-    mx_quant_scatter_packed_kernel<<<grid, kQuantThreads, 0, (cudaStream_t)stream>>>(
-        static_cast<const uint16_t*>(in_bf16), expanded_row_idx, static_cast<uint8_t*>(packed_out), tokens, n, top_k,
-        g.tiny_block_rule != 0 ? 1u : 0u);
-    g_launches++;
-    CUDA_TRY(cudaGetLastError());
+    const uint64_t warps = (uint64_t)tokens * ((n + kQuantColsPerWarpStep - 1) / kQuantColsPerWarpStep);
+    const unsigned grid = (unsigned)((warps + kQuantThreads / 32 - 1) / (kQuantThreads / 32));
+    CUDA_TRY(launch_after(mx_quant_scatter_packed_kernel, dim3(grid), kQuantThreads, 0, (cudaStream_t)stream,
+                          static_cast<const uint16_t*>(in_bf16), expanded_row_idx, static_cast<uint8_t*>(packed_out), tokens, n,
+                          top_k, g.tiny_block_rule != 0 ? 1u : 0u));
     return 0;
 }
 

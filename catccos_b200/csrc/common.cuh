@@ -48,6 +48,14 @@ __device__ __forceinline__ void st_global_v8(void* p, const uint32_t (&v)[8])
                  : "memory");
 }
 
+// 32-byte streaming load (one full sector per lane); the address must be 32-byte aligned
+__device__ __forceinline__ void ld_global_stream_v8(const void* p, uint4& a, uint4& b)
+{
+    asm volatile("ld.global.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+                 : "l"(p));
+}
+
 __device__ __forceinline__ uint64_t globaltimer_ns()
 {
     uint64_t t;

@@ -133,6 +133,18 @@ __device__ __forceinline__ uint4 quant16(uint4 v0, uint4 v1, bool device_tiny, b
     return o;
 }
 
+// 16 bf16 values (half a 32-block) of one lane.  The caller's pointer is 16-byte aligned at least; where it is 32-byte
+// aligned (the same answer for every lane) one full-sector load takes both halves.
+__device__ __forceinline__ void load_half_block(const void* p, uint4& v0, uint4& v1)
+{
+    if (((uintptr_t)p & 31u) == 0u) {
+        ld_global_stream_v8(p, v0, v1);
+    } else {
+        v0 = __ldcs(static_cast<const uint4*>(p));
+        v1 = __ldcs(static_cast<const uint4*>(p) + 1);
+    }
+}
+
 // Barrier among the 256 threads of one quantise group (barrier 0 when the group is the whole CTA).
 __device__ __forceinline__ void quant_group_sync(uint32_t bar_id)
 {
@@ -310,6 +322,35 @@ __device__ __forceinline__ void quant_push_producer(const QuantPushParams& p, ui
         }
         if (p.publish) {
             publish_item(p, chunk * p.segs_per_chunk + seg, tid, bar_id);
+        }
+    }
+}
+
+// The quantiser for one destination and no flags (a single rank, the plain quantise calls).  Rows hold whole 32-blocks
+// and all three arrays are dense, so the matrix is a flat run of blocks whatever its shape: a lane takes 16 consecutive
+// values (32 bytes in, 16 bytes of codes out, two lanes share a scale), a warp 1 KiB, and every block of the grid is one
+// such step per warp and ends.  HBM-bound: the loads of a few hundred resident warps are all in flight at once, ragged
+// shapes split evenly, nothing loops.  Measured (B200, back to back): bf16 [4096, 7168] 24.4 us with the item loop of
+// quant_push_producer, 14.4 us here (6.2 TB/s); [1024, 7168] 8.4 -> 3.5 us.  More steps per warp, or a grid of one wave
+// that loops, measure 1-5 % slower.
+template <bool kE5m2>
+__global__ void __launch_bounds__(kQuantThreads) mx_quant_flat_kernel(const uint8_t* __restrict__ in, uint8_t* __restrict__ codes,
+                                                                      uint8_t* __restrict__ scales, uint64_t halves,
+                                                                      uint32_t device_tiny)
+{
+    grid_dep_wait();
+    grid_dep_launch();
+    const uint64_t i = (uint64_t)blockIdx.x * kQuantThreads + threadIdx.x;
+    uint4 v0 = make_uint4(0, 0, 0, 0), v1 = v0;
+    if (i < halves) {
+        load_half_block(in + i * 32, v0, v1);
+    }
+    uint32_t byte;
+    const uint4 o = quant16(v0, v1, device_tiny != 0u, kE5m2, byte);
+    if (i < halves) {
+        *reinterpret_cast<uint4*>(codes + i * 16) = o;
+        if ((i & 1u) == 0u) {
+            scales[i >> 1] = (uint8_t)byte;
         }
     }
 }
@@ -717,7 +758,6 @@ __global__ void __launch_bounds__(kQuantThreads, 2) mx_quant_push_ordered_kernel
 // [N E4M3 codes | ceil(N / 32) E8M0 scales, padded to an even count | zero padding to a multiple of 32 bytes];
 // expanded_row_idx[token * top_k + route] names the destination row, a negative entry drops the route.
 // It replaces CommBlockMxQuant::QuantScatterPacked (include/catccos/comm/block/comm_block_mx_quant.hpp:312-368).
-// One warp per token; a lane quantises 16 consecutive values per 512-column step (two lanes share a 32-block).
 __host__ __device__ __forceinline__ uint32_t packed_row_bytes(uint32_t n)
 {
     const uint32_t scale_bytes = ((n + 31u) / 32u + 1u) / 2u * 2u;
@@ -725,46 +765,55 @@ __host__ __device__ __forceinline__ uint32_t packed_row_bytes(uint32_t n)
 }
 
 __global__ void __launch_bounds__(kQuantThreads) mx_quant_scatter_packed_kernel(const uint16_t* __restrict__ in,
+// One warp per (token, 512-column step): a lane quantises 16 consecutive values (two lanes share a 32-block) and stores
+// its 16 bytes of codes once per route; the warp of a token's last step also writes the padding.  Bound by the writes
+// (top_k packed rows per token): every warp has all its loads, then all its stores in flight, and a token's steps run
+// side by side instead of one after the other.
                                                                                const int32_t* __restrict__ expanded_row_idx,
                                                                                uint8_t* __restrict__ packed_out, uint32_t tokens,
                                                                                uint32_t n, uint32_t top_k, uint32_t device_tiny)
 {
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    grid_dep_wait();
+    grid_dep_launch();
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t steps = (n + kQuantColsPerWarpStep - 1) / kQuantColsPerWarpStep;
+    const uint64_t w = (uint64_t)blockIdx.x * (kQuantThreads / 32) + (threadIdx.x >> 5);
+    const uint32_t token = (uint32_t)(w / steps), step = (uint32_t)(w % steps);
+    if (token >= tokens) {
+        return;
+    }
     const uint32_t row_bytes = packed_row_bytes(n);
-    const uint32_t scale_raw = n / 32u;
-    for (uint32_t token = blockIdx.x * (kQuantThreads / 32) + warp; token < tokens; token += gridDim.x * (kQuantThreads / 32)) {
-        for (uint32_t cb = 0; cb < n; cb += kQuantColsPerWarpStep) {
-            const uint32_t col = cb + lane * 16;
-            const bool ok = col < n;
-            uint4 v0 = make_uint4(0, 0, 0, 0), v1 = v0;
-            if (ok) {
-                const uint4* src = reinterpret_cast<const uint4*>(in + (size_t)token * n + col);
-                v0 = __ldcs(src);
-                v1 = __ldcs(src + 1);
+    const uint32_t col = step * kQuantColsPerWarpStep + lane * 16;
+    const bool ok = col < n;
+    uint4 v0 = make_uint4(0, 0, 0, 0), v1 = v0;
+    if (ok) {
+        load_half_block(in + (size_t)token * n + col, v0, v1);
+    }
+    const int32_t* routes = expanded_row_idx + (size_t)token * top_k;
+    const bool last = step == steps - 1;
+    uint32_t byte = 0;
+    uint4 o = v0;
+    for (uint32_t r0 = 0; r0 < top_k; r0 += 32) {
+        const int32_t mine = r0 + lane < top_k ? __ldg(routes + r0 + lane) : -1;
+        if (r0 == 0) {
+            o = quant16(v0, v1, device_tiny != 0u, false, byte);
+        }
+        const uint32_t here = min(32u, top_k - r0);
+        for (uint32_t r = 0; r < here; ++r) {
+            const int32_t dst = __shfl_sync(0xFFFFFFFFu, mine, r);
+            if (dst < 0) {
+                continue;
             }
-            uint32_t byte;
-            const uint4 o = quant16(v0, v1, device_tiny != 0u, false, byte);
-            for (uint32_t route = 0; route < top_k; ++route) {
-                const int32_t dst = expanded_row_idx[(size_t)token * top_k + route];
-                if (dst < 0 || !ok) {
-                    continue;
-                }
-                uint8_t* row = packed_out + (size_t)dst * row_bytes;
+            uint8_t* row = packed_out + (size_t)dst * row_bytes;
+            if (ok) {
                 *reinterpret_cast<uint4*>(row + col) = o;
                 if ((lane & 1u) == 0u) {
                     row[n + col / 32u] = (uint8_t)byte;
                 }
             }
-        }
-        // the tail of the row: the scale count rounded up to even, then zeros up to the 32-byte boundary
-        for (uint32_t route = 0; route < top_k; ++route) {
-            const int32_t dst = expanded_row_idx[(size_t)token * top_k + route];
-            if (dst < 0) {
-                continue;
-            }
-            uint8_t* row = packed_out + (size_t)dst * row_bytes;
-            for (uint32_t b = n + scale_raw + lane; b < row_bytes; b += 32) {
-                row[b] = 0;
+            // the tail of the row: the scale count rounded up to even, then zeros up to the 32-byte boundary
+            if (last && n + n / 32u + lane < row_bytes) {
+                row[n + n / 32u + lane] = 0;
             }
         }
     }
@@ -818,49 +867,42 @@ __global__ void __launch_bounds__(256) fp4_transpose_kernel(const uint8_t* __res
 // bf16 [rows, K] -> FP4 E2M1 codes, two per byte (low nibble = even column), + one E8M0 scale per 32 elements.
 // The FP4 branch of the reference's quantiser (include/catccos/comm/block/comm_block_mx_quant.hpp:525-568, emax
 // constant block_epilogue_dynamic_mx_quant.hpp:53): the same exponent rule with emax 2, saturation at +-6,
-// round to nearest even (cvt.rn.satfinite.e2m1x2.f32).  A warp takes a row; a lane quantises 16 consecutive
-// values per 512-column step (two lanes share a 32-block) and stores 8 bytes of codes.
-__global__ void __launch_bounds__(kQuantThreads) mx_quant_e2m1_kernel(const uint16_t* __restrict__ in, uint32_t rows, uint32_t K,
+// round to nearest even (cvt.rn.satfinite.e2m1x2.f32).  Flat, as mx_quant_flat_kernel: a lane quantises 16 consecutive
+// values (two lanes share a 32-block) and stores 8 bytes of codes.  [1024, 7168]: 12.8 us with a warp walking each row.
+__global__ void __launch_bounds__(kQuantThreads) mx_quant_e2m1_kernel(const uint8_t* __restrict__ in, uint64_t halves,
                                                                       uint8_t* __restrict__ packed,
                                                                       uint8_t* __restrict__ scales, uint32_t device_tiny)
 {
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t sf_cols = K / 32;
-    for (uint32_t row = blockIdx.x * (kQuantThreads / 32) + warp; row < rows; row += gridDim.x * (kQuantThreads / 32)) {
-        for (uint32_t cb = 0; cb < K; cb += kQuantColsPerWarpStep) {
-            const uint32_t col = cb + lane * 16;
-            const bool ok = col < K;
-            uint4 v0 = make_uint4(0, 0, 0, 0), v1 = v0;
-            if (ok) {
-                const uint4* src = reinterpret_cast<const uint4*>(in + (size_t)row * K + col);
-                v0 = __ldcs(src);
-                v1 = __ldcs(src + 1);
-            }
-            uint32_t amax = max(absmax_bits8(v0), absmax_bits8(v1));
-            amax = max(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
-            uint32_t byte;
-            float mul;
-            bool nonfinite;
-            block_scale(amax, device_tiny != 0u, 2u, byte, mul, nonfinite);
-            const uint32_t w[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-            uint32_t o[2] = {0u, 0u};
+    grid_dep_wait();
+    grid_dep_launch();
+    const uint64_t i = (uint64_t)blockIdx.x * kQuantThreads + threadIdx.x;
+    uint4 v0 = make_uint4(0, 0, 0, 0), v1 = v0;
+    if (i < halves) {
+        load_half_block(in + i * 32, v0, v1);
+    }
+    uint32_t amax = max(absmax_bits8(v0), absmax_bits8(v1));
+    amax = max(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
+    uint32_t byte;
+    float mul;
+    bool nonfinite;
+    block_scale(amax, device_tiny != 0u, 2u, byte, mul, nonfinite);
+    const uint32_t w[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+    uint32_t o[2] = {0u, 0u};
 #pragma unroll
-            for (uint32_t i = 0; i < 8; ++i) {
-                const float lo = __uint_as_float(w[i] << 16) * mul, hi = __uint_as_float(w[i] & 0xFFFF0000u) * mul;
-                const uint32_t b = __nv_cvt_float2_to_fp4x2(make_float2(lo, hi), __NV_E2M1, cudaRoundNearest);
-                o[i >> 2] |= (b & 0xFFu) << (8u * (i & 3u));
-            }
-            if (nonfinite) {
-                o[0] = o[1] = 0x77777777u;  // E2M1 has no NaN: the largest magnitude stands in
-            } else if (mul == 0.0f && device_tiny == 0u) {
-                o[0] = o[1] = 0u;  // the golden writes +0 for every element of a block below 1e-12
-            }
-            if (ok) {
-                *reinterpret_cast<uint2*>(packed + (size_t)row * (K / 2) + col / 2) = make_uint2(o[0], o[1]);
-                if ((lane & 1u) == 0u) {
-                    scales[(size_t)row * sf_cols + col / 32] = (uint8_t)byte;
-                }
-            }
+    for (uint32_t k = 0; k < 8; ++k) {
+        const float lo = __uint_as_float(w[k] << 16) * mul, hi = __uint_as_float(w[k] & 0xFFFF0000u) * mul;
+        const uint32_t b = __nv_cvt_float2_to_fp4x2(make_float2(lo, hi), __NV_E2M1, cudaRoundNearest);
+        o[k >> 2] |= (b & 0xFFu) << (8u * (k & 3u));
+    }
+    if (nonfinite) {
+        o[0] = o[1] = 0x77777777u;  // E2M1 has no NaN: the largest magnitude stands in
+    } else if (mul == 0.0f && device_tiny == 0u) {
+        o[0] = o[1] = 0u;  // the golden writes +0 for every element of a block below 1e-12
+    }
+    if (i < halves) {
+        *reinterpret_cast<uint2*>(packed + i * 8) = make_uint2(o[0], o[1]);
+        if ((i & 1u) == 0u) {
+            scales[i >> 1] = (uint8_t)byte;
         }
     }
 }
