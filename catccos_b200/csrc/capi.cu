@@ -396,13 +396,8 @@ int launch_quant_push(RankCtx& rc, cudaStream_t st, QuantPushParams& p, bool pre
     p.mode = quant_mode(prequant);
     p.e5m2 = g.a_dtype == 1 ? 1u : 0u;
     p.sys_scope = local_only ? quant_sys_scope(1) : quant_sys_scope(p.world);  // no peer sees these stores directly
-    if (grid <= 2 * rc.num_sms && items > (uint32_t)grid) {
-        mx_quant_push_kernel<true><<<grid, kQuantThreads, 0, st>>>(p);
-    } else {
-        mx_quant_push_kernel<false><<<grid, kQuantThreads, 0, st>>>(p);
-    }
-    g_launches++;
-    CUDA_TRY(cudaGetLastError());
+    const bool prefetch = grid <= 2 * rc.num_sms && items > (uint32_t)grid;
+    CUDA_TRY(launch_after(prefetch ? mx_quant_push_kernel<true> : mx_quant_push_kernel<false>, dim3(grid), kQuantThreads, 0, st, p));
     return 0;
 }
 
@@ -522,7 +517,9 @@ int launch_gemm_inst(int grid, cudaStream_t st, const CUtensorMap& ta, const CUt
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
-    cfg.numAttrs = overlap_predecessor ? 1 : 0;
+    // Without flags the kernel waits for its predecessor itself; with flags it does not, and only the quantise kernel
+    // that feeds it may still be running.
+    cfg.numAttrs = (overlap_predecessor || (!FUSED && p.flags == nullptr)) ? 1 : 0;
     CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, ta, tb, p));
     g_launches++;
     CUDA_TRY(cudaGetLastError());
@@ -574,7 +571,9 @@ int launch_gemm_pair_inst(int max_pairs_hint, uint32_t tiles, cudaStream_t st, c
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
-    cfg.numAttrs = overlap_predecessor ? 1 : 0;
+    // Without flags the kernel waits for its predecessor itself; with flags it does not, and only the quantise kernel
+    // that feeds it may still be running.
+    cfg.numAttrs = (overlap_predecessor || (!FUSED && p.flags == nullptr)) ? 1 : 0;
     CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, ta, tb, p));
     g_launches++;
     CUDA_TRY(cudaGetLastError());
@@ -688,9 +687,7 @@ int launch_gemm(RankCtx& rc, cudaStream_t st, const void* a, const void* b, Gemm
             rc.fp4_bt_bytes = need;
         }
         dim3 tg((p.N + kFp4TransN - 1) / kFp4TransN, (p.K + kFp4TransK - 1) / kFp4TransK);
-        fp4_transpose_kernel<<<tg, 256, 0, st>>>(static_cast<const uint8_t*>(b), rc.fp4_bt, p.K, p.N);
-        g_launches++;
-        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(launch_after(fp4_transpose_kernel, tg, 256, 0, st, static_cast<const uint8_t*>(b), rc.fp4_bt, p.K, p.N));
         b = rc.fp4_bt;
         p.b_kmajor = 1;
         overlap_predecessor = false;
@@ -768,6 +765,8 @@ int launch_gemm(RankCtx& rc, cudaStream_t st, const void* a, const void* b, Gemm
 // Sets n flag words to the epoch (the rows they stand for were put in place by stream-ordered copies).
 __global__ void fill_flags_kernel(uint32_t* flags, uint32_t n, uint32_t epoch)
 {
+    grid_dep_wait();
+    grid_dep_launch();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         flags[i] = epoch;
     }
@@ -778,6 +777,8 @@ __global__ void fill_flags_kernel(uint32_t* flags, uint32_t n, uint32_t epoch)
 __global__ void wait_flags_kernel(const uint32_t* flags, uint32_t flag_stride, uint32_t world, uint32_t rank, uint32_t chunks,
                                   uint32_t segs, uint32_t epoch, uint64_t timeout_ns, StatusBlock* status)
 {
+    grid_dep_wait();
+    grid_dep_launch();
     for (uint32_t i = threadIdx.x; i + 1 < world; i += blockDim.x) {
         const uint32_t src = (rank + 1 + i) % world;
         const uint32_t last_chunk = chunks - 1u;
@@ -1482,10 +1483,8 @@ int catccos_b200_mx_quant_allgather(void* stream, const void* in_bf16, void* out
     }
     if (consume) {
         if (direct) {
-            wait_flags_kernel<<<1, 128, 0, st>>>(my_flags, kMaxFlags, W, rank, chunks, q.segs_per_chunk, epoch, g.timeout_ns,
-                                                 rc.status);
-            g_launches++;
-            CUDA_TRY(cudaGetLastError());
+            CUDA_TRY(launch_after(wait_flags_kernel, dim3(1), 128, 0, st, my_flags, kMaxFlags, W, rank, chunks, q.segs_per_chunk,
+                                  epoch, g.timeout_ns, rc.status));
         } else {
             QuantPushParams qc = q;
             qc.consume = 1;
@@ -1582,9 +1581,7 @@ int catccos_b200_fp4_mx_allgather_matmul(void* stream, const void* a, const void
         // and the copy engines forward all three to the peers (one flag word per 16-row chunk, one K segment)
         CUDA_TRY(cudaMemcpyAsync(dc[rank], a, (size_t)M * row_bytes, cudaMemcpyDeviceToDevice, st));
         CUDA_TRY(cudaMemcpyAsync(ds[rank], a_scale, (size_t)M * sf, cudaMemcpyDeviceToDevice, st));
-        fill_flags_kernel<<<(chunks + 255) / 256, 256, 0, st>>>(df[rank], chunks, epoch);
-        g_launches++;
-        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(launch_after(fill_flags_kernel, dim3((chunks + 255) / 256), 256, 0, st, df[rank], chunks, epoch));
         rcode = copy_engine_push(rc, st, W, rank, M, K, 1, kCopySliceRows, dc[rank], ds[rank], df[rank], dc, ds, df, row_bytes);
         if (rcode != 0) return rcode;
     }
@@ -1747,14 +1744,12 @@ int catccos_b200_mxfp8_matmul_reduce_scatter(void* stream, const void* a, const 
         const float* parts = reinterpret_cast<const float*>(sa->base[rank] + stage_off);
         const uint32_t* flags = reinterpret_cast<const uint32_t*>(sa->base[rank] + kFlagsOff);
         if (g.c_dtype == 1) {
-            mx_reduce_scatter_kernel<__half><<<grid, 256, 0, st>>>(parts, flags, kMaxFlags, W, rows, N, bn, epoch, (__half*)d,
-                                                                   g.timeout_ns, rc.status);
+            CUDA_TRY(launch_after(mx_reduce_scatter_kernel<__half>, dim3(grid), 256, 0, st, parts, flags, kMaxFlags, W, rows, N, bn,
+                                  epoch, (__half*)d, g.timeout_ns, rc.status));
         } else {
-            mx_reduce_scatter_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(parts, flags, kMaxFlags, W, rows, N, bn, epoch,
-                                                                          (__nv_bfloat16*)d, g.timeout_ns, rc.status);
+            CUDA_TRY(launch_after(mx_reduce_scatter_kernel<__nv_bfloat16>, dim3(grid), 256, 0, st, parts, flags, kMaxFlags, W, rows,
+                                  N, bn, epoch, (__nv_bfloat16*)d, g.timeout_ns, rc.status));
         }
-        g_launches++;
-        CUDA_TRY(cudaGetLastError());
     }
     return 0;
 }

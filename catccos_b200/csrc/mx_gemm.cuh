@@ -397,6 +397,8 @@ __global__ void __launch_bounds__(256) mx_reduce_scatter_kernel(const float* __r
                                                                 uint32_t bn, uint32_t epoch, OutT* __restrict__ d,
                                                                 uint64_t timeout_ns, StatusBlock* status)
 {
+    grid_dep_wait();
+    grid_dep_launch();
     const uint32_t n_tiles = (N + bn - 1) / bn;
     const uint32_t units = (rs_rows / 32u) * n_tiles;
     for (uint32_t unit = blockIdx.x; unit < units; unit += gridDim.x) {
@@ -438,6 +440,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     constexpr uint32_t kStages = S::kStages;
     static_assert(BLOCK_N == 128 || BLOCK_N == 256, "tile widths wired up: 128 and 256");
 
+    grid_dep_launch();  // what follows on the stream may be set up meanwhile; it waits for this kernel before it reads
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::kOffBar);
@@ -957,6 +960,9 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         CATCCOS_TR_STAMP(p.trace, kTrCtaEnd);
     }
     drain_after_abort(p.status);
+    if (p.flags != nullptr) {
+        grid_dep_wait();  // a gated launch ends after the quantise kernel it overlaps: the successor waits for this one only
+    }
     if (warp == 5) {
         tcgen05_fence_after();
         tmem_dealloc(tmem_base, kTmemCols);

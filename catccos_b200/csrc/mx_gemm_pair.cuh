@@ -71,6 +71,7 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     using S = PairSmem;
     constexpr uint32_t kStages = S::kStages;
 
+    grid_dep_launch();  // as in mx_gemm_kernel
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::kOffBar);
@@ -446,6 +447,9 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     __syncthreads();
     drain_after_abort(p.status);  // both CTAs stay while loads that report to the other's barriers may be in flight
     cluster_sync_all();  // nobody leaves while the other CTA may still arrive on its barriers
+    if (p.flags != nullptr) {
+        grid_dep_wait();
+    }
     if (threadIdx.x == 0) {
         CATCCOS_TR_STAMP(p.trace, kTrCtaEnd);
     }

@@ -524,6 +524,7 @@ __device__ __forceinline__ void push_worker(const PushParams& p, uint32_t lane, 
 template <bool kPrefetch>
 __global__ void __launch_bounds__(kQuantThreads) mx_quant_push_kernel(QuantPushParams p)
 {
+    grid_dep_wait();    // `in` may be the predecessor's output, and the outputs may be what it still reads
     grid_dep_launch();  // a GEMM launched behind this kernel may set itself up while the quantiser drains
 #ifdef CATCCOS_TRACE
     if (p.trace != nullptr && threadIdx.x == 0) {
@@ -764,11 +765,11 @@ __host__ __device__ __forceinline__ uint32_t packed_row_bytes(uint32_t n)
     return (n + scale_bytes + 31u) / 32u * 32u;
 }
 
-__global__ void __launch_bounds__(kQuantThreads) mx_quant_scatter_packed_kernel(const uint16_t* __restrict__ in,
 // One warp per (token, 512-column step): a lane quantises 16 consecutive values (two lanes share a 32-block) and stores
 // its 16 bytes of codes once per route; the warp of a token's last step also writes the padding.  Bound by the writes
 // (top_k packed rows per token): every warp has all its loads, then all its stores in flight, and a token's steps run
 // side by side instead of one after the other.
+__global__ void __launch_bounds__(kQuantThreads) mx_quant_scatter_packed_kernel(const uint16_t* __restrict__ in,
                                                                                const int32_t* __restrict__ expanded_row_idx,
                                                                                uint8_t* __restrict__ packed_out, uint32_t tokens,
                                                                                uint32_t n, uint32_t top_k, uint32_t device_tiny)
@@ -829,6 +830,8 @@ constexpr uint32_t kFp4TransK = 64, kFp4TransN = 256;
 __global__ void __launch_bounds__(256) fp4_transpose_kernel(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, uint32_t K,
                                                             uint32_t N)
 {
+    grid_dep_wait();
+    grid_dep_launch();
     constexpr uint32_t kStride = kFp4TransN + 4;  // bytes per tile row: rows stay 4-byte aligned, columns shift banks
     __shared__ __align__(4) uint8_t tile[kFp4TransK * kStride];
     const uint32_t k0 = blockIdx.y * kFp4TransK, n0 = blockIdx.x * kFp4TransN;
