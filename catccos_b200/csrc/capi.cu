@@ -961,6 +961,13 @@ int allgather_matmul(void* stream, const void* a, const void* a_scale, bool preq
     // transfer like everybody's: the tiles then follow the send groups, slice by slice over all ranks.
     p.own_first = g.tile_order >= 0 ? (uint32_t)g.tile_order : ((fuse_mode == 6 || fuse_mode == 7) ? 0u : 1u);
     if (produce && consume && fuse_mode == 3) {
+        if (prequant && ((uintptr_t)a & 15u) == 0u && ((uintptr_t)a_scale & 3u) == 0u) {
+            // nothing to quantise and nobody to send to: the GEMM reads the caller's operands in place (operands that are
+            // aligned for neither TMA nor word loads go through the stage)
+            p.a_scales = (const uint8_t*)a_scale;
+            p.flags = nullptr;
+            return launch_gemm(rc, st, a, b, p);
+        }
         if (prequant) {
             q.publish = 0;
             rcode = launch_quant_push(rc, st, q, prequant, true);
