@@ -1,8 +1,9 @@
 """ctypes binding of libcatccos_b200.so (the C ABI declared in include/catccos_b200.h).
 
 This is the host harness the tests and the benchmark drive the library through; torch is used only
-for device memory and streams.  There is no fallback: when the shared library is missing or a call
-fails, an exception is raised.
+for device memory and streams.  The operator calls on tensors go through the extension module
+_torch_calls (csrc/torch_calls.cpp), bound to the functions of the library loaded here.  There is no
+fallback: when the shared library or the extension is missing or a call fails, an exception is raised.
 """
 from __future__ import annotations
 
@@ -113,15 +114,29 @@ def load() -> ctypes.CDLL:
     return L
 
 
+_calls = None
+
+
+def _load_calls():
+    """The extension module with the operator calls, bound to the loaded library."""
+    global _calls
+    L = load()
+    import torch  # noqa: F401  (the extension links against it)
+
+    try:
+        from . import _torch_calls
+    except ImportError as e:
+        raise FileNotFoundError(
+            f"{os.path.join(_HERE, '_torch_calls.so')} cannot be loaded ({e}): build it with `python -m catccos_b200.build`.") from e
+    for name in EXPORTS:
+        _torch_calls.bind(name, ctypes.cast(getattr(L, name), ctypes.c_void_p).value)
+    _calls = _torch_calls
+    return _calls
+
+
 def _check(fn: str, code: int) -> None:
     if code != 0:
         raise CatccosError(fn, code)
-
-
-def _stream() -> int:
-    import torch
-
-    return torch.cuda.current_stream().cuda_stream
 
 
 def make_tiling(m: int, k: int, n: int, world: int) -> Tiling:
@@ -225,55 +240,37 @@ def trace_read():
 # ---------------------------------------------------------------------------------------------
 def mx_quant(x_bf16):
     """bf16 [rows, K] -> (codes uint8 [rows, K], scales uint8 [rows, K/32]); no communication."""
-    import torch
-
-    rows, k = x_bf16.shape
-    assert x_bf16.is_cuda and x_bf16.is_contiguous() and x_bf16.element_size() == 2
-    codes = torch.empty((rows, k), dtype=torch.uint8, device=x_bf16.device)
-    scales = torch.empty((rows, k // 32), dtype=torch.uint8, device=x_bf16.device)
-    _check("catccos_b200_mx_quant",
-           load().catccos_b200_mx_quant(_stream(), x_bf16.data_ptr(), rows, k, codes.data_ptr(), scales.data_ptr()))
+    code, codes, scales = (_calls or _load_calls()).mx_quant(x_bf16)
+    if code:
+        raise CatccosError("catccos_b200_mx_quant", code)
     return codes, scales
 
 
 def mx_quant_fp4(x_bf16):
     """bf16 [rows, K] -> (packed E2M1 codes uint8 [rows, K/2], scales uint8 [rows, K/32]); no communication."""
-    import torch
-
-    rows, k = x_bf16.shape
-    assert x_bf16.is_cuda and x_bf16.is_contiguous() and x_bf16.element_size() == 2
-    packed = torch.empty((rows, k // 2), dtype=torch.uint8, device=x_bf16.device)
-    scales = torch.empty((rows, k // 32), dtype=torch.uint8, device=x_bf16.device)
-    _check("catccos_b200_mx_quant_fp4",
-           load().catccos_b200_mx_quant_fp4(_stream(), x_bf16.data_ptr(), rows, k, packed.data_ptr(), scales.data_ptr()))
+    code, packed, scales = (_calls or _load_calls()).mx_quant_fp4(x_bf16)
+    if code:
+        raise CatccosError("catccos_b200_mx_quant_fp4", code)
     return packed, scales
 
 
 def mx_gemm(a_codes, a_scales, b, b_scales, out=None, out_dtype=None):
     """c [M, N] = dequant(a)[M, K] x dequant(b [K, N])."""
-    import torch
-
-    m, k = a_codes.shape
-    n = b_scales.shape[1]
     if out is None:
-        out = torch.empty((m, n), dtype=out_dtype or torch.bfloat16, device=a_codes.device)
-    _check("catccos_b200_mx_gemm",
-           load().catccos_b200_mx_gemm(_stream(), a_codes.data_ptr(), a_scales.data_ptr(), b.data_ptr(),
-                                       b_scales.data_ptr(), out.data_ptr(), m, n, k))
+        import torch
+
+        out = torch.empty((a_codes.shape[0], b_scales.shape[1]), dtype=out_dtype or torch.bfloat16, device=a_codes.device)
+    code = (_calls or _load_calls()).mx_gemm(a_codes, a_scales, b, b_scales, out)
+    if code:
+        raise CatccosError("catccos_b200_mx_gemm", code)
     return out
 
 
 def mx_gemm_quant_out(a_codes, a_scales, b, b_scales):
     """The GEMM whose epilogue MX-quantises its output: (codes uint8 [M, N], scales uint8 [M, N/32])."""
-    import torch
-
-    m, k = a_codes.shape
-    n = b_scales.shape[1]
-    codes = torch.empty((m, n), dtype=torch.uint8, device=a_codes.device)
-    scales = torch.empty((m, n // 32), dtype=torch.uint8, device=a_codes.device)
-    _check("catccos_b200_mx_gemm_quant_out",
-           load().catccos_b200_mx_gemm_quant_out(_stream(), a_codes.data_ptr(), a_scales.data_ptr(), b.data_ptr(),
-                                                 b_scales.data_ptr(), codes.data_ptr(), scales.data_ptr(), m, n, k))
+    code, codes, scales = (_calls or _load_calls()).mx_gemm_quant_out(a_codes, a_scales, b, b_scales)
+    if code:
+        raise CatccosError("catccos_b200_mx_gemm_quant_out", code)
     return codes, scales
 
 
@@ -283,64 +280,45 @@ def packed_row_bytes(n: int) -> int:
 
 def mx_quant_scatter_packed(x_bf16, expanded_row_idx, packed_out, top_k: int) -> None:
     """Quantises every token (row of x) once and writes its packed row to each of its top_k destination rows."""
-    tokens, n = x_bf16.shape
-    _check("catccos_b200_mx_quant_scatter_packed",
-           load().catccos_b200_mx_quant_scatter_packed(_stream(), x_bf16.data_ptr(), expanded_row_idx.data_ptr(),
-                                                       packed_out.data_ptr(), tokens, n, top_k))
+    code = (_calls or _load_calls()).mx_quant_scatter_packed(x_bf16, expanded_row_idx, packed_out, top_k)
+    if code:
+        raise CatccosError("catccos_b200_mx_quant_scatter_packed", code)
 
 
 def mxfp8_matmul_reduce_scatter(a_codes, a_scales, b, b_scales, d, symm: int, world: int) -> None:
     """d [m / world, n] = this rank's row chunk of the sum over ranks of dequant(a) x dequant(b); m is the whole M."""
-    m, k = a_codes.shape
-    n = b_scales.shape[1]
-    t = make_tiling(m, k, n, world)
-    _check("catccos_b200_mxfp8_matmul_reduce_scatter",
-           load().catccos_b200_mxfp8_matmul_reduce_scatter(_stream(), a_codes.data_ptr(), b.data_ptr(), a_scales.data_ptr(),
-                                                           b_scales.data_ptr(), d.data_ptr(), symm, ctypes.byref(t), 0))
+    code = (_calls or _load_calls()).mxfp8_matmul_reduce_scatter(a_codes, a_scales, b, b_scales, d, symm, world)
+    if code:
+        raise CatccosError("catccos_b200_mxfp8_matmul_reduce_scatter", code)
 
 
 def mx_quant_matmul_static(a_bf16, b, b_scales, c) -> None:
     """The allocation-free single-GPU fused call (scratch is the library's built-in device array)."""
-    m, k = a_bf16.shape
-    n = b_scales.shape[1]
-    _check("catccos_b200_mx_quant_matmul_static",
-           load().catccos_b200_mx_quant_matmul_static(_stream(), a_bf16.data_ptr(), b.data_ptr(), b_scales.data_ptr(),
-                                                      c.data_ptr(), m, n, k))
+    code = (_calls or _load_calls()).mx_quant_matmul_static(a_bf16, b, b_scales, c)
+    if code:
+        raise CatccosError("catccos_b200_mx_quant_matmul_static", code)
 
 
 def mx_quant_allgather(x_bf16, out_codes, out_scales, symm: int, world: int) -> None:
-    m, k = x_bf16.shape
-    t = make_tiling(m, 1, k, world)  # the quantised axis is `n` for this operator
-    _check("catccos_b200_mx_quant_allgather",
-           load().catccos_b200_mx_quant_allgather(_stream(), x_bf16.data_ptr(), out_codes.data_ptr(),
-                                                  out_scales.data_ptr(), symm, ctypes.byref(t), 0))
+    code = (_calls or _load_calls()).mx_quant_allgather(x_bf16, out_codes, out_scales, symm, world)
+    if code:
+        raise CatccosError("catccos_b200_mx_quant_allgather", code)
 
 
 def mx_quant_allgather_matmul(a_bf16, b, b_scales, c, symm: int, world: int) -> None:
-    m, k = a_bf16.shape
-    n = b_scales.shape[1]
-    t = make_tiling(m, k, n, world)
-    _check("catccos_b200_mx_quant_allgather_matmul",
-           load().catccos_b200_mx_quant_allgather_matmul(_stream(), a_bf16.data_ptr(), b.data_ptr(),
-                                                         b_scales.data_ptr(), c.data_ptr(), symm, ctypes.byref(t), 0))
+    code = (_calls or _load_calls()).mx_quant_allgather_matmul(a_bf16, b, b_scales, c, symm, world)
+    if code:
+        raise CatccosError("catccos_b200_mx_quant_allgather_matmul", code)
 
 
 def fp8_mx_allgather_matmul(a_codes, a_scales, b, b_scales, c, symm: int, world: int) -> None:
-    m, k = a_codes.shape
-    n = b_scales.shape[1]
-    t = make_tiling(m, k, n, world)
-    _check("catccos_b200_fp8_mx_allgather_matmul",
-           load().catccos_b200_fp8_mx_allgather_matmul(_stream(), a_codes.data_ptr(), b.data_ptr(),
-                                                       a_scales.data_ptr(), b_scales.data_ptr(), c.data_ptr(), symm,
-                                                       ctypes.byref(t), 0))
+    code = (_calls or _load_calls()).fp8_mx_allgather_matmul(a_codes, a_scales, b, b_scales, c, symm, world)
+    if code:
+        raise CatccosError("catccos_b200_fp8_mx_allgather_matmul", code)
 
 
 def fp4_mx_allgather_matmul(a_packed, a_scales, b_packed, b_scales, c, symm: int, world: int) -> None:
     """The FP4 operator: a packed E2M1 [m, k/2], b packed E2M1 [k, n/2]."""
-    m, k = a_packed.shape[0], a_packed.shape[1] * 2
-    n = b_scales.shape[1]
-    t = make_tiling(m, k, n, world)
-    _check("catccos_b200_fp4_mx_allgather_matmul",
-           load().catccos_b200_fp4_mx_allgather_matmul(_stream(), a_packed.data_ptr(), b_packed.data_ptr(),
-                                                       a_scales.data_ptr(), b_scales.data_ptr(), c.data_ptr(), symm,
-                                                       ctypes.byref(t), 0))
+    code = (_calls or _load_calls()).fp4_mx_allgather_matmul(a_packed, a_scales, b_packed, b_scales, c, symm, world)
+    if code:
+        raise CatccosError("catccos_b200_fp4_mx_allgather_matmul", code)
