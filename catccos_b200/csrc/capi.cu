@@ -437,10 +437,11 @@ struct MapKey {
     uint64_t inner, outer;
     uint32_t box_inner, box_outer;
     bool fp4;
+    uint32_t elem;
     bool operator==(const MapKey& o) const
     {
         return base == o.base && inner == o.inner && outer == o.outer && box_inner == o.box_inner &&
-               box_outer == o.box_outer && fp4 == o.fp4;
+               box_outer == o.box_outer && fp4 == o.fp4 && elem == o.elem;
     }
 };
 constexpr int kMapCacheSize = 16;
@@ -452,13 +453,13 @@ struct MapCache {
 } g_maps;
 
 int encode_map_2d_uncached(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer, uint32_t box_inner,
-                           uint32_t box_outer, bool fp4);
+                           uint32_t box_outer, bool fp4, uint32_t elem);
 
-// inner / outer / box in elements; fp4: two E2M1 values per byte in global memory
+// inner / outer / box in elements of `elem` bytes; fp4: two E2M1 values per byte in global memory
 int encode_map_2d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer, uint32_t box_inner,
-                  uint32_t box_outer, bool fp4 = false)
+                  uint32_t box_outer, bool fp4 = false, uint32_t elem = 1)
 {
-    const MapKey k{base, inner, outer, box_inner, box_outer, fp4};
+    const MapKey k{base, inner, outer, box_inner, box_outer, fp4, elem};
     int victim = 0;
     for (int i = 0; i < kMapCacheSize; ++i) {
         if (g_maps.used[i] != 0 && g_maps.key[i] == k) {
@@ -470,7 +471,7 @@ int encode_map_2d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t o
             victim = i;
         }
     }
-    int rc = encode_map_2d_uncached(map, base, inner, outer, box_inner, box_outer, fp4);
+    int rc = encode_map_2d_uncached(map, base, inner, outer, box_inner, box_outer, fp4, elem);
     if (rc == 0) {
         g_maps.key[victim] = k;
         g_maps.map[victim] = *map;
@@ -480,15 +481,16 @@ int encode_map_2d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t o
 }
 
 int encode_map_2d_uncached(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer, uint32_t box_inner,
-                           uint32_t box_outer, bool fp4)
+                           uint32_t box_outer, bool fp4, uint32_t elem)
 {
     cuuint64_t dims[2] = {inner, outer};
-    cuuint64_t strides[1] = {fp4 ? inner / 2 : inner};  // bytes: 8-bit elements, or 4-bit ones packed in pairs
+    cuuint64_t strides[1] = {fp4 ? inner / 2 : inner * elem};  // bytes; 4-bit elements are packed in pairs
     cuuint32_t box[2] = {box_inner, box_outer};
     cuuint32_t estr[2] = {1, 1};
     // packed 4-bit values land in shared memory sixteen to a 16-byte chunk (8 bytes of values, 8 bytes of gap):
     // the same 128 bytes per 128 values as the 8-bit types, so boxes, swizzle and descriptors stay as they are
-    const CUtensorMapDataType dt = fp4 ? CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B : CU_TENSOR_MAP_DATA_TYPE_UINT8;
+    const CUtensorMapDataType dt = fp4 ? CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B
+                                       : (elem == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8);
     CU_TRY(g.drv.TensorMapEncodeTiled(map, dt, 2, const_cast<void*>(base), dims, strides, box,
                                       estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
@@ -526,23 +528,21 @@ int launch_gemm_inst(int grid, cudaStream_t st, const CUtensorMap& ta, const CUt
     return 0;
 }
 
+// CTA pairs that can be resident at once.  A launch never has more: CTAs of one launch wait on flags that other CTAs of
+// the same launch publish.
 template <typename OutT, bool FUSED>
-int launch_gemm_pair_inst(int max_pairs_hint, uint32_t tiles, cudaStream_t st, const CUtensorMap& ta,
-                          const CUtensorMap& tb, const GemmParams& p, bool overlap_predecessor)
+int resident_pairs(uint32_t max_pairs, uint32_t* pairs)
 {
     auto kern = mx_gemm_pair_kernel<OutT, FUSED>;
-    const int threads = FUSED ? kGemmFusedThreads : kGemmThreads;
     static bool attr_done[kMaxRanks * 2] = {};
     static int max_clusters[kMaxRanks * 2] = {};
     int dev = 0;
     CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < kMaxRanks * 2 && !attr_done[dev]) {
+    if (dev >= kMaxRanks * 2 || !attr_done[dev]) {
         CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PairSmem::kDynamicBytes));
-        // how many pairs can be resident at once: the grid never exceeds it, because CTAs of one launch wait
-        // on flags that the quantise warps of other CTAs of the same launch publish
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2 * max_pairs_hint);
-        cfg.blockDim = dim3(threads);
+        cfg.gridDim = dim3(2 * max_pairs);
+        cfg.blockDim = dim3(FUSED ? kGemmFusedThreads : kGemmThreads);
         cfg.dynamicSmemBytes = PairSmem::kDynamicBytes;
         cudaLaunchAttribute attr;
         attr.id = cudaLaunchAttributeClusterDimension;
@@ -554,17 +554,46 @@ int launch_gemm_pair_inst(int max_pairs_hint, uint32_t tiles, cudaStream_t st, c
         int n = 0;
         if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
             cudaGetLastError();
-            n = max_pairs_hint;
+            n = (int)max_pairs;
+        }
+        if (dev >= kMaxRanks * 2) {
+            *pairs = std::min((uint32_t)n, max_pairs);
+            return 0;
         }
         max_clusters[dev] = n;
         attr_done[dev] = true;
     }
-    uint32_t pairs = (uint32_t)(dev < kMaxRanks * 2 ? max_clusters[dev] : max_pairs_hint);
-    if (pairs > (uint32_t)max_pairs_hint) pairs = (uint32_t)max_pairs_hint;
-    if (pairs > tiles) pairs = tiles;
+    *pairs = std::min((uint32_t)max_clusters[dev], max_pairs);
+    return 0;
+}
+
+// Whole rounds of tiles, then the rest cut along K (mx_gemm_pair.cuh).  `parts` <= 1: the rest stays whole.
+struct PairGrid {
+    uint32_t pairs, ksplit;
+};
+
+PairGrid pair_grid(uint32_t tiles, uint32_t pairs, uint32_t parts)
+{
+    const uint32_t rem = tiles % pairs;
+    if (rem == 0 || parts <= 1) {
+        return {std::min(tiles, pairs), 1};
+    }
+    parts = std::min(parts, pairs / rem);
+    return {tiles < pairs ? rem * parts : pairs, parts};
+}
+
+template <typename OutT, bool FUSED>
+int launch_gemm_pair_inst(uint32_t max_pairs, uint32_t tiles, uint32_t parts, cudaStream_t st, const CUtensorMap& ta,
+                          const CUtensorMap& tb, const CUtensorMap& tc, GemmParams& p, bool overlap_predecessor)
+{
+    uint32_t pairs = 0;
+    int rc = resident_pairs<OutT, FUSED>(max_pairs, &pairs);
+    if (rc != 0) return rc;
+    const PairGrid grid = pair_grid(tiles, pairs, parts);
+    p.ksplit = grid.ksplit;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * pairs);
-    cfg.blockDim = dim3(threads);
+    cfg.gridDim = dim3(2 * grid.pairs);
+    cfg.blockDim = dim3(FUSED ? kGemmFusedThreads : kGemmThreads);
     cfg.dynamicSmemBytes = PairSmem::kDynamicBytes;
     cfg.stream = st;
     cudaLaunchAttribute attr;  // the cluster shape is the kernel's own (__cluster_dims__)
@@ -574,61 +603,80 @@ int launch_gemm_pair_inst(int max_pairs_hint, uint32_t tiles, cudaStream_t st, c
     // Without flags the kernel waits for its predecessor itself; with flags it does not, and only the quantise kernel
     // that feeds it may still be running.
     cfg.numAttrs = (overlap_predecessor || (!FUSED && p.flags == nullptr)) ? 1 : 0;
-    CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, ta, tb, p));
+    CUDA_TRY(cudaLaunchKernelEx(&cfg, mx_gemm_pair_kernel<OutT, FUSED>, ta, tb, tc, p));
     g_launches++;
-    CUDA_TRY(cudaGetLastError());
     return 0;
 }
 
-// Rough K-tile periods (microseconds) measured on B200 for the three tilings; used only to pick one.
-constexpr double kPeriodPair256 = 0.43, kPeriodSingle256 = 0.47, kPeriodSingle128 = 0.32;
+// What the tilings cost, in microseconds measured on B200 (kernel alone, back to back): a launch of one K tile, each
+// further K tile of a round with every SM busy, and what splitting K adds (partial tiles written, flagged, read, added;
+// more where more of them cross).  Used only to pick one.
+constexpr double kBasePair = 4.7, kBaseSingle256 = 4.0, kBaseSingle128 = 2.9;
+constexpr double kPeriodPair = 0.37, kPeriodSingle256 = 0.43, kPeriodSingle128 = 0.39;
+constexpr double kSplitCost = 3.5, kSplitCostPerCta = 0.012;
 
 struct GemmPlan {
     bool use_pair;
-    uint32_t block_n, ksplit;
+    uint32_t block_n, ksplit;  // ksplit: CTA pairs: most parts of a last-round tile; single CTAs: parts of every tile
 };
 
 // Tiling of one GEMM launch: CTA pairs or single CTAs, tile width, and the number of K parts.
 GemmPlan plan_gemm(const RankCtx& rc, uint32_t Mg, uint32_t N, uint32_t K, bool no_split = false)
 {
-    // waves x K-tile period of each candidate (same K for all, so K drops out)
     const uint32_t m128 = (Mg + 127) / 128, m256 = (Mg + 255) / 256;
     const uint32_t n128 = (N + 127) / 128, n256 = (N + 255) / 256;
     const uint32_t sms = (uint32_t)rc.num_sms, max_pairs = sms / 2;
-    auto waves = [](uint32_t tiles, uint32_t slots) { return (double)((tiles + slots - 1) / slots); };
-    const double t_pair = waves(m256 * n256, max_pairs) * kPeriodPair256;
-    const double t_256 = waves(m128 * n256, sms) * kPeriodSingle256;
-    const double t_128 = waves(m128 * n128, sms) * kPeriodSingle128;
-    GemmPlan plan;
-    plan.use_pair = (g.cta_pair == 1 || (g.cta_pair == 0 && g.block_n == 0 && t_pair < t_256 && t_pair < t_128));
-    plan.ksplit = 1;
-    uint32_t bn = (uint32_t)g.block_n;
-    // Split K when the tiles would leave at least half of the SMs idle: every (tile, K part) pair gets its
-    // own CTA, the parts' partial tiles meet in this rank's scratch.  Needs the scratch (the allocation-free
-    // entry point has none), an even split and at least four K tiles per part.
-    if (rc.splitk_ws != nullptr && g.split_k != 1 && g.cta_pair != 1 && !no_split) {
-        const uint32_t sbn = (bn == 128 || N <= 128) ? 128u : 256u;
-        const uint32_t stiles = m128 * (sbn == 128 ? n128 : n256);
-        const uint32_t k_tiles = K / kGemmBlockK;
-        // a power of two, at most one part per 32 output columns of the tile
-        const uint32_t cap_opt = g.split_k >= 2 ? (uint32_t)g.split_k : 8u;
-        const uint32_t cap = std::min(std::min(sms / stiles, sbn / 32u), cap_opt);
-        uint32_t s = 1;
-        for (uint32_t t = 2; t <= cap; t *= 2) {
-            if (k_tiles % t == 0 && k_tiles / t >= 4) {
-                s = t;
-            }
-        }
-        if (s >= 2) {
-            plan.ksplit = s;
-            bn = sbn;
-            plan.use_pair = false;
+    const uint32_t k_tiles = K / kGemmBlockK;
+    // Splitting needs the scratch (the allocation-free entry point has none).
+    const bool may_split = rc.splitk_ws != nullptr && g.split_k != 1 && !no_split;
+    const uint32_t cap = may_split ? (g.split_k >= 2 ? (uint32_t)g.split_k : kSplitKMax) : 1u;
+    const bool forced_split = g.split_k >= 2;
+    auto split_cost = [](uint32_t ctas) { return kSplitCost + kSplitCostPerCta * ctas; };
+
+    // CTA pairs: whole rounds, and a last round whose tiles are cut in as many parts as shorten it
+    const uint32_t tiles = m256 * n256, rem = tiles % max_pairs;
+    uint32_t pair_parts = 1;
+    double last = rem != 0 ? k_tiles * kPeriodPair : 0.0;
+    for (uint32_t s = 2; rem != 0 && s <= std::min(std::min(cap, max_pairs / rem), k_tiles); ++s) {
+        const double t = ((k_tiles + s - 1) / s) * kPeriodPair + split_cost(2 * rem * s);
+        if (t < last) {
+            last = t;
+            pair_parts = s;
         }
     }
+    const double t_pair = kBasePair + (tiles / max_pairs) * k_tiles * kPeriodPair + last;
+
+    // single CTAs: rounds of whole tiles, or, when the tiles leave at least half of the SMs idle, every (tile, K part) on
+    // its own CTA (a power of two that divides the K tiles, at least four K tiles per part, one part per 32 columns)
+    auto single = [&](uint32_t bn, uint32_t* parts) {
+        const uint32_t t1 = m128 * (bn == 128 ? n128 : n256);
+        const double base = bn == 128 ? kBaseSingle128 : kBaseSingle256, period = bn == 128 ? kPeriodSingle128 : kPeriodSingle256;
+        double best = base + (double)((t1 + sms - 1) / sms) * k_tiles * period;
+        *parts = 1;
+        for (uint32_t s = 2; s <= std::min(std::min(cap, sms / t1), bn / 32u); s *= 2) {
+            if (k_tiles % s != 0 || k_tiles / s < 4) {
+                continue;
+            }
+            const double t = base + k_tiles / s * period + split_cost(t1 * s);
+            if (t < best || forced_split) {
+                best = t;
+                *parts = s;
+            }
+        }
+        return best;
+    };
+    uint32_t parts128 = 1, parts256 = 1;
+    const double t_128 = single(128, &parts128);
+    const double t_256 = single(256, &parts256);
+    uint32_t bn = (uint32_t)g.block_n;
     if (bn != 128 && bn != 256) {
         bn = (N > 128 && t_256 <= t_128) ? 256 : 128;
     }
-    plan.block_n = bn;
+
+    GemmPlan plan;
+    plan.use_pair = g.cta_pair == 1 || (g.cta_pair == 0 && g.block_n == 0 && t_pair < (bn == 256 ? t_256 : t_128));
+    plan.block_n = plan.use_pair ? kPairBlockN : bn;
+    plan.ksplit = plan.use_pair ? pair_parts : (bn == 256 ? parts256 : parts128);
     return plan;
 }
 
@@ -690,39 +738,49 @@ int launch_gemm(RankCtx& rc, cudaStream_t st, const void* a, const void* b, Gemm
         CUDA_TRY(launch_after(fp4_transpose_kernel, tg, 256, 0, st, static_cast<const uint8_t*>(b), rc.fp4_bt, p.K, p.N));
         b = rc.fp4_bt;
         p.b_kmajor = 1;
+        p.b_early = 0;  // the copy is the kernel launched just before
         overlap_predecessor = false;
     }
-    GemmPlan plan = plan_gemm(rc, p.Mg, p.N, p.K);
-    if (scatter && plan.ksplit > 1) {
-        plan = plan_gemm(rc, p.Mg, p.N, p.K, true);  // the owner adds whole tiles: K stays in one piece
-    }
+    const GemmPlan plan = plan_gemm(rc, p.Mg, p.N, p.K, scatter);  // scatter: the owner adds whole tiles, K stays in one piece
     const bool use_pair = plan.use_pair;
     const uint32_t bn = plan.block_n, ksplit = plan.ksplit;
-    const uint32_t m256 = (p.Mg + 255) / 256, n256 = (p.N + 255) / 256;
+    const uint32_t m256 = (p.Mg + 255) / 256;
     const uint32_t max_pairs = (uint32_t)rc.num_sms / 2;
+    if (ksplit > 1) {
+        p.splitk_ws = rc.splitk_ws;
+        p.splitk_flags = rc.splitk_flags;
+        p.splitk_epoch = ++rc.splitk_epoch;
+    }
     if (use_pair) {
-        CUtensorMap pa, pb;
+        CUtensorMap pa, pb, pc;
         int rc2 = encode_map_2d(&pa, a, p.K, p.Mg, kGemmBlockK, 128, a_fp4);
         if (rc2 != 0) return rc2;
         rc2 = b_fp4 ? encode_map_2d(&pb, b, p.K, p.N, kGemmBlockK, 128, true)
                     : encode_map_2d(&pb, b, p.N, p.K, 128, kGemmBlockK, false);
         if (rc2 != 0) return rc2;
-        const uint32_t tiles = m256 * n256;
+        if (scatter) {
+            pc = pa;  // the epilogue stores to several ranks without a map
+        } else {
+            rc2 = mx_out ? encode_map_2d(&pc, p.c, p.N, p.Mg, 128, 32) : encode_map_2d(&pc, p.c, p.N, p.Mg, 64, 32, false, 2);
+            if (rc2 != 0) return rc2;
+        }
+        const uint32_t tiles = m256 * ((p.N + kPairBlockN - 1) / kPairBlockN);
 #ifdef CATCCOS_TRACE
-        rc.trace_grid = (int)(2 * std::min(tiles, max_pairs));
+        rc.trace_grid = (int)(2 * pair_grid(tiles, max_pairs, ksplit).pairs);
 #endif
+#define CATCCOS_PAIR(OUT, FUSED) \
+    launch_gemm_pair_inst<OUT, FUSED>(max_pairs, tiles, ksplit, st, pa, pb, pc, p, overlap_predecessor)
         if (mx_out) {
-            return launch_gemm_pair_inst<MxOut, false>((int)max_pairs, tiles, st, pa, pb, p, overlap_predecessor);
+            return CATCCOS_PAIR(MxOut, false);
         }
         if (scatter) {
-            return launch_gemm_pair_inst<ScatterOut, false>((int)max_pairs, tiles, st, pa, pb, p, overlap_predecessor);
+            return CATCCOS_PAIR(ScatterOut, false);
         }
         if (fused_quant) {
-            return f16 ? launch_gemm_pair_inst<__half, true>((int)max_pairs, tiles, st, pa, pb, p, overlap_predecessor)
-                       : launch_gemm_pair_inst<__nv_bfloat16, true>((int)max_pairs, tiles, st, pa, pb, p, overlap_predecessor);
+            return f16 ? CATCCOS_PAIR(__half, true) : CATCCOS_PAIR(__nv_bfloat16, true);
         }
-        return f16 ? launch_gemm_pair_inst<__half, false>((int)max_pairs, tiles, st, pa, pb, p, overlap_predecessor)
-                   : launch_gemm_pair_inst<__nv_bfloat16, false>((int)max_pairs, tiles, st, pa, pb, p, overlap_predecessor);
+        return f16 ? CATCCOS_PAIR(__half, false) : CATCCOS_PAIR(__nv_bfloat16, false);
+#undef CATCCOS_PAIR
     }
     CUtensorMap ta, tb;
     int rcode = encode_map_2d(&ta, a, p.K, p.Mg, kGemmBlockK, kGemmBlockM, a_fp4);
@@ -734,9 +792,6 @@ int launch_gemm(RankCtx& rc, cudaStream_t st, const void* a, const void* b, Gemm
     p.ksplit = ksplit;
     if (ksplit > 1) {
         grid = (int)(tiles * ksplit);  // <= SMs by construction: all units are resident at once
-        p.splitk_ws = rc.splitk_ws;
-        p.splitk_flags = rc.splitk_flags;
-        p.splitk_epoch = ++rc.splitk_epoch;
     }
 #ifdef CATCCOS_TRACE
     rc.trace_grid = grid;
@@ -976,6 +1031,8 @@ int allgather_matmul(void* stream, const void* a, const void* a_scale, bool preq
         }
         if (rcode != 0) return rcode;
         p.flags = nullptr;  // stream order is the only dependency
+        // The quantiser waits for its own predecessor before it lets this launch go, so the weights are in place.
+        p.b_early = prequant ? 0u : 1u;
         return launch_gemm(rc, st, a_stage, b, p, false, true);
     }
     if (fuse_mode == 6) {
@@ -1665,11 +1722,7 @@ int catccos_b200_mx_gemm_quant_out(void* stream, const void* a, const void* a_sc
 // Matmul + ReduceScatter: what plan_gemm will choose for the N tile (the reducer walks the same tiles)
 static uint32_t scatter_block_n(const RankCtx& rc, uint32_t M, uint32_t N, uint32_t K)
 {
-    GemmPlan plan = plan_gemm(rc, M, N, K);
-    if (plan.ksplit > 1) {
-        plan = plan_gemm(rc, M, N, K, true);
-    }
-    return plan.use_pair ? kPairBlockN : plan.block_n;
+    return plan_gemm(rc, M, N, K, true).block_n;
 }
 
 int catccos_b200_mxfp8_matmul_reduce_scatter(void* stream, const void* a, const void* b, const void* a_scale,

@@ -79,6 +79,8 @@ struct GemmParams {
     uint32_t flag_stride;
     uint32_t segs, seg_ktiles;
     uint32_t world, rank, m_local, epoch;
+    uint32_t b_early;         // 1: B and its scales were in place before the kernel launched just before this one (the
+                              // quantiser of the same call): they are loaded while that kernel drains
     uint32_t gemm_off;        // 1: the GEMM warps stay idle (the producer half of a call, run apart)
     uint32_t own_first;       // tile order of a gated launch: 1 = this rank's whole shard first (it is there before any
                               // peer's rows), 0 = slice by slice over ALL ranks, own slice leading (every rank's
@@ -89,10 +91,10 @@ struct GemmParams {
     unsigned long long* trace;  // timeline side buffer (trace build only), else nullptr
     QuantPushParams q;  // the producer's work when the quantise warps ride in this kernel (local stage only)
     PushParams push;    // the pusher warps' work: local stage -> the peers' stages
-    // Split K (ksplit > 1): K is cut in ksplit equal parts and every (tile, part) pair is a work unit of its
-    // own CTA (units == grid, so all of them are resident together).  Every part owns an equal share of the
-    // tile's columns, writes the rest of its fp32 partial tile to the workspace, and adds the other parts'
-    // pieces of its own columns in ascending part order.  ksplit is a power of two <= BLOCK_N / 32.
+    // Split K (ksplit > 1): the K range of a tile is cut in ksplit parts, every (tile, part) is a work unit of its own
+    // CTA (or CTA pair), and all of them are resident together.  Every part owns an equal share of the tile's columns,
+    // writes the rest of its fp32 partial tile to the workspace, and adds the other parts' pieces of its own columns in
+    // ascending part order (SplitExchange).  ksplit <= BLOCK_N / 32.
     uint32_t ksplit;
     float* splitk_ws;        // [tiles][ksplit][BLOCK_N / 32][128][32]
     uint32_t* splitk_flags;  // [tiles][ksplit][4] epoch words, one per epilogue warp
@@ -118,6 +120,7 @@ struct GemmSmem {
     static constexpr uint32_t kOffTmemPtr = kOffBar + kNumBars * 8;
     static constexpr uint32_t kOffGate = kOffTmemPtr + 8;  // K-tile iterations whose rows the producer has seen ready
     static constexpr uint32_t kBytes = kOffTmemPtr + 16;
+    static_assert(4 * 49152 <= kOffSfa, "the split-K pieces land in the idle operand stages");
     static constexpr uint32_t kDynamicBytes = kBytes + 1024;  // slack to align the base to 1024 bytes
     // Tensor memory: two 128 x BLOCK_N fp32 accumulators and one set of scale factors per stage (12 columns:
     // SFA 4, then SFB 4 per 128 columns of N).  For BLOCK_N = 256 the accumulators overlap by 64 columns
@@ -314,6 +317,25 @@ __device__ __forceinline__ void store_c_chunk(OutT* c, const GemmParams& p, uint
 // the core, without materialising the 16-bit tensor.
 struct MxOut {};
 
+__device__ __forceinline__ void mx_quantise_chunk(const GemmParams& p, const uint32_t (&r)[32], uint32_t (&o)[8], uint32_t& byte)
+{
+    uint32_t w[16];
+    uint32_t amax = 0;
+#pragma unroll
+    for (uint32_t e = 0; e < 16; ++e) {
+        w[e] = pack2<__nv_bfloat16>(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]));
+        amax = __vmaxu2(amax, w[e] & 0x7FFF7FFFu);
+    }
+    amax = max(amax & 0xFFFFu, amax >> 16);
+    float mul;
+    bool nonfinite;
+    block_scale(amax, p.c_tiny_rule == kQuantDeviceTiny, 8u, byte, mul, nonfinite);
+#pragma unroll
+    for (uint32_t e = 0; e < 8; ++e) {
+        o[e] = nonfinite ? 0x7F7F7F7Fu : encode4(w[2 * e], w[2 * e + 1], mul, false);
+    }
+}
+
 template <>
 __device__ __forceinline__ void store_c_chunk<MxOut>(MxOut*, const GemmParams& p, uint32_t row, uint32_t col,
                                                      const uint32_t (&r)[32])
@@ -321,23 +343,8 @@ __device__ __forceinline__ void store_c_chunk<MxOut>(MxOut*, const GemmParams& p
     if (row >= p.Mg || col >= p.N) {
         return;  // N is a multiple of 32 here (checked by the host), so a chunk is inside or outside as a whole
     }
-    uint32_t w[16];
-    uint32_t amax = 0;
-#pragma unroll
-    for (uint32_t e = 0; e < 16; ++e) {
-        w[e] = pack2<__nv_bfloat16>(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]));
-        const uint32_t a = w[e] & 0x7FFF7FFFu;
-        amax = max(amax, max(a & 0xFFFFu, a >> 16));
-    }
-    uint32_t byte;
-    float mul;
-    bool nonfinite;
-    block_scale(amax, p.c_tiny_rule == kQuantDeviceTiny, 8u, byte, mul, nonfinite);
-    uint32_t o[8];
-#pragma unroll
-    for (uint32_t e = 0; e < 8; ++e) {
-        o[e] = nonfinite ? 0x7F7F7F7Fu : encode4(w[2 * e], w[2 * e + 1], mul, false);
-    }
+    uint32_t o[8], byte;
+    mx_quantise_chunk(p, r, o, byte);
     st_global_v8(static_cast<uint8_t*>(p.c) + (size_t)row * p.N + col, o);
     p.c_scales[(size_t)row * (p.N / 32u) + col / 32u] = (uint8_t)byte;
 }
@@ -388,6 +395,187 @@ __device__ __forceinline__ void publish_tile_rows(const GemmParams& p, uint32_t 
     }
 }
 
+// ---- output through shared memory: 32 rows x 128 bytes of one epilogue warp leave as one TMA store (128-byte swizzle) ----
+// A lane holds a row, so stores straight from registers touch 32 lines per instruction; staged, the rows leave as whole
+// 128-byte lines and the ragged edge is the tensor map's business.
+constexpr uint32_t kOutStageBytes = 32 * 128;
+
+__device__ __forceinline__ void out_stage_free(uint32_t lane)
+{
+    if (lane == 0) {
+        bulk_store_wait_read();  // the previous store from this buffer has been read
+    }
+    __syncwarp();
+}
+
+// 32 bytes of this lane's row, at 16-byte slots `slot` and slot + 1
+__device__ __forceinline__ void out_stage_put(uint8_t* stage, uint32_t lane, uint32_t slot, const uint32_t (&o)[8])
+{
+    *reinterpret_cast<uint4*>(stage + lane * 128u + ((slot ^ (lane & 7u)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+    *reinterpret_cast<uint4*>(stage + lane * 128u + (((slot + 1u) ^ (lane & 7u)) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
+}
+
+__device__ __forceinline__ void out_stage_send(const uint8_t* stage, const void* tmap, uint32_t lane, bool inside, uint32_t col,
+                                               uint32_t row0)
+{
+    fence_proxy_async_shared();
+    __syncwarp();
+    if (lane == 0 && inside) {
+        tma_store_2d(tmap, stage, (int32_t)col, (int32_t)row0);
+        bulk_store_commit();
+    }
+}
+
+// 32 accumulator columns of this lane's row as 64 bytes of 16-bit output, at 16-byte slots `slot` .. slot + 3
+template <typename OutT>
+__device__ __forceinline__ void out_stage_put_chunk(uint8_t* stage, uint32_t lane, uint32_t slot, const uint32_t (&r)[32])
+{
+#pragma unroll
+    for (uint32_t v = 0; v < 2; ++v) {
+        uint32_t o[8];
+#pragma unroll
+        for (uint32_t e = 0; e < 8; ++e) {
+            o[e] = pack2<OutT>(__uint_as_float(r[v * 16 + 2 * e]), __uint_as_float(r[v * 16 + 2 * e + 1]));
+        }
+        out_stage_put(stage, lane, slot + 2u * v, o);
+    }
+}
+
+// MxOut: the scales of columns col .. col + 127 of one row (col is a multiple of 128)
+__device__ __forceinline__ void store_scale_word(const GemmParams& p, uint32_t row, uint32_t col, uint32_t word)
+{
+    if (row >= p.Mg || col >= p.N) {
+        return;
+    }
+    uint8_t* dst = p.c_scales + (size_t)row * (p.N / 32u) + col / 32u;
+    if (p.N % 128u == 0u && ((uintptr_t)p.c_scales & 3u) == 0u) {
+        *reinterpret_cast<uint32_t*>(dst) = word;
+    } else {
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+            if (col + 32u * i < p.N) {
+                dst[i] = (uint8_t)(word >> (8u * i));
+            }
+        }
+    }
+}
+
+// ---- split K: the parts of a tile add up their fp32 partial tiles ----
+// Every part owns an equal share of the tile's 32-column chunks.  A warp first writes the chunks its part does not own
+// to the workspace ([part][chunk][128 rows x 32 floats], 4 KiB per chunk and warp) and raises its flag; then lane 0
+// pulls the other parts' pieces of the owned chunks into idle operand stages with bulk copies, all in flight at once,
+// and the warp adds them to its own accumulator in ascending part order and writes C.
+constexpr uint32_t kSplitKMax = 8;
+constexpr uint32_t kSplitPieceBytes = 32u * 32u * 4u;           // 32 rows x 32 floats
+constexpr uint32_t kSplitRedBytes = 12u * kSplitPieceBytes;     // most pieces a warp takes in: two chunks from six parts
+
+template <typename OutT, uint32_t kChunks>
+struct SplitExchange {
+    float* ws;            // part 0's partial tile
+    size_t part_stride;   // floats between the parts' partial tiles
+    uint32_t* flags;      // this warp's flag word of part 0
+    uint32_t flag_stride;
+    uint8_t* red;         // kSplitRedBytes of shared memory
+    uint64_t* bar;
+
+    // row0: the warp's first row; id names the tile in a status record.  Returns false when a wait gave up (then C keeps
+    // what the caller put there).
+    __device__ __forceinline__ bool run(const GemmParams& p, OutT* c, uint32_t tmem_acc, uint32_t part, uint32_t parts, uint32_t q,
+                                        uint32_t lane, uint32_t row0, uint32_t n0, uint32_t id, uint64_t bar_ns)
+    {
+        // a warp whose 32 rows all lie below the matrix has nothing to add up (its peers in the other parts take the
+        // same decision, so nobody waits for its flag); lanes below the matrix skip their partial stores
+        if (row0 >= p.Mg) {
+            return true;
+        }
+        const uint32_t row = row0 + lane;
+        const bool lane_row = row < p.Mg;
+        const uint32_t own0 = (part * kChunks + parts - 1u) / parts, own1 = ((part + 1u) * kChunks + parts - 1u) / parts;
+        const uint32_t owned = own1 - own0;
+        for (uint32_t chunk = 0; chunk < kChunks; ++chunk) {
+            if (chunk - own0 < owned || n0 + chunk * 32u >= p.N) {
+                continue;
+            }
+            uint32_t r[32];
+            tmem_ld_32x32(tmem_acc + chunk * 32u, r);
+            tmem_ld_wait();
+            // inside a 4 KiB piece (32 rows x 32 floats) the 16-byte vector v of row `lane` sits at slot
+            // v * 32 + lane: every store instruction of the warp covers 512 contiguous bytes, and the
+            // reader's shared-memory loads are free of bank conflicts
+            float4* dst = reinterpret_cast<float4*>(ws + part * part_stride + ((size_t)chunk * 128u + q * 32u) * 32u) + lane;
+#pragma unroll
+            for (uint32_t v = 0; v < 8; ++v) {
+                if (lane_row) {
+                    dst[v * 32u] = make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]),
+                                               __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
+                }
+            }
+        }
+        __syncwarp();  // every lane's partial stores are ordered before lane 0's release
+        if (lane == 0) {
+            st_release_gpu(flags + part * flag_stride, p.splitk_epoch);
+        }
+        // chunks right of the matrix were not written by anybody
+        const uint32_t own_end = n0 >= p.N ? own0 : max(own0, min(own1, (p.N - n0 + 31u) / 32u));
+        if (own_end == own0) {
+            return true;
+        }
+        // lanes 0 .. parts-1 each watch one part's flag (the polls overlap instead of queueing up)
+        bool ok = true;
+        if (lane < parts && lane != part &&
+            !wait_flag_ge_gpu(flags + lane * flag_stride, p.splitk_epoch, p.timeout_ns, p.status)) {
+            report_status(p.status, kStatusFlagTimeout, 0x100u + lane, id, p.splitk_epoch);
+            ok = false;
+        }
+        if (!__all_sync(0xFFFFFFFFu, ok)) {
+            return false;
+        }
+        if (lane == 0) {
+            mbar_arrive_expect_tx(bar, (parts - 1u) * (own_end - own0) * kSplitPieceBytes);
+            fence_proxy_async_all();  // the other parts' generic-proxy stores before this thread's bulk copies
+            uint32_t slot = 0;
+            for (uint32_t other = 0; other < parts; ++other) {
+                for (uint32_t chunk = own0; other != part && chunk < own_end; ++chunk, ++slot) {
+                    bulk_load(red + slot * kSplitPieceBytes, ws + other * part_stride + ((size_t)chunk * 128u + q * 32u) * 32u,
+                              kSplitPieceBytes, bar);
+                }
+            }
+        }
+        __syncwarp();
+        if (!mbar_wait_warp(bar, 0, p.status, 107, q, bar_ns)) {
+            return false;
+        }
+        for (uint32_t chunk = own0; chunk < own_end; ++chunk) {
+            uint32_t r[32];
+            tmem_ld_32x32(tmem_acc + chunk * 32u, r);
+            tmem_ld_wait();
+            for (uint32_t pi = 0; pi + 1u < parts; ++pi) {
+                // four 16-byte loads at a time: enough to hide the shared-memory latency without
+                // crowding the 32 accumulator registers
+                const uint32_t src = smem_u32(red + (pi * (own_end - own0) + (chunk - own0)) * kSplitPieceBytes + lane * 16u);
+#pragma unroll
+                for (uint32_t h = 0; h < 2; ++h) {
+                    float4 f[4];
+#pragma unroll
+                    for (uint32_t v = 0; v < 4; ++v) {
+                        f[v] = ld_shared_v4(src + (h * 4u + v) * 512u);
+                    }
+#pragma unroll
+                    for (uint32_t v = 0; v < 4; ++v) {
+                        const uint32_t e = (h * 4u + v) * 4u;
+                        r[e] = __float_as_uint(__uint_as_float(r[e]) + f[v].x);
+                        r[e + 1] = __float_as_uint(__uint_as_float(r[e + 1]) + f[v].y);
+                        r[e + 2] = __float_as_uint(__uint_as_float(r[e + 2]) + f[v].z);
+                        r[e + 3] = __float_as_uint(__uint_as_float(r[e + 3]) + f[v].w);
+                    }
+                }
+            }
+            store_c_chunk<OutT>(c, p, row, n0 + chunk * 32u, r);
+        }
+        return true;
+    }
+};
+
 // The consumer half of Matmul + ReduceScatter: this rank's rows of the product, D [rs_rows, N] = the sum over the
 // source ranks, in rank order, of the fp32 partials in this rank's stage.  One CTA per (32-row block, N tile) of
 // the producing GEMM, as soon as all ranks have flagged it (bounded wait).
@@ -434,7 +622,8 @@ __global__ void __launch_bounds__(256) mx_reduce_scatter_kernel(const float* __r
 
 template <uint32_t BLOCK_N, typename OutT, bool FUSED_QUANT>
 __global__ void __launch_bounds__(FUSED_QUANT ? kGemmFusedThreads : kGemmThreads, 1)
-mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, GemmParams p)
+mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+               const __grid_constant__ GemmParams p)
 {
     using S = GemmSmem<BLOCK_N>;
     constexpr uint32_t kStages = S::kStages;
@@ -491,22 +680,47 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     __syncthreads();
     tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_ptr_smem;
+    bool alive = true;  // false once a wait of this role has given up
     if (threadIdx.x == 0) {
         CATCCOS_TR_STAMP(p.trace, kTrSetupDone);
     }
 
     if (warp == 4) {
         // ------------------------------- TMA producer -------------------------------------
-        if (p.flags == nullptr) {
-            grid_dep_wait();  // A is the output of the kernel launched just before (no-op for a plain launch);
-        }                     // with flags, the flags say when its rows are there
+        uint32_t early = 0;   // iterations whose B tile is already on its way
         const uint32_t ksplit = p.ksplit > 1u ? p.ksplit : 1u;
         const uint32_t kper = k_tiles / ksplit;  // K tiles per work unit (the host only splits evenly)
         const uint32_t num_units = num_tiles * ksplit;
         uint32_t it = 0, ti = 0;
-        bool alive = true;
         // packed 4-bit operands arrive as half the bytes they occupy in shared memory (the gaps are not written)
         const uint32_t tx_bytes = (p.a_fmt == 5u ? S::kABytes / 2u : S::kABytes) + (p.b_fmt == 5u ? S::kBBytes / 2u : S::kBBytes);
+        auto load_b = [&](uint32_t n0, uint32_t kt, uint32_t s) {
+            if (p.b_kmajor) {
+                // the transposed copy [N, K]: box = 128 (K, contiguous) x BLOCK_N rows
+                tma_load_2d(smem + S::kOffB + s * S::kBBytes, &tmap_b, &full[s], (int32_t)(kt * kGemmBlockK), (int32_t)n0);
+            } else {
+                // B is [K, N] row-major: box = 128 (N, contiguous) x 128 (K); one box per 128 columns
+                for (uint32_t h = 0; h < BLOCK_N / 128; ++h) {
+                    tma_load_2d(smem + S::kOffB + s * S::kBBytes + h * 16384u, &tmap_b, &full[s], (int32_t)(n0 + h * 128u),
+                                (int32_t)(kt * kGemmBlockK));
+                }
+            }
+        };
+        if (p.flags == nullptr) {
+            if (p.b_early && blockIdx.x < num_units) {
+                // the weights do not come from the kernel launched just before: fill the ring's B half meanwhile
+                const uint32_t ks = blockIdx.x / num_tiles;
+                const uint32_t n0 = tile_coord(blockIdx.x - ks * num_tiles, n_tiles, m_tiles, p).n_tile * BLOCK_N;
+                early = min(kStages, kper);
+                if (lane == 0) {
+                    for (uint32_t s = 0; s < early; ++s) {
+                        mbar_arrive_expect_tx(&full[s], tx_bytes);
+                        load_b(n0, ks * kper + s, s);
+                    }
+                }
+            }
+            grid_dep_wait();  // A is the output of the kernel launched just before (no-op for a plain launch);
+        }                     // with flags, the flags say when its rows are there
         for (uint32_t unit = blockIdx.x; alive && unit < num_units; unit += gridDim.x, ++ti) {
             const uint32_t ks = unit / num_tiles;
             TileCoord tc = tile_coord(unit - ks * num_tiles, n_tiles, m_tiles, p);
@@ -532,27 +746,21 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 if (lane == 0 && alive) {
                     const uint32_t s = it % kStages;
                     const uint32_t ph = (it / kStages) & 1u;
-                    const unsigned long long t1 = CATCCOS_TR_NOW();
-                    (void)t1;
-                    alive = mbar_wait(&empty[s], ph ^ 1u, p.status, 100, s, bar_ns);
-                    CATCCOS_TR_ADD(p.trace, kTrProdEmptyWaitNs, CATCCOS_TR_NOW() - t1);
+                    if (it >= early) {
+                        const unsigned long long t1 = CATCCOS_TR_NOW();
+                        (void)t1;
+                        alive = mbar_wait(&empty[s], ph ^ 1u, p.status, 100, s, bar_ns);
+                        CATCCOS_TR_ADD(p.trace, kTrProdEmptyWaitNs, CATCCOS_TR_NOW() - t1);
+                        mbar_arrive_expect_tx(&full[s], tx_bytes);
+                    }
                     if (kt == kt0 && ti < kTraceTiles) {
                         CATCCOS_TR_STAMP(p.trace, kTrTileStart + ti);
                     }
                     CATCCOS_TR_STAMP_FIRST(p.trace, kTrProdFirstTma);
-                    mbar_arrive_expect_tx(&full[s], tx_bytes);
                     tma_load_2d(smem + S::kOffA + s * S::kABytes, &tmap_a, &full[s], (int32_t)(kt * kGemmBlockK),
                                 (int32_t)m0);
-                    if (p.b_kmajor) {
-                        // the transposed copy [N, K]: box = 128 (K, contiguous) x BLOCK_N rows
-                        tma_load_2d(smem + S::kOffB + s * S::kBBytes, &tmap_b, &full[s], (int32_t)(kt * kGemmBlockK),
-                                    (int32_t)n0);
-                    } else {
-                        // B is [K, N] row-major: box = 128 (N, contiguous) x 128 (K); one box per 128 columns
-                        for (uint32_t h = 0; h < BLOCK_N / 128; ++h) {
-                            tma_load_2d(smem + S::kOffB + s * S::kBBytes + h * 16384u, &tmap_b, &full[s],
-                                        (int32_t)(n0 + h * 128u), (int32_t)(kt * kGemmBlockK));
-                        }
+                    if (it >= early) {
+                        load_b(n0, kt, s);
                     }
                     CATCCOS_TR_STAMP(p.trace, kTrProdLastTma);
                 }
@@ -561,87 +769,78 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         }
     } else if (warp == 5) {
         // ------------------------------- MMA issuer ---------------------------------------
-        // One thread gets a tcgen05 instruction out only every ~70 cycles, so this thread issues what nobody
-        // else can (the MMAs, and the commit that releases the stage) and nothing more: four MMAs of 128 cycles
-        // each leave it enough time for the commit, the wait for the next stage and its address arithmetic.
-        if (lane == 0) {
-            const bool bk = p.b_kmajor != 0u;
-            const uint32_t idesc = make_idesc_mxf8(kGemmBlockM, BLOCK_N, !bk) | ((p.a_fmt & 7u) << 7) |
-                                   ((p.b_fmt & 7u) << 10);  // operand formats: E4M3 = 0, E5M2 = 1, E2M1 = 5
-            const uint32_t ksplit = p.ksplit > 1u ? p.ksplit : 1u;
-            const uint32_t kper = k_tiles / ksplit;  // K tiles per work unit (the host only splits evenly)
-            const uint32_t num_units = num_tiles * ksplit;
-            const uint32_t my_units = (num_units > blockIdx.x) ? (num_units - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u;
-            const uint32_t total_it = my_units * kper;
+        // The whole warp runs the loop and one elected lane issues: inside a branch on the lane the operands of a tcgen05
+        // instruction cannot stay in uniform registers, and each then takes about 70 cycles to get out.  The issuer
+        // issues what nobody else can (the MMAs, and the commit that releases the stage) and nothing more.
+        const bool bk = p.b_kmajor != 0u;
+        const uint32_t idesc = make_idesc_mxf8(kGemmBlockM, BLOCK_N, !bk) | ((p.a_fmt & 7u) << 7) |
+                               ((p.b_fmt & 7u) << 10);  // operand formats: E4M3 = 0, E5M2 = 1, E2M1 = 5
+        const uint32_t ksplit = p.ksplit > 1u ? p.ksplit : 1u;
+        const uint32_t kper = k_tiles / ksplit;  // K tiles per work unit (the host only splits evenly)
+        const uint32_t num_units = num_tiles * ksplit;
+        const uint32_t my_units = (num_units > blockIdx.x) ? (num_units - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u;
 
-            // descriptor halves: the high words are constants, the low words are start addresses >> 4
-            // A: K-major, 128-byte swizzle, 8-row groups 1024 bytes apart; K advances 32 bytes in the row.
-            // B: MN-major, 128-byte swizzle: 128 columns contiguous, K rows 128 bytes apart, 8-row K groups
-            // 1024 bytes apart (SBO), 128-column groups 16 KiB apart (LBO).
-            const uint32_t hi_a = (uint32_t)(make_smem_desc(0, 16, 1024, 2) >> 32);
-            const uint32_t hi_b = bk ? hi_a : (uint32_t)(make_smem_desc(0, 16384, 1024, 2) >> 32);
-            const uint32_t a_lo0 = (uint32_t)make_smem_desc(0, 16, 1024, 2) | (smem_u32(smem + S::kOffA) >> 4);
-            const uint32_t b_lo0 = (uint32_t)make_smem_desc(0, bk ? 16 : 16384, 1024, 2) | (smem_u32(smem + S::kOffB) >> 4);
-            constexpr uint32_t kKbStepA = 32u >> 4;                // 32 bytes along K
-            const uint32_t kKbStepB = (bk ? 32u : 4096u) >> 4;     // 32 bytes along K, or 32 K rows of 128 bytes
-            const uint32_t sf_tmem0 = tmem_base + S::kSfCol;
-            bool alive = true;
-
-            auto stage_wait = [&](uint32_t s, uint32_t ph) {
-                const unsigned long long t0 = CATCCOS_TR_NOW();
-                (void)t0;
-                alive = mbar_wait(&full[s], ph, p.status, 103, s, bar_ns);
-                tcgen05_fence_after();
-                CATCCOS_TR_ADD(p.trace, kTrMmaFullWaitNs, CATCCOS_TR_NOW() - t0);
-            };
-            auto issue_mma = [&](uint32_t a_lo, uint32_t b_lo, uint32_t sf, uint32_t kb, uint32_t d_col, uint32_t accumulate) {
-                umma_mxf8_lohi(d_col, a_lo + kb * kKbStepA, hi_a, b_lo + kb * kKbStepB, hi_b, idesc_with_sf_id(idesc, kb), sf,
-                               sf + 4, accumulate);
-            };
-
-            if (total_it > 0) {
-                stage_wait(0, 0);
+        // descriptor halves: the high words are constants, the low words are start addresses >> 4
+        // A: K-major, 128-byte swizzle, 8-row groups 1024 bytes apart; K advances 32 bytes in the row.
+        // B: MN-major, 128-byte swizzle: 128 columns contiguous, K rows 128 bytes apart, 8-row K groups
+        // 1024 bytes apart (SBO), 128-column groups 16 KiB apart (LBO).
+        const uint32_t hi_a = (uint32_t)(make_smem_desc(0, 16, 1024, 2) >> 32);
+        const uint32_t hi_b = bk ? hi_a : (uint32_t)(make_smem_desc(0, 16384, 1024, 2) >> 32);
+        const uint32_t a_lo0 = (uint32_t)make_smem_desc(0, 16, 1024, 2) | (smem_u32(smem + S::kOffA) >> 4);
+        const uint32_t b_lo0 = (uint32_t)make_smem_desc(0, bk ? 16 : 16384, 1024, 2) | (smem_u32(smem + S::kOffB) >> 4);
+        constexpr uint32_t kKbStepA = 32u >> 4;                // 32 bytes along K
+        const uint32_t kKbStepB = (bk ? 32u : 4096u) >> 4;     // 32 bytes along K, or 32 K rows of 128 bytes
+        uint32_t s = 0, ph = 0;
+        for (uint32_t ti = 0; alive && ti < my_units; ++ti) {
+            const uint32_t acc = ti & 1u;
+            const uint32_t acc_ph = (ti >> 1) & 1u;
+            const uint32_t d_col = tmem_base + (acc ? S::kAccCol1 : 0u);
+            const unsigned long long t0 = CATCCOS_TR_NOW();
+            (void)t0;
+            alive = mbar_wait_warp(&tmem_empty[acc], acc_ph ^ 1u, p.status, 101, acc, bar_ns);
+            if (S::kOverlap && ti > 0 && alive) {
+                alive = mbar_wait_warp(&overlap_free[acc ^ 1u], ((ti - 1) >> 1) & 1u, p.status, 102, acc, bar_ns);
             }
-            uint32_t it = 0, s = 0, ph = 0;
-            for (uint32_t ti = 0; alive && ti < my_units; ++ti) {
-                const uint32_t acc = ti & 1u;
-                const uint32_t acc_ph = (ti >> 1) & 1u;
-                const uint32_t d_col = tmem_base + (acc ? S::kAccCol1 : 0u);
-                const unsigned long long t0 = CATCCOS_TR_NOW();
-                (void)t0;
-                alive = mbar_wait(&tmem_empty[acc], acc_ph ^ 1u, p.status, 101, acc, bar_ns);
-                if (S::kOverlap && ti > 0 && alive) {
-                    alive = mbar_wait(&overlap_free[acc ^ 1u], ((ti - 1) >> 1) & 1u, p.status, 102, acc, bar_ns);
-                }
+            if (lane == 0) {
                 CATCCOS_TR_ADD(p.trace, kTrMmaAccWaitNs, CATCCOS_TR_NOW() - t0);
-                tcgen05_fence_after();
-                CATCCOS_TR_STAMP_FIRST(p.trace, kTrMmaFirst);
-                for (uint32_t kt = 0; alive && kt < kper; ++kt, ++it) {
-                    const uint32_t a_lo = a_lo0 + s * (S::kABytes >> 4);
-                    const uint32_t b_lo = b_lo0 + s * (S::kBBytes >> 4);
-                    const uint32_t sf = sf_tmem0 + s * S::kSfSetCols;
-                    const uint32_t s_next = (s + 1 == kStages) ? 0u : s + 1;
-                    const uint32_t ph_next = ph ^ (s_next == 0u ? 1u : 0u);
-                    const bool more = it + 1 < total_it;
-                    issue_mma(a_lo, b_lo, sf, 0, d_col, kt != 0 ? 1u : 0u);
-                    issue_mma(a_lo, b_lo, sf, 1, d_col, 1u);
-                    issue_mma(a_lo, b_lo, sf, 2, d_col, 1u);
-                    issue_mma(a_lo, b_lo, sf, 3, d_col, 1u);
-                    tcgen05_commit(&empty[s]);
-                    if (more) {
-                        stage_wait(s_next, ph_next);
-                    }
-                    s = s_next;
-                    ph = ph_next;
+            }
+            for (uint32_t kt = 0; alive && kt < kper; ++kt) {
+                const unsigned long long t1 = CATCCOS_TR_NOW();
+                (void)t1;
+                alive = mbar_wait_warp(&full[s], ph, p.status, 103, s, bar_ns);
+                if (!alive) {
+                    break;  // nothing is issued, and the accumulator never reported, after a wait has given up
                 }
-                tcgen05_commit(&tmem_full[acc]);
+                tcgen05_fence_after();
+                if (lane == 0) {
+                    CATCCOS_TR_ADD(p.trace, kTrMmaFullWaitNs, CATCCOS_TR_NOW() - t1);
+                    CATCCOS_TR_STAMP_FIRST(p.trace, kTrMmaFirst);
+                }
+                const uint32_t a_lo = a_lo0 + s * (S::kABytes >> 4);
+                const uint32_t b_lo = b_lo0 + s * (S::kBBytes >> 4);
+                const uint32_t sf = tmem_base + S::kSfCol + s * S::kSfSetCols;
+                if (elect_one()) {
+#pragma unroll
+                    for (uint32_t kb = 0; kb < 4; ++kb) {
+                        umma_mxf8_lohi(d_col, a_lo + kb * kKbStepA, hi_a, b_lo + kb * kKbStepB, hi_b, idesc_with_sf_id(idesc, kb),
+                                       sf, sf + 4, (kb != 0u || kt != 0u) ? 1u : 0u);
+                    }
+                    tcgen05_commit(&empty[s]);
+                    if (kt + 1u == kper) {
+                        tcgen05_commit(&tmem_full[acc]);
+                    }
+                }
+                __syncwarp();
+                s = (s + 1 == kStages) ? 0u : s + 1;
+                ph ^= s == 0u ? 1u : 0u;
+            }
+            if (lane == 0) {
                 if (ti < kTraceTiles) {
                     CATCCOS_TR_STAMP(p.trace, kTrTileEnd + ti);
                 }
                 CATCCOS_TR_STAMP(p.trace, kTrMmaLast);
             }
         }
-        __syncwarp();
     } else if (FUSED_QUANT && warp >= 10) {
         // ------------------------------- quantise-and-push producer -----------------------
         // Of the fourteen extra warps, eight quantise this rank's shard into the local stage (warps 10-19
@@ -677,7 +876,6 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         uint32_t cur_a[4], cur_lo[kNB], cur_hi[kNB];
         uint32_t nxt_a[4], nxt_lo[kNB], nxt_hi[kNB];
         uint32_t known_end = 0;  // K-tile iterations below this index have their rows in place
-        bool alive = true;
 
         auto issue_loads = [&](uint32_t it, uint32_t (&ra)[4], uint32_t (&rlo)[kNB], uint32_t (&rhi)[kNB]) {
             const uint32_t seq = it / kper;
@@ -791,118 +989,27 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         const uint32_t ksplit = p.ksplit > 1u ? p.ksplit : 1u;
         const uint32_t num_units = num_tiles * ksplit;
         if (ksplit > 1u && num_tiles > 0u) {
-            // Split K: this CTA is work unit blockIdx.x = (tile, part ks) and the only one on its SM.  Each part
-            // owns kChunks / ksplit of the tile's 32-column chunks.  A part first writes the chunks it does not
-            // own to its partial tile in the workspace ([part][chunk][128 rows x 32 floats], 4 KiB per chunk and
-            // warp) and raises a flag per epilogue warp; then lane 0 of every warp pulls the other parts' pieces
-            // of the owned chunks into the (now idle) operand stages with bulk copies, all in flight at once,
-            // and the warp adds them to its own accumulator in ascending part order and writes C.
-            const uint32_t unit = blockIdx.x;
-            const uint32_t ks = unit / num_tiles;
-            const uint32_t tile = unit - ks * num_tiles;
+            // Split K: this CTA is work unit blockIdx.x = (tile, part ks) and the only one on its SM.
+            const uint32_t ks = blockIdx.x / num_tiles;
+            const uint32_t tile = blockIdx.x - ks * num_tiles;
             TileCoord tc = tile_coord(tile, n_tiles, m_tiles, p);
-            const uint32_t m0 = tc.m_tile * kGemmBlockM;
-            const uint32_t n0 = tc.n_tile * BLOCK_N;
-            const uint32_t row = m0 + q * 32 + lane;
-            const uint32_t cps = kChunks / ksplit;
-            const uint32_t own0 = ks * cps;
-            constexpr size_t kPartFloats = (size_t)kGemmBlockM * BLOCK_N;
-            constexpr uint32_t kPieceBytes = 32u * 32u * 4u;  // 32 rows x 32 floats
-            float* parts = p.splitk_ws + (size_t)tile * ksplit * kPartFloats;
-            uint32_t* flags = p.splitk_flags + (size_t)tile * ksplit * 4u;
-            bool alive = mbar_wait_warp(&tmem_full[0], 0, p.status, 106, 0, bar_ns);
+            alive = mbar_wait_warp(&tmem_full[0], 0, p.status, 106, 0, bar_ns);
             tcgen05_fence_after();
-            // a warp whose 32 rows all lie below the matrix has nothing to add up (its peers in the other
-            // parts take the same decision, so nobody waits for its flag); lanes below the matrix skip
-            // their partial stores
-            const bool warp_rows = m0 + q * 32u < p.Mg;
-            const bool lane_row = row < p.Mg;
-            for (uint32_t chunk = 0; warp_rows && chunk < kChunks; ++chunk) {
-                if (chunk - own0 < cps) {
-                    continue;
-                }
-                uint32_t r[32];
-                tmem_ld_32x32(tmem_base + ((q * 32u) << 16) + chunk * 32u, r);
-                tmem_ld_wait();
-                // inside a 4 KiB piece (32 rows x 32 floats) the 16-byte vector v of row `lane` sits at slot
-                // v * 32 + lane: every store instruction of the warp covers 512 contiguous bytes, and the
-                // reader's shared-memory loads are free of bank conflicts
-                float4* dst = reinterpret_cast<float4*>(parts + ks * kPartFloats + ((size_t)chunk * kGemmBlockM + q * 32u) * 32u) + lane;
-#pragma unroll
-                for (uint32_t v = 0; v < 8; ++v) {
-                    if (lane_row) {
-                        dst[v * 32u] = make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]),
-                                                   __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
-                    }
-                }
-            }
-            __syncwarp();  // every lane's partial stores are ordered before lane 0's release
-            uint8_t* red = smem + S::kOffA + q * ((kChunks - 1u) * kPieceBytes);
-            if (warp_rows) {
-                if (lane == 0) {
-                    st_release_gpu(flags + ks * 4u + q, p.splitk_epoch);
-                }
-                // lanes 0 .. ksplit-1 each watch one part's flag (the polls overlap instead of queueing up)
-                bool ok = true;
-                if (lane < ksplit && lane != ks &&
-                    !wait_flag_ge_gpu(flags + lane * 4u + q, p.splitk_epoch, p.timeout_ns, p.status)) {
-                    report_status(p.status, kStatusFlagTimeout, 0x100u + lane, tile, p.splitk_epoch);
-                    ok = false;
-                }
-                alive = __all_sync(0xFFFFFFFFu, ok) && alive;
-                if (lane == 0 && alive) {
-                    mbar_arrive_expect_tx(&red_bar[q], (ksplit - 1u) * cps * kPieceBytes);
-                    fence_proxy_async_all();  // the other parts' generic-proxy stores before this thread's bulk copies
-                    uint32_t slot = 0;
-                    for (uint32_t part = 0; part < ksplit; ++part) {
-                        if (part == ks) {
-                            continue;
-                        }
-                        for (uint32_t oc = 0; oc < cps; ++oc, ++slot) {
-                            bulk_load(red + slot * kPieceBytes,
-                                      parts + part * kPartFloats + ((size_t)(own0 + oc) * kGemmBlockM + q * 32u) * 32u,
-                                      kPieceBytes, &red_bar[q]);
-                        }
-                    }
-                }
-                __syncwarp();
-                alive = mbar_wait_warp(&red_bar[q], 0, p.status, 107, q, bar_ns) && alive;
-                // a part that gave up writes nothing: C keeps what the caller put there
-                for (uint32_t oc = 0; alive && oc < cps; ++oc) {
-                    uint32_t r[32];
-                    tmem_ld_32x32(tmem_base + ((q * 32u) << 16) + (own0 + oc) * 32u, r);
-                    tmem_ld_wait();
-                    for (uint32_t pi = 0; pi + 1u < ksplit; ++pi) {
-                        // four 16-byte loads at a time: enough to hide the shared-memory latency without
-                        // crowding the 32 accumulator registers
-                        const uint32_t src = smem_u32(red + (pi * cps + oc) * kPieceBytes + lane * 16u);
-#pragma unroll
-                        for (uint32_t h = 0; h < 2; ++h) {
-                            float4 f[4];
-#pragma unroll
-                            for (uint32_t v = 0; v < 4; ++v) {
-                                f[v] = ld_shared_v4(src + (h * 4u + v) * 512u);
-                            }
-#pragma unroll
-                            for (uint32_t v = 0; v < 4; ++v) {
-                                const uint32_t e = (h * 4u + v) * 4u;
-                                r[e] = __float_as_uint(__uint_as_float(r[e]) + f[v].x);
-                                r[e + 1] = __float_as_uint(__uint_as_float(r[e + 1]) + f[v].y);
-                                r[e + 2] = __float_as_uint(__uint_as_float(r[e + 2]) + f[v].z);
-                                r[e + 3] = __float_as_uint(__uint_as_float(r[e + 3]) + f[v].w);
-                            }
-                        }
-                    }
-                    store_c_chunk<OutT>(c, p, row, n0 + (own0 + oc) * 32u, r);
-                }
-            }
+            SplitExchange<OutT, kChunks> x;
+            x.part_stride = (size_t)kGemmBlockM * BLOCK_N;
+            x.ws = p.splitk_ws + (size_t)tile * ksplit * x.part_stride;
+            x.flags = p.splitk_flags + (size_t)tile * ksplit * 4u + q;
+            x.flag_stride = 4u;
+            x.red = smem + S::kOffA + q * kSplitRedBytes;
+            x.bar = &red_bar[q];
+            alive = alive && x.run(p, c, tmem_base + ((q * 32u) << 16), ks, ksplit, q, lane, tc.m_tile * kGemmBlockM + q * 32u,
+                                   tc.n_tile * BLOCK_N, tile, bar_ns);
             tcgen05_fence_before();
             if (q == 0 && lane == 0) {
                 CATCCOS_TR_STAMP(p.trace, kTrEpiLast);
             }
         }
         uint32_t ti = 0;
-        bool alive = true;
         for (uint32_t unit = blockIdx.x; alive && ksplit == 1u && unit < num_units; unit += gridDim.x, ++ti) {
             const uint32_t ks = unit / num_tiles;
             const uint32_t tile = unit - ks * num_tiles;
@@ -955,11 +1062,12 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     }
 
     tcgen05_fence_before();
-    __syncthreads();
+    if (__syncthreads_or(alive ? 0 : 1)) {
+        drain_after_abort(p.status);
+    }
     if (threadIdx.x == 0) {
         CATCCOS_TR_STAMP(p.trace, kTrCtaEnd);
     }
-    drain_after_abort(p.status);
     if (p.flags != nullptr) {
         grid_dep_wait();  // a gated launch ends after the quantise kernel it overlaps: the successor waits for this one only
     }

@@ -7,12 +7,28 @@
 // each CTA ends up with the accumulator of its own 128 rows x 256 columns in its own tensor memory.
 // Every CTA loads its own tiles with plain TMA (no cluster multicast anywhere); what crosses the pair is
 // only barrier traffic:
-//   full[s]                     lives in the leader; both CTAs' TMA bytes go there, and the commit behind the
-//                               leader's scale copies (tcgen05.cp.cta_group::2 reads the atoms of both CTAs)
-//   atoms_written[s]            lives in the leader; both CTAs' scale loaders arrive once their atoms are in
-//                               shared memory
+//   full[s]                     lives in the leader; both CTAs' TMA bytes go there
 //   empty[s], tmem_full[a]      live in each CTA; the leader's tcgen05.commit arrives on both copies
 //   tmem_empty[a], overlap_free[a]  live in the leader; the epilogue warps of both CTAs arrive there
+//   atoms[b], sf_full[b]        live in the leader, sf_empty[b] in each CTA: see below
+//
+// Two rings.  The round trip of a stage (commit, empty, TMA, full, MMA) takes about 3000 cycles on a loaded GPU
+// against 512 cycles of MMA per K tile, so the operand ring is as deep as shared memory allows and carries
+// nothing but TMA.  The scale factors have a ring of their own that moves in groups of four K tiles: the scale-loader
+// warps load the E8M0 bytes one group ahead into registers, write the atoms, and the leader's lane 0 of every warp
+// copies one K tile's atoms of both CTAs into tensor memory; two groups are in flight.
+//
+// What bounds it: a K tile moves 32 KB into and 32 KB out of each SM's shared memory (500 of the 512 MMA cycles) and
+// 64 B per cycle and SM out of L2, so both are close to their limits when the tensor pipe is; long launches are held by
+// the power cap instead.  Pairs on 256 x 128 tiles (48 KB per 256 MMA cycles) were measured 1.4 to 1.6 times slower.
+// Measured (B200, 3 operand sets in turn, kernel alone): 1024 x 2304 x 7168 25.7 -> 21.2 us, 3001 x 2064 x 5120
+// 41.3 -> 33.3, 4096 x 3456 x 5120 66.5 -> 58.9, 8192 x 2304 x 7168 105 -> 99, 32768 x 3456 x 5120 450 -> 428 us
+// against one ring of five stages that also carried the scales, no split, and stores straight from registers.
+//
+// Work units.  num_tiles = rounds * pairs + rem: every pair takes `rounds` whole tiles, then the rem tiles that
+// would leave pairs idle are cut into ksplit parts along K, one (tile, part) per pair.  The parts exchange fp32 pieces
+// through the rank's split-K scratch: every part owns an equal share of the tile's 32-column chunks and adds the other
+// parts' pieces in ascending part order, so the result does not depend on timing.
 #pragma once
 
 #include "mx_gemm.cuh"
@@ -21,30 +37,35 @@ namespace catccos {
 
 constexpr uint32_t kPairBlockM = 256;
 constexpr uint32_t kPairBlockN = 256;
+constexpr uint32_t kSfGroup = 4;  // K tiles whose scale factors travel together (one per scale-loader warp)
 
 struct PairSmem {
-    static constexpr uint32_t kStages = 5;
+    static constexpr uint32_t kStages = 6;
     static constexpr uint32_t kABytes = 128 * kGemmBlockK;  // this CTA's 128 rows
     static constexpr uint32_t kBBytes = 128 * kGemmBlockK;  // this CTA's 128 columns
-    static constexpr uint32_t kSfaBytes = 512;
+    static constexpr uint32_t kSfaBytes = 512;              // per K tile
     static constexpr uint32_t kSfbBytes = 1024;  // all 256 columns: each CTA multiplies by the whole N tile
+    static constexpr uint32_t kSfBufBytes = kSfGroup * (kSfaBytes + kSfbBytes);
     static constexpr uint32_t kOffA = 0;
     static constexpr uint32_t kOffB = kOffA + kStages * kABytes;
-    static constexpr uint32_t kOffSfa = kOffB + kStages * kBBytes;
-    static constexpr uint32_t kOffSfb = kOffSfa + kStages * kSfaBytes;
-    static constexpr uint32_t kOffBar = kOffSfb + kStages * kSfbBytes;
-    // full[S], empty[S], tmem_full[2], tmem_empty[2], overlap_free[2], atoms_written[S] (leader only: both
-    // CTAs' scale loaders have put a stage's atoms into shared memory)
-    static constexpr uint32_t kNumBars = 3 * kStages + 6;
+    static constexpr uint32_t kOffOut = kOffB + kStages * kBBytes;
+    static constexpr uint32_t kOffSf = kOffOut + 4 * kOutStageBytes;
+    static constexpr uint32_t kOffBar = kOffSf + 2 * kSfBufBytes;
+    // full[S], empty[S], tmem_full[2], tmem_empty[2], overlap_free[2], sf_full[2], sf_empty[2], atoms[2], red[4]
+    static constexpr uint32_t kNumBars = 2 * kStages + 12 + 4;
     static constexpr uint32_t kOffTmemPtr = kOffBar + kNumBars * 8;
     static constexpr uint32_t kOffGate = kOffTmemPtr + 8;  // K-tile iterations whose rows this CTA's producer has seen ready
     static constexpr uint32_t kBytes = kOffTmemPtr + 16;
     static constexpr uint32_t kDynamicBytes = kBytes + 1024;
-    static constexpr uint32_t kOverlapChunks = 2;
-    static constexpr uint32_t kAccCol1 = 192;  // the two accumulators share columns 192..255 (see mx_gemm.cuh)
-    static constexpr uint32_t kSfCol = 448;    // one scale-factor set of 12 columns per stage
+    static_assert(kDynamicBytes <= 232448, "one CTA's shared memory");
+    static_assert(4 * kSplitRedBytes <= kOffOut, "the split-K pieces land in the idle operand stages");
+    // Tensor memory: two 256-column accumulators that share 96 columns (the epilogue drains those first and then lets
+    // the next tile start), and two groups of four scale sets (SFA 4 + SFB 8 columns).
+    static constexpr uint32_t kAccCol1 = 160;
+    static constexpr uint32_t kSfCol = 416;
     static constexpr uint32_t kSfSetCols = 12;
-    static_assert(kSfCol + kStages * kSfSetCols <= 512, "scale-factor sets must fit in tensor memory");
+    static constexpr uint32_t kSfGroupCols = kSfGroup * kSfSetCols;
+    static_assert(kAccCol1 + 256 <= kSfCol && kSfCol + 2 * kSfGroupCols <= 512, "tensor memory columns");
 };
 
 // Tile order for pairs: as tile_coord, with 256-row tiles.
@@ -64,9 +85,60 @@ __host__ __device__ __forceinline__ TileCoord pair_tile_coord(uint32_t idx, uint
     return t;
 }
 
+// One work unit of a pair: a whole tile, or one K part of a tile of the last round.
+struct PairUnit {
+    uint32_t m0, n0, n_tile;  // first row and column of the pair's tile
+    uint32_t kt0, kt1;        // K tiles
+    uint32_t part, rem_ix;    // split units: which part, and which of the rem tiles
+    bool split;
+};
+
+struct PairWork {
+    uint32_t m_tiles, n_tiles, num_tiles, k_tiles, pair, num_pairs, rounds, rem, ksplit, units;
+
+    __host__ __device__ __forceinline__ PairWork(const GemmParams& p, uint32_t pair_, uint32_t num_pairs_)
+    {
+        m_tiles = (p.Mg + kPairBlockM - 1) / kPairBlockM;
+        n_tiles = (p.N + kPairBlockN - 1) / kPairBlockN;
+        num_tiles = m_tiles * n_tiles;
+        k_tiles = p.K / kGemmBlockK;
+        pair = pair_;
+        num_pairs = num_pairs_;
+        ksplit = p.ksplit > 1u ? p.ksplit : 1u;
+        // a grid of exactly num_tiles * ksplit pairs splits every tile
+        rounds = ksplit > 1u && num_tiles * ksplit == num_pairs ? 0u : num_tiles / num_pairs;
+        rem = num_tiles - rounds * num_pairs;
+        units = p.gemm_off ? 0u : rounds + (pair < rem * ksplit ? 1u : 0u);
+    }
+
+    __host__ __device__ __forceinline__ PairUnit unit(uint32_t i, const GemmParams& p) const
+    {
+        PairUnit u;
+        uint32_t tile = pair + i * num_pairs;
+        u.part = 0;
+        u.rem_ix = 0;
+        u.kt0 = 0;
+        u.kt1 = k_tiles;
+        u.split = i >= rounds && ksplit > 1u;
+        if (u.split) {
+            u.part = pair / rem;
+            u.rem_ix = pair - u.part * rem;
+            tile = rounds * num_pairs + u.rem_ix;
+            u.kt0 = u.part * k_tiles / ksplit;
+            u.kt1 = (u.part + 1u) * k_tiles / ksplit;
+        }
+        const TileCoord tc = pair_tile_coord(tile, n_tiles, m_tiles, p);
+        u.m0 = tc.m_tile * kPairBlockM;
+        u.n0 = tc.n_tile * kPairBlockN;
+        u.n_tile = tc.n_tile;
+        return u;
+    }
+};
+
 template <typename OutT, bool FUSED_QUANT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FUSED_QUANT ? kGemmFusedThreads : kGemmThreads, 1)
-mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, GemmParams p)
+mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                    const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ GemmParams p)
 {
     using S = PairSmem;
     constexpr uint32_t kStages = S::kStages;
@@ -76,11 +148,14 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::kOffBar);
     uint64_t* full = bars;
-    uint64_t* empty = bars + kStages;
-    uint64_t* tmem_full = bars + 2 * kStages;
+    uint64_t* empty = full + kStages;
+    uint64_t* tmem_full = empty + kStages;
     uint64_t* tmem_empty = tmem_full + 2;
     uint64_t* overlap_free = tmem_empty + 2;
-    uint64_t* atoms_written = overlap_free + 2;
+    uint64_t* sf_full = overlap_free + 2;
+    uint64_t* sf_empty = sf_full + 2;
+    uint64_t* atoms = sf_empty + 2;
+    uint64_t* red_bar = atoms + 2;
     uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem + S::kOffTmemPtr);
     uint32_t* gate = reinterpret_cast<uint32_t*>(smem + S::kOffGate);
     uint32_t* push_turn = gate + 1;  // the pushers of this CTA store one after the other (mx_quant.cuh, push_worker)
@@ -89,41 +164,44 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t cta = cluster_ctarank();  // 0 = leader
     const uint64_t bar_ns = p.bar_timeout_ns;
-    const uint32_t pair = blockIdx.x >> 1;
-    const uint32_t num_pairs = gridDim.x >> 1;
-
-    const uint32_t m_tiles = (p.Mg + kPairBlockM - 1) / kPairBlockM;
-    const uint32_t n_tiles = (p.N + kPairBlockN - 1) / kPairBlockN;
-    const uint32_t num_tiles = p.gemm_off ? 0u : m_tiles * n_tiles;
-    const uint32_t k_tiles = p.K / kGemmBlockK;
+    const PairWork work(p, blockIdx.x >> 1, gridDim.x >> 1);
 
     if (threadIdx.x == 0) {
         CATCCOS_TR_STAMP(p.trace, kTrCtaStart);
         *gate = 0u;
         *push_turn = 0u;
         for (uint32_t s = 0; s < kStages; ++s) {
-            mbar_init(&full[s], 3);  // both CTAs' producers (expect_tx) and the commit behind the scale copies
+            mbar_init(&full[s], 2);  // both CTAs' producers (expect_tx)
             mbar_init(&empty[s], 1);
-            mbar_init(&atoms_written[s], 2);  // one scale-loader warp in each CTA
         }
         for (uint32_t a = 0; a < 2; ++a) {
             mbar_init(&tmem_full[a], 1);
             mbar_init(&tmem_empty[a], 8);    // four epilogue warps in each CTA
             mbar_init(&overlap_free[a], 8);
+            mbar_init(&sf_full[a], kSfGroup);  // one commit behind each K tile's copies
+            mbar_init(&sf_empty[a], 1);
+            mbar_init(&atoms[a], 8);           // four scale-loader warps in each CTA
+        }
+        for (uint32_t w = 0; w < 4; ++w) {
+            mbar_init(&red_bar[w], 1);
         }
         mbar_fence_init();
-        tma_prefetch_desc(&tmap_a);
-        tma_prefetch_desc(&tmap_b);
     }
     if (warp == 5) {
         tmem_alloc_pair(tmem_ptr_smem, kTmemCols);
         tmem_relinquish_pair();
+    }
+    if (warp == 4 && lane == 0) {
+        tma_prefetch_desc(&tmap_a);
+        tma_prefetch_desc(&tmap_b);
+        tma_prefetch_desc(&tmap_c);
     }
     tcgen05_fence_before();
     __syncthreads();
     cluster_sync_all();  // both CTAs' barriers exist before anybody arrives on the other's
     tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_ptr_smem;
+    bool alive = true;  // false once a wait of this role has given up
 
     if (threadIdx.x == 0) {
         CATCCOS_TR_STAMP(p.trace, kTrSetupDone);
@@ -131,26 +209,45 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 
     if (warp == 4) {
         // ------------------------------- TMA producer (both CTAs) -------------------------
-        if (p.flags == nullptr) {
-            grid_dep_wait();  // A is the output of the kernel launched just before (no-op for a plain launch);
-        }                     // with flags, the flags say when its rows are there
-        uint32_t it = 0, ti = 0;
-        bool alive = true;
+        uint32_t it = 0;
         // packed 4-bit operands arrive as half the bytes they occupy in shared memory (the gaps are not written)
         const uint32_t tx_bytes = (p.a_fmt == 5u ? S::kABytes / 2u : S::kABytes) + (p.b_fmt == 5u ? S::kBBytes / 2u : S::kBBytes);
-        for (uint32_t tile = pair; alive && tile < num_tiles; tile += num_pairs, ++ti) {
-            TileCoord tc = pair_tile_coord(tile, n_tiles, m_tiles, p);
-            const uint32_t m0 = tc.m_tile * kPairBlockM + cta * 128u;
-            const uint32_t n0 = tc.n_tile * kPairBlockN + cta * 128u;
-            uint32_t ready_end = 0;  // K tiles below this index are known to be there
-            for (uint32_t kt = 0; alive && kt < k_tiles; ++kt, ++it) {
+        auto load_b = [&](const PairUnit& u, uint32_t kt, uint32_t s, uint32_t leader_bar) {
+            const int32_t n = (int32_t)(u.n0 + cta * 128u), k = (int32_t)(kt * kGemmBlockK);
+            if (p.b_kmajor) {  // the transposed copy [N, K]: this CTA's columns are rows of it
+                tma_load_2d_pair(smem + S::kOffB + s * S::kBBytes, &tmap_b, leader_bar, k, n);
+            } else {
+                tma_load_2d_pair(smem + S::kOffB + s * S::kBBytes, &tmap_b, leader_bar, n, k);
+            }
+        };
+        uint32_t early = 0;  // iterations whose B tile is already on its way
+        if (p.flags == nullptr) {
+            if (p.b_early && work.units > 0u) {
+                // the weights do not come from the kernel launched just before: fill the ring's B half meanwhile
+                const PairUnit u = work.unit(0, p);
+                early = min(kStages, u.kt1 - u.kt0);
+                if (lane == 0) {
+                    for (uint32_t s = 0; s < early; ++s) {
+                        const uint32_t leader_bar = map_to_cta(smem_u32(&full[s]), 0);
+                        mbar_arrive_expect_tx_cluster(leader_bar, tx_bytes);
+                        load_b(u, u.kt0 + s, s, leader_bar);
+                    }
+                }
+            }
+            grid_dep_wait();  // A is the output of the kernel launched just before (no-op for a plain launch);
+        }                     // with flags, the flags say when its rows are there
+        for (uint32_t ui = 0; alive && ui < work.units; ++ui) {
+            const PairUnit u = work.unit(ui, p);
+            const uint32_t m0 = u.m0 + cta * 128u;
+            uint32_t ready_end = u.kt0;  // K tiles below this index are known to be there
+            for (uint32_t kt = u.kt0; alive && kt < u.kt1; ++kt, ++it) {
                 if (p.flags != nullptr && kt >= ready_end) {
                     const unsigned long long t0 = CATCCOS_TR_NOW();
                     (void)t0;
                     const uint32_t seg0 = kt / p.seg_ktiles;
                     const uint32_t nready = wait_rows_ready(p, m0, lane, seg0);
                     alive = nready != 0u;
-                    ready_end = min((seg0 + nready) * p.seg_ktiles, k_tiles);
+                    ready_end = min((seg0 + nready) * p.seg_ktiles, u.kt1);
                     fence_proxy_async_all();
                     if (lane == 0) {
                         st_release_cta_shared(gate, it + (ready_end - kt));
@@ -159,25 +256,22 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 }
                 if (lane == 0 && alive) {
                     const uint32_t s = it % kStages;
-                    const uint32_t ph = (it / kStages) & 1u;
-                    const unsigned long long t1 = CATCCOS_TR_NOW();
-                    (void)t1;
-                    alive = mbar_wait_cluster(&empty[s], ph ^ 1u, p.status, 200, s, bar_ns);
-                    CATCCOS_TR_ADD(p.trace, kTrProdEmptyWaitNs, CATCCOS_TR_NOW() - t1);
-                    if (kt == 0 && ti < kTraceTiles) {
-                        CATCCOS_TR_STAMP(p.trace, kTrTileStart + ti);
+                    const uint32_t leader_bar = map_to_cta(smem_u32(&full[s]), 0);
+                    if (it >= early) {
+                        const unsigned long long t1 = CATCCOS_TR_NOW();
+                        (void)t1;
+                        alive = mbar_wait_cluster(&empty[s], ((it / kStages) & 1u) ^ 1u, p.status, 200, s, bar_ns);
+                        CATCCOS_TR_ADD(p.trace, kTrProdEmptyWaitNs, CATCCOS_TR_NOW() - t1);
+                        mbar_arrive_expect_tx_cluster(leader_bar, tx_bytes);
+                    }
+                    if (kt == u.kt0 && ui < kTraceTiles) {
+                        CATCCOS_TR_STAMP(p.trace, kTrTileStart + ui);
                     }
                     CATCCOS_TR_STAMP_FIRST(p.trace, kTrProdFirstTma);
-                    const uint32_t leader_bar = map_to_cta(smem_u32(&full[s]), 0);
-                    mbar_arrive_expect_tx_cluster(leader_bar, tx_bytes);
                     tma_load_2d_pair(smem + S::kOffA + s * S::kABytes, &tmap_a, leader_bar, (int32_t)(kt * kGemmBlockK),
                                      (int32_t)m0);
-                    if (p.b_kmajor) {  // the transposed copy [N, K]: this CTA's 128 columns are 128 rows of it
-                        tma_load_2d_pair(smem + S::kOffB + s * S::kBBytes, &tmap_b, leader_bar, (int32_t)(kt * kGemmBlockK),
-                                         (int32_t)n0);
-                    } else {
-                        tma_load_2d_pair(smem + S::kOffB + s * S::kBBytes, &tmap_b, leader_bar, (int32_t)n0,
-                                         (int32_t)(kt * kGemmBlockK));
+                    if (it >= early) {
+                        load_b(u, kt, s, leader_bar);
                     }
                     CATCCOS_TR_STAMP(p.trace, kTrProdLastTma);
                 }
@@ -186,78 +280,84 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         }
     } else if (warp == 5) {
         // ------------------------------- MMA issuer (leader CTA only) ---------------------
-        // As in the single-CTA kernel the issuer issues the MMAs and the stage-releasing commit, nothing else.
-        if (cta == 0 && lane == 0) {
+        // The whole warp runs the loop and one elected lane issues: inside a branch on the lane the operands of a tcgen05
+        // instruction cannot stay in uniform registers, and each then takes about 70 cycles to get out.  The issuer
+        // issues the MMAs and the commits, nothing else.
+        if (cta == 0) {
             const bool bk = p.b_kmajor != 0u;
             const uint32_t idesc = make_idesc_mxf8(kPairBlockM, kPairBlockN, !bk) | ((p.a_fmt & 7u) << 7) |
                                    ((p.b_fmt & 7u) << 10);  // operand formats: E4M3 = 0, E5M2 = 1, E2M1 = 5
-            const uint32_t my_tiles = (num_tiles > pair) ? (num_tiles - pair + num_pairs - 1) / num_pairs : 0u;
-            const uint32_t total_it = my_tiles * k_tiles;
-
             const uint32_t hi_a = (uint32_t)(make_smem_desc(0, 16, 1024, 2) >> 32);
-            const uint32_t hi_b = bk ? hi_a : (uint32_t)(make_smem_desc(0, 16384, 1024, 2) >> 32);
+            // B, MN-major: each CTA's 128 columns are one 128-byte swizzle row per K row
+            const uint64_t desc_b = bk ? make_smem_desc(0, 16, 1024, 2) : make_smem_desc(0, 16384, 1024, 2);
+            const uint32_t hi_b = (uint32_t)(desc_b >> 32);
             const uint32_t a_lo0 = (uint32_t)make_smem_desc(0, 16, 1024, 2) | (smem_u32(smem + S::kOffA) >> 4);
-            // each CTA holds 128 columns of B (one 128-byte swizzle row per K): MN-major
-            const uint32_t b_lo0 = (uint32_t)make_smem_desc(0, bk ? 16 : 16384, 1024, 2) | (smem_u32(smem + S::kOffB) >> 4);
+            const uint32_t b_lo0 = (uint32_t)desc_b | (smem_u32(smem + S::kOffB) >> 4);
             const uint32_t kb_step_b = (bk ? 32u : 4096u) >> 4;
-            const uint32_t sf_tmem0 = tmem_base + S::kSfCol;
-
-            bool alive = true;
-            auto stage_wait = [&](uint32_t s, uint32_t ph) {
-                const unsigned long long t0 = CATCCOS_TR_NOW();
-                (void)t0;
-                alive = mbar_wait_cluster(&full[s], ph, p.status, 203, s, bar_ns);
-                tcgen05_fence_after();
-                CATCCOS_TR_ADD(p.trace, kTrMmaFullWaitNs, CATCCOS_TR_NOW() - t0);
-            };
-            auto issue_mma = [&](uint32_t a_lo, uint32_t b_lo, uint32_t sf, uint32_t kb, uint32_t d_col, uint32_t accumulate) {
-                umma_mxf8_pair_lohi(d_col, a_lo + kb * (32u >> 4), hi_a, b_lo + kb * kb_step_b, hi_b,
-                                    idesc_with_sf_id(idesc, kb), sf, sf + 4, accumulate);
-            };
-
-            if (total_it > 0) {
-                stage_wait(0, 0);
-            }
-            uint32_t it = 0, s = 0, ph = 0;
-            for (uint32_t ti = 0; alive && ti < my_tiles; ++ti) {
-                const uint32_t acc = ti & 1u;
-                const uint32_t acc_ph = (ti >> 1) & 1u;
+            uint32_t s = 0, ph = 0;   // operand stage and its phase
+            uint32_t group = 0;       // scale groups consumed
+            for (uint32_t ui = 0; alive && ui < work.units; ++ui) {
+                const PairUnit u = work.unit(ui, p);
+                const uint32_t acc = ui & 1u;
+                const uint32_t acc_ph = (ui >> 1) & 1u;
                 const uint32_t d_col = tmem_base + (acc ? S::kAccCol1 : 0u);
                 const unsigned long long t0 = CATCCOS_TR_NOW();
                 (void)t0;
-                alive = mbar_wait_cluster(&tmem_empty[acc], acc_ph ^ 1u, p.status, 201, acc, bar_ns);
-                if (ti > 0 && alive) {
-                    alive = mbar_wait_cluster(&overlap_free[acc ^ 1u], ((ti - 1) >> 1) & 1u, p.status, 202, acc, bar_ns);
+                alive = mbar_wait_warp(&tmem_empty[acc], acc_ph ^ 1u, p.status, 201, acc, bar_ns);
+                if (ui > 0 && alive) {
+                    alive = mbar_wait_warp(&overlap_free[acc ^ 1u], ((ui - 1) >> 1) & 1u, p.status, 202, acc, bar_ns);
                 }
-                CATCCOS_TR_ADD(p.trace, kTrMmaAccWaitNs, CATCCOS_TR_NOW() - t0);
-                tcgen05_fence_after();
-                CATCCOS_TR_STAMP_FIRST(p.trace, kTrMmaFirst);
-                for (uint32_t kt = 0; alive && kt < k_tiles; ++kt, ++it) {
+                if (lane == 0) {
+                    CATCCOS_TR_ADD(p.trace, kTrMmaAccWaitNs, CATCCOS_TR_NOW() - t0);
+                }
+                const uint32_t n_it = u.kt1 - u.kt0;
+                for (uint32_t i = 0; alive && i < n_it; ++i) {
+                    const uint32_t buf = group & 1u;
+                    const unsigned long long t1 = CATCCOS_TR_NOW();
+                    (void)t1;
+                    if (i % kSfGroup == 0u) {
+                        alive = mbar_wait_warp(&sf_full[buf], (group >> 1) & 1u, p.status, 207, buf, bar_ns);
+                    }
+                    alive = alive && mbar_wait_warp(&full[s], ph, p.status, 203, s, bar_ns);
+                    if (!alive) {
+                        break;  // nothing is issued, and the accumulator never reported, after a wait has given up
+                    }
+                    tcgen05_fence_after();
+                    if (lane == 0) {
+                        CATCCOS_TR_ADD(p.trace, kTrMmaFullWaitNs, CATCCOS_TR_NOW() - t1);
+                        CATCCOS_TR_STAMP_FIRST(p.trace, kTrMmaFirst);
+                    }
                     const uint32_t a_lo = a_lo0 + s * (S::kABytes >> 4);
                     const uint32_t b_lo = b_lo0 + s * (S::kBBytes >> 4);
-                    const uint32_t sf = sf_tmem0 + s * S::kSfSetCols;
-                    const uint32_t s_next = (s + 1 == kStages) ? 0u : s + 1;
-                    const uint32_t ph_next = ph ^ (s_next == 0u ? 1u : 0u);
-                    const bool more = it + 1 < total_it;
-                    issue_mma(a_lo, b_lo, sf, 0, d_col, kt != 0 ? 1u : 0u);
-                    issue_mma(a_lo, b_lo, sf, 1, d_col, 1u);
-                    issue_mma(a_lo, b_lo, sf, 2, d_col, 1u);
-                    issue_mma(a_lo, b_lo, sf, 3, d_col, 1u);
-                    tcgen05_commit_pair(&empty[s], 3);
-                    if (more) {
-                        stage_wait(s_next, ph_next);
+                    const uint32_t sf = tmem_base + S::kSfCol + buf * S::kSfGroupCols + (i % kSfGroup) * S::kSfSetCols;
+                    const bool group_end = i % kSfGroup == kSfGroup - 1u || i + 1u == n_it;
+                    if (elect_one()) {
+#pragma unroll
+                        for (uint32_t kb = 0; kb < 4; ++kb) {
+                            umma_mxf8_pair_lohi(d_col, a_lo + kb * (32u >> 4), hi_a, b_lo + kb * kb_step_b, hi_b,
+                                                idesc_with_sf_id(idesc, kb), sf, sf + 4, (kb != 0u || i != 0u) ? 1u : 0u);
+                        }
+                        tcgen05_commit_pair(&empty[s], 3);
+                        if (group_end) {
+                            tcgen05_commit_pair(&sf_empty[buf], 3);
+                        }
+                        if (i + 1u == n_it) {
+                            tcgen05_commit_pair(&tmem_full[acc], 3);
+                        }
                     }
-                    s = s_next;
-                    ph = ph_next;
+                    __syncwarp();
+                    group += group_end ? 1u : 0u;
+                    s = (s + 1 == kStages) ? 0u : s + 1;
+                    ph ^= s == 0u ? 1u : 0u;
                 }
-                tcgen05_commit_pair(&tmem_full[acc], 3);
-                if (ti < kTraceTiles) {
-                    CATCCOS_TR_STAMP(p.trace, kTrTileEnd + ti);
+                if (lane == 0) {
+                    if (ui < kTraceTiles) {
+                        CATCCOS_TR_STAMP(p.trace, kTrTileEnd + ui);
+                    }
+                    CATCCOS_TR_STAMP(p.trace, kTrMmaLast);
                 }
-                CATCCOS_TR_STAMP(p.trace, kTrMmaLast);
             }
         }
-        __syncwarp();
     } else if (FUSED_QUANT && warp >= 10) {
         // ------------------------------- quantise-and-push producer -----------------------
         // Of the fourteen extra warps, eight quantise this rank's shard into the local stage (warps 10-19
@@ -273,85 +373,125 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         }
     } else if (warp >= 6) {
         // ------------------------------- scale loaders (both CTAs) ------------------------
-        // A scales of this CTA's 128 rows; B scales of all 256 columns of the pair's tile.
+        // Warp j loads the A scales of this CTA's rows [32 j, +32) for all four K tiles of a group (16 bytes per row) and
+        // the B scales of all columns of the pair's tile for K tile j.
         constexpr uint32_t kNB = kPairBlockN / 32;
         const uint32_t j = warp - 6;
-        if (p.flags == nullptr) {
-            grid_dep_wait();  // the A scales are the output of the kernel launched just before (or: see the flags)
-        }
         const uint32_t sf_row_bytes = p.K / 32;
-        const uint32_t my_tiles = (num_tiles > pair) ? (num_tiles - pair + num_pairs - 1) / num_pairs : 0u;
-        const uint32_t total_it = my_tiles * k_tiles;
-        uint32_t cur_a[4], cur_lo[kNB], cur_hi[kNB];
-        uint32_t nxt_a[4], nxt_lo[kNB], nxt_hi[kNB];
+        const bool a_wide = p.K % 512u == 0u && ((uintptr_t)p.a_scales & 15u) == 0u;
+        uint32_t cur_lo[kNB], cur_hi[kNB], nxt_lo[kNB], nxt_hi[kNB];
+        uint4 cur_a, nxt_a;
         uint32_t known_end = 0;  // K-tile iterations below this index have their rows in place
-        bool alive = true;
 
-        auto issue_loads = [&](uint32_t it, uint32_t (&ra)[4], uint32_t (&rlo)[kNB], uint32_t (&rhi)[kNB]) {
-            const uint32_t seq = it / k_tiles;
-            const uint32_t kt = it - seq * k_tiles;
-            TileCoord tc = pair_tile_coord(pair + seq * num_pairs, n_tiles, m_tiles, p);
-            const uint32_t m0 = tc.m_tile * kPairBlockM + cta * 128u;
-            const uint32_t n0 = tc.n_tile * kPairBlockN;
-            if (p.flags != nullptr && it >= known_end) {
+        // where this warp is: unit ui, first K tile of the group, running index of that K tile
+        struct Cursor {
+            uint32_t ui, kt, it;
+            PairUnit u;
+        };
+        auto next = [&](Cursor& c) {
+            c.kt += kSfGroup;
+            c.it += kSfGroup;
+            if (c.kt >= c.u.kt1) {
+                c.it -= c.kt - c.u.kt1;
+                if (++c.ui < work.units) {
+                    c.u = work.unit(c.ui, p);
+                    c.kt = c.u.kt0;
+                }
+            }
+        };
+        auto load_b = [&](const Cursor& c, uint32_t (&rlo)[kNB], uint32_t (&rhi)[kNB]) {
+            const uint32_t kt = c.kt + j;
+#pragma unroll
+            for (uint32_t i = 0; i < kNB; ++i) {
+                const uint32_t n = c.u.n0 + i * 32 + lane;
+                rlo[i] = 0x7F7Fu;
+                rhi[i] = 0x7F7Fu;
+                if (n < p.N && kt < c.u.kt1) {
+                    rlo[i] = __ldcg(reinterpret_cast<const uint16_t*>(p.b_scales + ((size_t)(2 * kt) * p.N + n) * 2));
+                    rhi[i] = __ldcg(reinterpret_cast<const uint16_t*>(p.b_scales + ((size_t)(2 * kt + 1) * p.N + n) * 2));
+                }
+            }
+        };
+        auto load_a = [&](const Cursor& c, uint4& ra) {
+            const uint32_t m0 = c.u.m0 + cta * 128u;
+            const uint32_t last = min(c.kt + kSfGroup, c.u.kt1);  // K tiles [c.kt, last) of the group exist
+            while (p.flags != nullptr && alive && c.it + (last - c.kt) > known_end) {
                 // this CTA's producer has usually seen these rows' flags already and said so in shared memory
                 // one lane reads the word for the warp: the producer may be updating it, and the branch below holds
                 // warp-wide operations, so every lane has to take the same side
                 const uint32_t g = __shfl_sync(0xFFFFFFFFu, ld_acquire_cta_shared(gate), 0);
-                if (g > it) {
+                if (g >= c.it + (last - c.kt)) {
                     known_end = g;
                 } else {
                     const unsigned long long t0 = CATCCOS_TR_NOW();
                     (void)t0;
+                    // the first K tile of the group that is not known to be there
+                    const uint32_t kt = max(known_end, c.it) - c.it + c.kt;
                     const uint32_t seg0 = kt / p.seg_ktiles;
                     const uint32_t nready = wait_rows_ready(p, m0, lane, seg0);
-                    alive = alive && nready != 0u;
-                    known_end = it + (min((seg0 + nready) * p.seg_ktiles, k_tiles) - kt);
+                    alive = nready != 0u;
+                    known_end = c.it + (min((seg0 + nready) * p.seg_ktiles, c.u.kt1) - c.kt);
                     if (lane == 0) {
                         CATCCOS_TR_ADD(p.trace, kTrSfGateWaitNs + j, CATCCOS_TR_NOW() - t0);
                     }
                 }
             }
-#pragma unroll
-            for (uint32_t i = 0; i < 4; ++i) {
-                const uint32_t row = m0 + i * 32 + lane;
-                ra[i] = 0x7F7F7F7Fu;
-                if (row < p.Mg) {
-                    ra[i] = __ldcg(reinterpret_cast<const uint32_t*>(p.a_scales + (size_t)row * sf_row_bytes + kt * 4u));
-                }
-            }
-#pragma unroll
-            for (uint32_t i = 0; i < kNB; ++i) {
-                const uint32_t n = n0 + i * 32 + lane;
-                rlo[i] = 0x7F7Fu;
-                rhi[i] = 0x7F7Fu;
-                if (n < p.N) {
-                    rlo[i] = __ldg(reinterpret_cast<const uint16_t*>(p.b_scales + ((size_t)(2 * kt) * p.N + n) * 2));
-                    rhi[i] = __ldg(reinterpret_cast<const uint16_t*>(p.b_scales + ((size_t)(2 * kt + 1) * p.N + n) * 2));
+            const uint32_t row = m0 + j * 32 + lane;
+            ra = make_uint4(0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu);
+            if (row < p.Mg) {
+                const uint32_t* src = reinterpret_cast<const uint32_t*>(p.a_scales + (size_t)row * sf_row_bytes) + c.kt;
+                if (a_wide && c.kt % kSfGroup == 0u) {
+                    ra = __ldcg(reinterpret_cast<const uint4*>(src));  // K % 512 == 0: the four K tiles are in the row
+                } else {
+                    ra.x = __ldcg(src);
+                    ra.y = c.kt + 1u < last ? __ldcg(src + 1) : ra.y;
+                    ra.z = c.kt + 2u < last ? __ldcg(src + 2) : ra.z;
+                    ra.w = c.kt + 3u < last ? __ldcg(src + 3) : ra.w;
                 }
             }
         };
 
-        uint32_t it = j;
-        if (it < total_it) {
-            issue_loads(it, cur_a, cur_lo, cur_hi);
-        }
-        for (; alive && it < total_it; it += kSfWarps) {
-            const bool has_next = it + kSfWarps < total_it;
-            if (has_next) {
-                issue_loads(it + kSfWarps, nxt_a, nxt_lo, nxt_hi);
+        Cursor c;
+        c.ui = 0;
+        c.it = 0;
+        c.kt = 0;
+        if (work.units > 0u) {
+            c.u = work.unit(0, p);
+            c.kt = c.u.kt0;
+            if (p.flags == nullptr && !p.b_early) {
+                grid_dep_wait();
             }
-            const uint32_t s = it % kStages;
-            const uint32_t ph = (it / kStages) & 1u;
+            load_b(c, cur_lo, cur_hi);
+            if (p.flags == nullptr && p.b_early) {
+                grid_dep_wait();  // only the A scales are the output of the kernel launched just before
+            }
+            load_a(c, cur_a);
+        }
+        uint32_t group = 0;
+        while (alive && c.ui < work.units) {
+            const bool real = c.kt + j < c.u.kt1;  // the last group of a unit may be short
+            next(c);
+            if (c.ui < work.units) {
+                load_b(c, nxt_lo, nxt_hi);
+                load_a(c, nxt_a);
+            }
+            const uint32_t buf = group & 1u, ph = (group >> 1) & 1u;
             const unsigned long long t1 = CATCCOS_TR_NOW();
             (void)t1;
-            alive = mbar_wait_warp(&empty[s], ph ^ 1u, p.status, 205, s, bar_ns) && alive;
+            alive = mbar_wait_warp(&sf_empty[buf], ph ^ 1u, p.status, 205, buf, bar_ns) && alive;
             if (lane == 0) {
                 CATCCOS_TR_ADD(p.trace, kTrSfEmptyWaitNs + j, CATCCOS_TR_NOW() - t1);
             }
-            uint8_t* sfa = smem + S::kOffSfa + s * S::kSfaBytes;
-            uint8_t* sfb = smem + S::kOffSfb + s * S::kSfbBytes;
-            *reinterpret_cast<uint4*>(sfa + lane * 16u) = make_uint4(cur_a[0], cur_a[1], cur_a[2], cur_a[3]);
+            uint8_t* sfa = smem + S::kOffSf + buf * S::kSfBufBytes;
+            uint8_t* sfb = sfa + kSfGroup * S::kSfaBytes + j * S::kSfbBytes;
+            {
+                // an atom row holds the words of tile rows lane, lane + 32, lane + 64, lane + 96: this warp's is word j
+                uint32_t* dst = reinterpret_cast<uint32_t*>(sfa + lane * 16u) + j;
+                dst[0] = cur_a.x;
+                dst[S::kSfaBytes / 4] = cur_a.y;
+                dst[2 * S::kSfaBytes / 4] = cur_a.z;
+                dst[3 * S::kSfaBytes / 4] = cur_a.w;
+            }
 #pragma unroll
             for (uint32_t h = 0; h < kNB / 4; ++h) {
                 uint4 v;
@@ -364,30 +504,32 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             fence_proxy_async_shared();
             __syncwarp();
             if (lane == 0) {
-                // Both CTAs report their atoms to the leader; the leader's scale loader then copies both CTAs'
-                // atoms into both CTAs' tensor memory (one cta_group::2 copy does the same offsets in the two) and
-                // its commit is the third arrival on the leader's full barrier.  The MMA issuer copies nothing:
-                // a thread gets a tcgen05 instruction out only every ~70 cycles.
-                mbar_arrive_cluster(map_to_cta(smem_u32(&atoms_written[s]), 0));
+                // All loader warps of both CTAs report their atoms to the leader; the leader's warp j then copies K tile
+                // j's atoms of both CTAs into both CTAs' tensor memory (one cta_group::2 copy does the same offsets in
+                // the two).
+                mbar_arrive_cluster(map_to_cta(smem_u32(&atoms[buf]), 0));
                 if (cta == 0) {
-                    mbar_wait_cluster(&atoms_written[s], ph, p.status, 207, s, bar_ns);
+                    alive = mbar_wait_cluster(&atoms[buf], ph, p.status, 208, buf, bar_ns) && alive;
                     tcgen05_fence_after();
-                    const uint32_t hi_sf = (uint32_t)(make_smem_desc(0, 0, 128, 0) >> 32);
-                    const uint32_t sf_t = tmem_base + S::kSfCol + s * S::kSfSetCols;
-                    tcgen05_cp_sf_pair_lohi(sf_t, smem_u32(sfa) >> 4, hi_sf);
-                    tcgen05_cp_sf_pair_lohi(sf_t + 4, smem_u32(sfb) >> 4, hi_sf);
-                    tcgen05_cp_sf_pair_lohi(sf_t + 8, (smem_u32(sfb) >> 4) + (512u >> 4), hi_sf);
-                    tcgen05_commit_pair(&full[s], 1);
+                    if (real) {
+                        const uint32_t hi_sf = (uint32_t)(make_smem_desc(0, 0, 128, 0) >> 32);
+                        const uint32_t sf_t = tmem_base + S::kSfCol + buf * S::kSfGroupCols + j * S::kSfSetCols;
+                        tcgen05_cp_sf_pair_lohi(sf_t, smem_u32(sfa + j * S::kSfaBytes) >> 4, hi_sf);
+#pragma unroll
+                        for (uint32_t h = 0; h < kPairBlockN / 128; ++h) {
+                            tcgen05_cp_sf_pair_lohi(sf_t + 4 + 4 * h, (smem_u32(sfb) >> 4) + h * (512u >> 4), hi_sf);
+                        }
+                    }
+                    tcgen05_commit_pair(&sf_full[buf], 1);
                 }
             }
-            if (has_next) {
+            alive = __all_sync(0xFFFFFFFFu, alive);
+            ++group;
+            cur_a = nxt_a;
 #pragma unroll
-                for (uint32_t i = 0; i < 4; ++i) cur_a[i] = nxt_a[i];
-#pragma unroll
-                for (uint32_t i = 0; i < kNB; ++i) {
-                    cur_lo[i] = nxt_lo[i];
-                    cur_hi[i] = nxt_hi[i];
-                }
+            for (uint32_t i = 0; i < kNB; ++i) {
+                cur_lo[i] = nxt_lo[i];
+                cur_hi[i] = nxt_hi[i];
             }
         }
     } else {
@@ -395,17 +537,17 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         const uint32_t q = warp;
         OutT* c = reinterpret_cast<OutT*>(p.c);
         constexpr uint32_t kChunks = kPairBlockN / 32;
-        uint32_t ti = 0;
-        for (uint32_t tile = pair; tile < num_tiles; tile += num_pairs, ++ti) {
-            TileCoord tc = pair_tile_coord(tile, n_tiles, m_tiles, p);
-            const uint32_t m0 = tc.m_tile * kPairBlockM + cta * 128u;
-            const uint32_t n0 = tc.n_tile * kPairBlockN;
-            const uint32_t acc = ti & 1u;
-            const uint32_t acc_ph = (ti >> 1) & 1u;
+        const uint32_t lane_base = tmem_base + ((q * 32u) << 16);
+        uint8_t* stage_out = smem + S::kOffOut + q * kOutStageBytes;
+        for (uint32_t ui = 0; alive && ui < work.units; ++ui) {
+            const PairUnit u = work.unit(ui, p);
+            const uint32_t row0 = u.m0 + cta * 128u + q * 32u;  // this warp's first row
+            const uint32_t row = row0 + lane;
+            const uint32_t acc = ui & 1u;
             const uint32_t d_col = acc ? S::kAccCol1 : 0u;
             const unsigned long long t0 = CATCCOS_TR_NOW();
             (void)t0;
-            const bool alive = mbar_wait_warp(&tmem_full[acc], acc_ph, p.status, 206, acc, bar_ns);
+            alive = mbar_wait_warp(&tmem_full[acc], (ui >> 1) & 1u, p.status, 206, acc, bar_ns);
             if (q == 0 && lane == 0) {
                 CATCCOS_TR_ADD(p.trace, kTrEpiWaitNs, CATCCOS_TR_NOW() - t0);
             }
@@ -413,39 +555,79 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 break;  // an accumulator that never filled is not written out
             }
             tcgen05_fence_after();
-            const uint32_t row = m0 + q * 32 + lane;
-            for (uint32_t ci = 0; ci < kChunks; ++ci) {
-                uint32_t chunk = ci;
-                if (acc == 0) {  // the shared columns first
-                    chunk = ci < S::kOverlapChunks ? kChunks - S::kOverlapChunks + ci : ci - S::kOverlapChunks;
-                }
-                uint32_t r[32];
-                tmem_ld_32x32(tmem_base + ((q * 32u) << 16) + d_col + chunk * 32u, r);
-                tmem_ld_wait();
-                if (ci == S::kOverlapChunks - 1) {
-                    tcgen05_fence_before();
-                    __syncwarp();
-                    if (lane == 0) {
-                        mbar_arrive_cluster(map_to_cta(smem_u32(&overlap_free[acc]), 0));
+            if (u.split) {
+                // always the last unit: the operand stages are idle by now and receive the other parts' pieces
+                SplitExchange<OutT, kChunks> x;
+                const uint32_t slot = u.rem_ix * work.ksplit * 2u + cta;
+                x.ws = p.splitk_ws + (size_t)slot * (128u * kPairBlockN);
+                x.part_stride = (size_t)2u * 128u * kPairBlockN;
+                x.flags = p.splitk_flags + slot * 4u + q;
+                x.flag_stride = 8u;
+                x.red = smem + S::kOffA + q * kSplitRedBytes;
+                x.bar = &red_bar[q];
+                alive = x.run(p, c, lane_base + d_col, u.part, work.ksplit, q, lane, row0, u.n0, u.rem_ix, bar_ns);
+                continue;
+            }
+            // the half that holds the columns shared with the other accumulator goes first, columns 128..255 of
+            // accumulator 0, 0..127 of accumulator 1
+            for (uint32_t hi = 0; hi < 2; ++hi) {
+                const uint32_t col0 = (acc == 0u ? 1u - hi : hi) * 128u;
+                const bool inside = row0 < p.Mg && u.n0 + col0 < p.N;
+                uint32_t scale_word = 0;
+#pragma unroll
+                for (uint32_t g = 0; g < 2; ++g) {
+                    uint32_t r0[32], r1[32];
+                    tmem_ld_32x32(lane_base + d_col + col0 + g * 64u, r0);
+                    tmem_ld_32x32(lane_base + d_col + col0 + g * 64u + 32u, r1);
+                    tmem_ld_wait();
+                    if (g == 1u) {
+                        tcgen05_fence_before();
+                        __syncwarp();
+                        if (lane == 0) {
+                            uint64_t* b = hi == 0u ? &overlap_free[acc] : &tmem_empty[acc];
+                            mbar_arrive_cluster(map_to_cta(smem_u32(b), 0));
+                        }
+                    }
+                    const uint32_t col = u.n0 + col0 + g * 64u;
+                    if constexpr (std::is_same<OutT, ScatterOut>::value) {
+                        store_c_chunk<OutT>(c, p, row, col, r0);
+                        store_c_chunk<OutT>(c, p, row, col + 32u, r1);
+                    } else if constexpr (std::is_same<OutT, MxOut>::value) {
+                        if (g == 0u) {
+                            out_stage_free(lane);
+                        }
+                        uint32_t o[8], byte0, byte1;
+                        mx_quantise_chunk(p, r0, o, byte0);
+                        out_stage_put(stage_out, lane, g * 4u, o);
+                        mx_quantise_chunk(p, r1, o, byte1);
+                        out_stage_put(stage_out, lane, g * 4u + 2u, o);
+                        scale_word |= (byte0 | (byte1 << 8)) << (16u * g);
+                        if (g == 1u) {
+                            out_stage_send(stage_out, &tmap_c, lane, inside, u.n0 + col0, row0);
+                            store_scale_word(p, row, u.n0 + col0, scale_word);
+                        }
+                    } else {
+                        out_stage_free(lane);
+                        out_stage_put_chunk<OutT>(stage_out, lane, 0u, r0);
+                        out_stage_put_chunk<OutT>(stage_out, lane, 4u, r1);
+                        out_stage_send(stage_out, &tmap_c, lane, inside && col < p.N, col, row0);
                     }
                 }
-                store_c_chunk<OutT>(c, p, row, n0 + chunk * 32u, r);
             }
-            publish_tile_rows<OutT>(p, m0 + q * 32u, tc.n_tile, n_tiles, lane);
-            tcgen05_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-                mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[acc]), 0));
-                if (q == 0) {
-                    CATCCOS_TR_STAMP(p.trace, kTrEpiLast);
-                }
+            publish_tile_rows<OutT>(p, row0, u.n_tile, work.n_tiles, lane);
+            if (lane == 0 && q == 0) {
+                CATCCOS_TR_STAMP(p.trace, kTrEpiLast);
             }
+        }
+        if (lane == 0) {
+            bulk_store_wait_all();  // the output is written before the CTA ends
         }
     }
 
     tcgen05_fence_before();
-    __syncthreads();
-    drain_after_abort(p.status);  // both CTAs stay while loads that report to the other's barriers may be in flight
+    if (__syncthreads_or(alive ? 0 : 1)) {
+        drain_after_abort(p.status);  // both CTAs stay while loads that report to the other's barriers may be in flight
+    }
     cluster_sync_all();  // nobody leaves while the other CTA may still arrive on its barriers
     if (p.flags != nullptr) {
         grid_dep_wait();
