@@ -367,12 +367,14 @@ void choose_segments(uint32_t M, uint32_t K, int num_sms, QuantPushParams& p, ui
 }
 
 // bf16 [M, K] -> codes and scales in one place, nobody waiting on flags: the flat quantiser.
-int launch_quant_flat(cudaStream_t st, const void* in, uint32_t M, uint32_t K, uint8_t* codes, uint8_t* scales)
+// `reset` (or nullptr): a wait record that starts anew with this call.
+int launch_quant_flat(cudaStream_t st, const void* in, uint32_t M, uint32_t K, uint8_t* codes, uint8_t* scales,
+                      StatusBlock* reset = nullptr)
 {
     const uint64_t halves = (uint64_t)M * (K / 16);
     const dim3 grid((unsigned)((halves + kQuantThreads - 1) / kQuantThreads));
     CUDA_TRY(launch_after(g.a_dtype == 1 ? mx_quant_flat_kernel<true> : mx_quant_flat_kernel<false>, grid, kQuantThreads, 0, st,
-                          static_cast<const uint8_t*>(in), codes, scales, halves, g.tiny_block_rule != 0 ? 1u : 0u));
+                          static_cast<const uint8_t*>(in), codes, scales, halves, g.tiny_block_rule != 0 ? 1u : 0u, reset));
     return 0;
 }
 
@@ -1903,13 +1905,12 @@ uint64_t catccos_b200_launch_count(void) { return g_launches.load(); }
 // =============================================================================================
 namespace {
 
-// Scratch of catccos_b200_mx_quant_matmul_static: the quantised copy of A and its ready flags live in
+// Scratch of catccos_b200_mx_quant_matmul_static: the quantised copy of A lives in
 // this file-scope device array instead of a buffer from catccos_b200_symm_alloc.  Every GPU that
 // loads the library carries it (about 8.3 MiB) until the process exits.
 constexpr size_t kStaticMaxElems = size_t(8) << 20;  // m * k may not exceed this
-constexpr uint32_t kStaticMaxFlags = 8192;           // (16-row chunks) x (K segments) may not exceed this
-constexpr size_t kStaticFlagsOff = 0;
-constexpr size_t kStaticStatusOff = kStaticMaxFlags * sizeof(uint32_t);
+constexpr uint32_t kStaticMaxItems = 8192;           // (16-row chunks) x (K segments) may not exceed this
+constexpr size_t kStaticStatusOff = 0;
 constexpr size_t kStaticScalesOff = kStaticStatusOff + 1024;
 constexpr size_t kStaticCodesOff = kStaticScalesOff + kStaticMaxElems / 32;
 constexpr size_t kStaticBytes = kStaticCodesOff + kStaticMaxElems;
@@ -1920,7 +1921,6 @@ static __device__ __align__(256) uint8_t g_static_scratch[kStaticBytes];
 struct StaticDeviceState {
     uint8_t* ptr = nullptr;  // device address of g_static_scratch on this device
     int num_sms = 0;
-    uint32_t epoch = 0;
 };
 StaticDeviceState g_static_dev[kMaxRanks * 2];
 std::mutex g_static_mu;
@@ -1975,52 +1975,33 @@ extern "C" int catccos_b200_mx_quant_matmul_static(void* stream, const void* a_b
     QuantPushParams seg = {};
     choose_segments(m, k, rc.num_sms, seg);
     const uint32_t chunks = (m + kRowsPerChunk - 1) / kRowsPerChunk;
-    if ((size_t)chunks * seg.segs_per_chunk > kStaticMaxFlags) {
-        ERROR_LOG("mx_quant_matmul_static: %u row chunks x %u K segments exceed the built-in %u flag words", chunks,
-                  seg.segs_per_chunk, kStaticMaxFlags);
+    if ((size_t)chunks * seg.segs_per_chunk > kStaticMaxItems) {
+        ERROR_LOG("mx_quant_matmul_static: %u row chunks x %u K segments exceed the limit of %u", chunks, seg.segs_per_chunk,
+                  kStaticMaxItems);
         return CATCCOS_B200_ENOMEM;
     }
+    if (g.b_dtype == 2) {
+        return CATCCOS_B200_ESTATE;  // packed weights need a transposed copy, and this path has no scratch for it
+    }
+    // Two launches on the caller's stream, as catccos_b200_mx_quant_allgather_matmul at one rank: the quantiser on every
+    // SM, then the GEMM (K in one piece: the array has no room for partial tiles).  One kernel that does both measured
+    // 36 us on 509 x 2320 x 3968.
     cudaStream_t st = (cudaStream_t)stream;
-    // the array keeps what the last call left: the flag words are epochs that only grow, so stale ones
-    // never satisfy this call; the status record must start at zero
-    CUDA_TRY(cudaMemsetAsync(rc.status, 0, sizeof(StatusBlock), st));
-    const uint32_t epoch = ++sd.epoch;
-
+    uint8_t* codes = sd.ptr + kStaticCodesOff;
+    uint8_t* scales = sd.ptr + kStaticScalesOff;
+    int rcode = launch_quant_flat(st, a_bf16, m, k, codes, scales, rc.status);
+    if (rcode != 0) return rcode;
     GemmParams p = {};
-    p.a_scales = sd.ptr + kStaticScalesOff;
+    p.a_scales = scales;
     p.b_scales = (const uint8_t*)b_scale;
     p.c = c;
     p.Mg = m;
     p.N = n;
     p.K = k;
-    p.flags = reinterpret_cast<const uint32_t*>(sd.ptr + kStaticFlagsOff);
-    p.flag_stride = kStaticMaxFlags;
-    p.segs = seg.segs_per_chunk;
-    p.seg_ktiles = seg.seg_cols / kGemmBlockK;
     p.world = 1;
-    p.rank = 0;
     p.m_local = m;
-    p.epoch = epoch;
-    QuantPushParams& q = p.q;
-    q.in = a_bf16;
-    q.M = m;
-    q.K = k;
-    q.world = 1;
-    q.epoch = epoch;
-    q.num_dst = 1;
-    q.publish = 1;
-    q.produce = 1;
-    q.mode = quant_mode(false);
-    q.e5m2 = g.a_dtype == 1 ? 1u : 0u;
-    q.sys_scope = 0;
-    q.segs_per_chunk = seg.segs_per_chunk;
-    q.seg_cols = seg.seg_cols;
-    q.dst_codes[0] = sd.ptr + kStaticCodesOff;
-    q.dst_scales[0] = sd.ptr + kStaticScalesOff;
-    q.dst_flags[0] = reinterpret_cast<uint32_t*>(sd.ptr + kStaticFlagsOff);
-    q.status = rc.status;
-    q.timeout_ns = g.timeout_ns;
-    return launch_gemm(rc, st, sd.ptr + kStaticCodesOff, b, p, true);
+    p.b_early = 1;
+    return launch_gemm(rc, st, codes, b, p, false, true);
 }
 
 #ifdef CATCCOS_TRACE

@@ -336,9 +336,13 @@ __device__ __forceinline__ void quant_push_producer(const QuantPushParams& p, ui
 template <bool kE5m2>
 __global__ void __launch_bounds__(kQuantThreads) mx_quant_flat_kernel(const uint8_t* __restrict__ in, uint8_t* __restrict__ codes,
                                                                       uint8_t* __restrict__ scales, uint64_t halves,
-                                                                      uint32_t device_tiny)
+                                                                      uint32_t device_tiny, StatusBlock* reset)
 {
     grid_dep_wait();
+    if (reset != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
+        *reset = StatusBlock{};
+        __threadfence();  // before the GEMM behind this kernel may look at it
+    }
     grid_dep_launch();
     const uint64_t i = (uint64_t)blockIdx.x * kQuantThreads + threadIdx.x;
     uint4 v0 = make_uint4(0, 0, 0, 0), v1 = v0;

@@ -147,10 +147,10 @@ size_t catccos_b200_packed_row_bytes(uint32_t n);
 int catccos_b200_mx_quant_scatter_packed(void* stream, const void* in_bf16, const int32_t* expanded_row_idx, void* packed_out,
                                          uint32_t tokens, uint32_t n, uint32_t top_k);
 
-/* Fused quantise + matmul on one GPU that allocates nothing.  It has no counterpart in the reference.
+/* Quantise + matmul on one GPU that allocates nothing.  It has no counterpart in the reference.
  * c [m, n] = dequant(quantise(a_bf16 [m, k])) x dequant(b [k, n], b_scale [k/64, n, 2]): the same two
- * fused stages as catccos_b200_mx_quant_allgather_matmul at rankSize 1, but the quantised copy of A and
- * its ready flags live in an array that is part of the library image (a file-scope __device__ array of
+ * stages as catccos_b200_mx_quant_allgather_matmul at rankSize 1, but the quantised copy of A
+ * lives in an array that is part of the library image (a file-scope __device__ array of
  * about 8.3 MiB that every GPU loading the library holds until the process exits) instead of a buffer
  * from catccos_b200_symm_alloc.
  *
