@@ -19,6 +19,7 @@
 #include "common.cuh"
 #include "mx_gemm.cuh"
 #include "mx_gemm_pair.cuh"
+#include "mx_gemm_small.cuh"
 #include "mx_quant.cuh"
 
 using namespace catccos;
@@ -164,6 +165,8 @@ struct State {
     int a_dtype = 0;         // element type of the A codes (what the quantiser writes, what the GEMM reads): 0 = E4M3, 1 = E5M2
     int b_dtype = 0;         // element type of the B codes the caller passes
     int split_k = 0;         // 0 = automatic, 1 = never split K, 2..8 = split K in that many parts when it fits
+    int small_tile = 0;      // 0 = automatic, 1 = always the small-tile kernel where it can run, 2 = never
+    int small_quant = 0;     // 0 = automatic, 1 = the small-tile kernel quantises a fused call itself, 2 = never
     int tile_order = -1;     // gated GEMM: -1 = automatic, 1 = own shard first, 0 = slice by slice over all ranks
     uint64_t timeout_ns = 2000ull * 1000000ull;
 #ifdef CATCCOS_TRACE
@@ -620,6 +623,7 @@ constexpr double kSplitCost = 3.5, kSplitCostPerCta = 0.012;
 struct GemmPlan {
     bool use_pair;
     uint32_t block_n, ksplit;  // ksplit: CTA pairs: most parts of a last-round tile; single CTAs: parts of every tile
+    double time;               // what the launch is expected to take, microseconds
 };
 
 // Tiling of one GEMM launch: CTA pairs or single CTAs, tile width, and the number of K parts.
@@ -679,7 +683,140 @@ GemmPlan plan_gemm(const RankCtx& rc, uint32_t Mg, uint32_t N, uint32_t K, bool 
     plan.use_pair = g.cta_pair == 1 || (g.cta_pair == 0 && g.block_n == 0 && t_pair < (bn == 256 ? t_256 : t_128));
     plan.block_n = plan.use_pair ? kPairBlockN : bn;
     plan.ksplit = plan.use_pair ? pair_parts : (bn == 256 ? parts256 : parts128);
+    plan.time = plan.use_pair ? t_pair : (bn == 256 ? t_256 : t_128);
     return plan;
+}
+
+// The small-tile kernel (mx_gemm_small.cuh) for a call: activation rows of a tile, K parts, and whether it quantises.
+struct SmallPlan {
+    bool use, quant;
+    uint32_t mt, parts;
+};
+
+// What it costs, as above: a launch of one K tile; each further K tile of a CTA while loads are latency-bound (with the
+// quantisation inside, four warps' work, more so with two CTAs on an SM); or, if that is longer, streaming every tile's
+// weights (rows of N bytes that are no multiple of 128 straddle two lines each); and the exchange of the parts.  CTAs
+// beyond two per SM start when others end and pay their start again, so splitting stops there.  A
+// quantiser in front costs a launch and a dependency, more in front of the kernels that need a whole SM's shared memory.
+constexpr double kSmallBase = 2.9, kSmallPeriod = 0.24, kSmallQuant16 = 0.40, kSmallQuant32 = 0.85, kSmallQuantShared = 1.5;
+constexpr double kSmallBytesPerUs = 6.0e6, kSmallBytesPerUsRagged = 3.3e6;
+constexpr double kSmallExchange16 = 0.8, kSmallExchange32 = 1.1, kSmallExchange32PerRow = 0.06;
+constexpr double kSmallMxOutPerRow = 0.08;  // a warp takes the block maximum of one row at a time
+constexpr double kQuantiserSmall = 1.6, kQuantiserLarge = 2.5;
+
+SmallPlan plan_small(const RankCtx& rc, uint32_t M, uint32_t N, uint32_t K, bool bf16_in, bool mx_out = false)
+{
+    SmallPlan s = {};
+    if (g.small_tile == 2 || g.cta_pair != 0 || g.block_n != 0) {
+        return s;  // another tiling is asked for
+    }
+    s.mt = M <= 16 ? 16 : 32;
+    const uint32_t tiles = ((M + s.mt - 1) / s.mt) * ((N + kSmallBlockN - 1) / kSmallBlockN), k_tiles = K / kGemmBlockK;
+    const uint32_t cap = std::min(g.split_k >= 1 ? (uint32_t)g.split_k : kSmallMaxParts, k_tiles);
+    const uint32_t sms = (uint32_t)rc.num_sms;
+    const double stream = (double)tiles * k_tiles * (kSmallBlockN * kGemmBlockK) / (N % 128u == 0u ? kSmallBytesPerUs : kSmallBytesPerUsRagged);
+    double best = 0.0;
+    for (uint32_t quant = 0; quant <= (bf16_in ? 1u : 0u); ++quant) {
+        if (bf16_in && g.small_quant != 0 && (quant != 0) != (g.small_quant == 1)) {
+            continue;
+        }
+        for (uint32_t parts = 1; parts <= cap; parts *= 2) {
+            if (parts > 1 && tiles * parts > 2 * sms && g.split_k <= 1) {
+                break;
+            }
+            const double rounds = (double)((tiles * parts + 2 * sms - 1) / (2 * sms));
+            double period = kSmallPeriod;
+            if (quant) {
+                period = (s.mt == 16 ? kSmallQuant16 : kSmallQuant32) * (tiles * parts > sms ? kSmallQuantShared : 1.0);
+            }
+            double t = rounds * kSmallBase + std::max(((k_tiles + parts - 1) / parts) * period * rounds, stream);
+            if (parts > 1) {
+                t += s.mt == 16 ? kSmallExchange16 : kSmallExchange32 + kSmallExchange32PerRow * (s.mt / parts);
+            }
+            t += bf16_in && !quant ? kQuantiserSmall : 0.0;
+            t += mx_out ? kSmallMxOutPerRow * (s.mt / parts) : 0.0;
+            if (s.parts == 0 || t < best || (g.split_k > 1 && parts * 2 > cap && quant == (uint32_t)s.quant)) {
+                best = t;
+                s.parts = parts;
+                s.quant = quant != 0;
+            }
+        }
+    }
+    s.use = g.small_tile == 1 || best < plan_gemm(rc, M, N, K).time + (bf16_in ? kQuantiserLarge : 0.0);
+    return s;
+}
+
+template <uint32_t MT, typename OutT, bool QUANT>
+int launch_small_inst(cudaStream_t st, const CUtensorMap& tw, const CUtensorMap& tx, const SmallParams& p)
+{
+    auto kern = mx_gemm_small_kernel<MT, OutT, QUANT>;
+    static bool attr_done[kMaxRanks * 2] = {};
+    int dev = 0;
+    CUDA_TRY(cudaGetDevice(&dev));
+    if (dev >= kMaxRanks * 2 || !attr_done[dev]) {
+        CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SmallSmem<MT>::kDynamicBytes));
+        CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        if (dev < kMaxRanks * 2) attr_done[dev] = true;
+    }
+    const uint32_t tiles = ((p.M + MT - 1) / MT) * ((p.N + kSmallBlockN - 1) / kSmallBlockN);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(tiles * p.parts);
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = SmallSmem<MT>::kDynamicBytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = p.parts;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    g_launches++;
+    CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tw, tx, p));
+    return 0;
+}
+
+// p: x or x_scales, w_scales, c, c_scales, M, N, K, w_early, w_kmajor, clear filled in.
+int launch_small(RankCtx& rc, cudaStream_t st, const SmallPlan& plan, const void* x_codes, const void* w, SmallParams p,
+                 bool mx_out)
+{
+    if (!g.drv.Load()) {
+        return CATCCOS_B200_ECUDA;
+    }
+    p.parts = plan.parts;
+    p.status = rc.status;
+    p.bar_timeout_ns = 2 * g.timeout_ns + 1000000000ull;
+    p.x_fmt = g.a_dtype == 2 ? 5u : (g.a_dtype == 1 ? 1u : 0u);
+    p.w_fmt = g.b_dtype == 2 ? 5u : (g.b_dtype == 1 ? 1u : 0u);
+    p.device_tiny = g.tiny_block_rule != 0 ? 1u : 0u;
+    CUtensorMap tw, tx;
+    int rcode = p.w_kmajor ? encode_map_2d(&tw, w, p.K, p.N, kGemmBlockK, kSmallBlockN, g.b_dtype == 2)
+                           : encode_map_2d(&tw, w, p.N, p.K, kSmallBlockN, kGemmBlockK);
+    if (rcode != 0) return rcode;
+    tx = tw;  // not read by a quantising launch
+    if (!plan.quant) {
+        rcode = encode_map_2d(&tx, x_codes, p.K, p.M, kGemmBlockK, plan.mt, g.a_dtype == 2);
+        if (rcode != 0) return rcode;
+    }
+    const bool f16 = g.c_dtype == 1;
+#define CATCCOS_SMALL_CASE(MT)                                                                   \
+    if (plan.mt == MT) {                                                                         \
+        if (mx_out) {                                                                            \
+            return launch_small_inst<MT, MxOut, false>(st, tw, tx, p);                           \
+        }                                                                                        \
+        if (plan.quant) {                                                                        \
+            return f16 ? launch_small_inst<MT, __half, true>(st, tw, tx, p)                      \
+                       : launch_small_inst<MT, __nv_bfloat16, true>(st, tw, tx, p);              \
+        }                                                                                        \
+        return f16 ? launch_small_inst<MT, __half, false>(st, tw, tx, p)                         \
+                   : launch_small_inst<MT, __nv_bfloat16, false>(st, tw, tx, p);                 \
+    }
+    CATCCOS_SMALL_CASE(16)
+    CATCCOS_SMALL_CASE(32)
+#undef CATCCOS_SMALL_CASE
+    return CATCCOS_B200_EINVAL;
 }
 
 // overlap_predecessor: the kernel launched just before on `st` is this library's quantise kernel, whose output
@@ -742,6 +879,22 @@ int launch_gemm(RankCtx& rc, cudaStream_t st, const void* a, const void* b, Gemm
         p.b_kmajor = 1;
         p.b_early = 0;  // the copy is the kernel launched just before
         overlap_predecessor = false;
+    }
+    if (p.flags == nullptr && !fused_quant && !scatter) {
+        const SmallPlan small = plan_small(rc, p.Mg, p.N, p.K, false, mx_out);
+        if (small.use) {
+            SmallParams sp = {};
+            sp.x_scales = p.a_scales;
+            sp.w_scales = p.b_scales;
+            sp.c = p.c;
+            sp.c_scales = p.c_scales;
+            sp.M = p.Mg;
+            sp.N = p.N;
+            sp.K = p.K;
+            sp.w_kmajor = p.b_kmajor;
+            sp.w_early = p.b_early;
+            return launch_small(rc, st, small, a, b, sp, mx_out);
+        }
     }
     const GemmPlan plan = plan_gemm(rc, p.Mg, p.N, p.K, scatter);  // scatter: the owner adds whole tiles, K stays in one piece
     const bool use_pair = plan.use_pair;
@@ -892,6 +1045,12 @@ int copy_engine_join(RankCtx& rc, cudaStream_t st, uint32_t W)
     return 0;
 }
 
+// Alignment a fused call needs; a call that lacks it takes the general path, which refuses it with a message.
+bool fused_operands_ok(const void* a, const void* b, const void* b_scale, const void* c)
+{
+    return (((uintptr_t)a | (uintptr_t)b) & 15u) == 0u && ((uintptr_t)c & 31u) == 0u && ((uintptr_t)b_scale & 1u) == 0u;
+}
+
 // Common part of the two AllGather-Matmul entry points.
 int allgather_matmul(void* stream, const void* a, const void* a_scale, bool prequant, const void* b,
                      const void* b_scale, void* c, void* symm, const catccos_b200_tiling_t* t)
@@ -1024,6 +1183,17 @@ int allgather_matmul(void* stream, const void* a, const void* a_scale, bool preq
             p.a_scales = (const uint8_t*)a_scale;
             p.flags = nullptr;
             return launch_gemm(rc, st, a, b, p);
+        }
+        const SmallPlan small = plan_small(rc, M, N, K, !prequant);
+        if (!prequant && small.use && small.quant && g.b_dtype != 2 && fused_operands_ok(a, b, b_scale, c)) {
+            SmallParams sp = {};
+            sp.x = a;
+            sp.w_scales = (const uint8_t*)b_scale;
+            sp.c = c;
+            sp.M = M;
+            sp.N = N;
+            sp.K = K;
+            return launch_small(rc, st, small, nullptr, b, sp, false);
         }
         if (prequant) {
             q.publish = 0;
@@ -1887,6 +2057,10 @@ int catccos_b200_set_option(const char* key, int64_t value)
         g.fuse_mode = (int)value;
     } else if (k == CATCCOS_B200_OPT_SPLIT_K && value >= 0 && value <= 8) {
         g.split_k = (int)value;
+    } else if (k == CATCCOS_B200_OPT_SMALL_TILE && value >= 0 && value <= 2) {
+        g.small_tile = (int)value;
+    } else if (k == CATCCOS_B200_OPT_SMALL_QUANT && value >= 0 && value <= 2) {
+        g.small_quant = (int)value;
     } else if (k == CATCCOS_B200_OPT_TILE_ORDER && value >= -1 && value <= 1) {
         g.tile_order = (int)value;
     } else {
@@ -1921,6 +2095,7 @@ static __device__ __align__(256) uint8_t g_static_scratch[kStaticBytes];
 struct StaticDeviceState {
     uint8_t* ptr = nullptr;  // device address of g_static_scratch on this device
     int num_sms = 0;
+    uint32_t record = 0;  // which of the two wait records the last call uses; the other one is clear
 };
 StaticDeviceState g_static_dev[kMaxRanks * 2];
 std::mutex g_static_mu;
@@ -1970,7 +2145,8 @@ extern "C" int catccos_b200_mx_quant_matmul_static(void* stream, const void* a_b
     RankCtx rc;  // a view for the launcher: nothing is created or owned here
     rc.device = dev;
     rc.num_sms = sd.num_sms;
-    rc.status = reinterpret_cast<StatusBlock*>(sd.ptr + kStaticStatusOff);
+    StatusBlock* records = reinterpret_cast<StatusBlock*>(sd.ptr + kStaticStatusOff);
+    rc.status = records + sd.record;
 
     QuantPushParams seg = {};
     choose_segments(m, k, rc.num_sms, seg);
@@ -1982,6 +2158,21 @@ extern "C" int catccos_b200_mx_quant_matmul_static(void* stream, const void* a_b
     }
     if (g.b_dtype == 2) {
         return CATCCOS_B200_ESTATE;  // packed weights need a transposed copy, and this path has no scratch for it
+    }
+    const SmallPlan small = plan_small(rc, m, n, k, true);
+    if (small.use && small.quant) {
+        // one launch; it takes the clear record, and clears the last call's once that call has finished
+        SmallParams sp = {};
+        sp.x = a_bf16;
+        sp.w_scales = (const uint8_t*)b_scale;
+        sp.c = c;
+        sp.M = m;
+        sp.N = n;
+        sp.K = k;
+        sp.clear = records + sd.record;
+        sd.record ^= 1u;
+        rc.status = records + sd.record;
+        return launch_small(rc, (cudaStream_t)stream, small, nullptr, b, sp, false);
     }
     // Two launches on the caller's stream, as catccos_b200_mx_quant_allgather_matmul at one rank: the quantiser on every
     // SM, then the GEMM (K in one piece: the array has no room for partial tiles).  One kernel that does both measured
@@ -2063,7 +2254,7 @@ extern "C" int catccos_b200_mx_quant_matmul_static_status(uint32_t out[4])
     }
     CUDA_TRY(cudaDeviceSynchronize());
     StatusBlock sb;
-    CUDA_TRY(cudaMemcpy(&sb, sd.ptr + kStaticStatusOff, sizeof(sb), cudaMemcpyDeviceToHost));
+    CUDA_TRY(cudaMemcpy(&sb, sd.ptr + kStaticStatusOff + sd.record * sizeof(sb), sizeof(sb), cudaMemcpyDeviceToHost));
     out[0] = sb.code;
     out[1] = sb.rank;
     out[2] = sb.chunk;

@@ -22,6 +22,10 @@
 // 0 = automatic (K is cut in up to eight parts when the output tiles would leave half of the SMs idle),
 // 1 = never, 2..8 = at most that many parts
 #define CATCCOS_B200_OPT_SPLIT_K "split_k"
+// small-tile kernel (one GPU, no flags): 0 = automatic, 1 = always where it can run, 2 = never
+#define CATCCOS_B200_OPT_SMALL_TILE "small_tile"
+// a fused call on the small-tile kernel: 0 = automatic, 1 = it quantises the activations itself, 2 = quantiser first
+#define CATCCOS_B200_OPT_SMALL_QUANT "small_quant"
 // order in which a flag-gated GEMM visits its row tiles: -1 = automatic (follows fuse_mode), 1 = this rank's own
 // shard first, then the peers slice by slice, 0 = slice by slice over all ranks, own slice leading
 #define CATCCOS_B200_OPT_TILE_ORDER "tile_order"

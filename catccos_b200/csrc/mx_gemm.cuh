@@ -628,6 +628,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     using S = GemmSmem<BLOCK_N>;
     constexpr uint32_t kStages = S::kStages;
     static_assert(BLOCK_N == 128 || BLOCK_N == 256, "tile widths wired up: 128 and 256");
+    static_assert(kSfWarps <= kStages, "a scale loader would take a stale phase of a stage for the one it waits for");
 
     grid_dep_launch();  // what follows on the stream may be set up meanwhile; it waits for this kernel before it reads
     extern __shared__ uint8_t smem_raw[];
