@@ -873,7 +873,7 @@ int launch_gemm(RankCtx& rc, cudaStream_t st, const void* a, const void* b, Gemm
             CUDA_TRY(cudaMalloc(&rc.fp4_bt, need));
             rc.fp4_bt_bytes = need;
         }
-        dim3 tg((p.N + kFp4TransN - 1) / kFp4TransN, (p.K + kFp4TransK - 1) / kFp4TransK);
+        const dim3 tg(((p.N / kFp4TransTile) * (p.K / kFp4TransTile) + 7) / 8);  // a warp per tile
         CUDA_TRY(launch_after(fp4_transpose_kernel, tg, 256, 0, st, static_cast<const uint8_t*>(b), rc.fp4_bt, p.K, p.N));
         b = rc.fp4_bt;
         p.b_kmajor = 1;
