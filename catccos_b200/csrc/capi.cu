@@ -619,6 +619,8 @@ int launch_gemm_pair_inst(uint32_t max_pairs, uint32_t tiles, uint32_t parts, cu
 constexpr double kBasePair = 4.7, kBaseSingle256 = 4.0, kBaseSingle128 = 2.9;
 constexpr double kPeriodPair = 0.37, kPeriodSingle256 = 0.43, kPeriodSingle128 = 0.39;
 constexpr double kSplitCost = 3.5, kSplitCostPerCta = 0.012;
+// with whole tiles to follow, beside which the exchange passes (but the partial tiles' traffic does not)
+constexpr double kSplitFirstCost = 3.0, kSplitFirstCostPerCta = 0.024;
 
 struct GemmPlan {
     bool use_pair;
@@ -644,7 +646,8 @@ GemmPlan plan_gemm(const RankCtx& rc, uint32_t Mg, uint32_t N, uint32_t K, bool 
     uint32_t pair_parts = 1;
     double last = rem != 0 ? k_tiles * kPeriodPair : 0.0;
     for (uint32_t s = 2; rem != 0 && s <= std::min(std::min(cap, max_pairs / rem), k_tiles); ++s) {
-        const double t = ((k_tiles + s - 1) / s) * kPeriodPair + split_cost(2 * rem * s);
+        const double cost = tiles >= max_pairs ? kSplitFirstCost + kSplitFirstCostPerCta * 2 * rem * s : split_cost(2 * rem * s);
+        const double t = ((k_tiles + s - 1) / s) * kPeriodPair + cost;
         if (t < last) {
             last = t;
             pair_parts = s;

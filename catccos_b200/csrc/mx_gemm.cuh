@@ -574,6 +574,74 @@ struct SplitExchange {
         }
         return true;
     }
+
+    // The same exchange when whole tiles follow on the CTA: nothing may hold tensor or shared memory meanwhile, so every
+    // chunk goes to the workspace at once (put), and the owner reads all parts' pieces back into registers (take), in
+    // ascending part order.  The time this takes passes beside the next tile's products.
+    __device__ __forceinline__ void put(const GemmParams& p, uint32_t tmem_acc, uint32_t part, uint32_t q, uint32_t lane,
+                                        uint32_t row0, uint32_t n0)
+    {
+        const bool lane_row = row0 + lane < p.Mg;
+        for (uint32_t chunk = 0; row0 < p.Mg && chunk < kChunks && n0 + chunk * 32u < p.N; ++chunk) {
+            uint32_t r[32];
+            tmem_ld_32x32(tmem_acc + chunk * 32u, r);
+            tmem_ld_wait();
+            float4* dst = reinterpret_cast<float4*>(ws + part * part_stride + ((size_t)chunk * 128u + q * 32u) * 32u) + lane;
+#pragma unroll
+            for (uint32_t v = 0; v < 8; ++v) {
+                if (lane_row) {
+                    dst[v * 32u] = make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]),
+                                               __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
+                }
+            }
+        }
+    }
+
+    __device__ __forceinline__ bool take(const GemmParams& p, OutT* c, uint32_t part, uint32_t parts, uint32_t q, uint32_t lane,
+                                         uint32_t row0, uint32_t n0, uint32_t id)
+    {
+        if (row0 >= p.Mg) {
+            return true;  // as in run()
+        }
+        __syncwarp();  // every lane's partial stores are ordered before lane 0's release
+        if (lane == 0) {
+            st_release_gpu(flags + part * flag_stride, p.splitk_epoch);
+        }
+        bool ok = true;
+        if (lane < parts && lane != part &&
+            !wait_flag_ge_gpu(flags + lane * flag_stride, p.splitk_epoch, p.timeout_ns, p.status)) {
+            report_status(p.status, kStatusFlagTimeout, 0x100u + lane, id, p.splitk_epoch);
+            ok = false;
+        }
+        if (!__all_sync(0xFFFFFFFFu, ok)) {
+            return false;
+        }
+        const uint32_t own0 = (part * kChunks + parts - 1u) / parts, own1 = ((part + 1u) * kChunks + parts - 1u) / parts;
+        for (uint32_t chunk = own0; chunk < own1 && n0 + chunk * 32u < p.N; ++chunk) {
+            uint32_t r[32];
+#pragma unroll
+            for (uint32_t e = 0; e < 32; ++e) {
+                r[e] = 0u;
+            }
+            for (uint32_t src = 0; src < parts; ++src) {
+                const float4* piece = reinterpret_cast<const float4*>(ws + src * part_stride + ((size_t)chunk * 128u + q * 32u) * 32u) + lane;
+                float4 f[8];
+#pragma unroll
+                for (uint32_t v = 0; v < 8; ++v) {
+                    f[v] = __ldcg(piece + v * 32u);
+                }
+#pragma unroll
+                for (uint32_t v = 0; v < 8; ++v) {
+                    r[4 * v] = __float_as_uint(__uint_as_float(r[4 * v]) + f[v].x);
+                    r[4 * v + 1] = __float_as_uint(__uint_as_float(r[4 * v + 1]) + f[v].y);
+                    r[4 * v + 2] = __float_as_uint(__uint_as_float(r[4 * v + 2]) + f[v].z);
+                    r[4 * v + 3] = __float_as_uint(__uint_as_float(r[4 * v + 3]) + f[v].w);
+                }
+            }
+            store_c_chunk<OutT>(c, p, row0 + lane, n0 + chunk * 32u, r);
+        }
+        return true;
+    }
 };
 
 // The consumer half of Matmul + ReduceScatter: this rank's rows of the product, D [rs_rows, N] = the sum over the

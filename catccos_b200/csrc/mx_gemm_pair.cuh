@@ -25,10 +25,12 @@
 // 41.3 -> 33.3, 4096 x 3456 x 5120 66.5 -> 58.9, 8192 x 2304 x 7168 105 -> 99, 32768 x 3456 x 5120 450 -> 428 us
 // against one ring of five stages that also carried the scales, no split, and stores straight from registers.
 //
-// Work units.  num_tiles = rounds * pairs + rem: every pair takes `rounds` whole tiles, then the rem tiles that
-// would leave pairs idle are cut into ksplit parts along K, one (tile, part) per pair.  The parts exchange fp32 pieces
-// through the rank's split-K scratch: every part owns an equal share of the tile's 32-column chunks and adds the other
-// parts' pieces in ascending part order, so the result does not depend on timing.
+// Work units.  num_tiles = rounds * pairs + rem: the rem tiles that would leave pairs idle in a round of their own are
+// cut into ksplit parts along K, one (tile, part) per pair, and every pair takes `rounds` whole tiles.  The parts
+// exchange fp32 pieces through the rank's split-K scratch: every part owns an equal share of the tile's 32-column chunks
+// and adds the parts' pieces in a fixed order, so the result does not depend on timing.  A pair with whole tiles starts
+// with its part: the exchange (4 to 6 us when it comes last) then passes beside the products of the tiles that follow.
+// A gated launch (flags) ends with it, because its last tiles' rows arrive last.
 #pragma once
 
 #include "mx_gemm.cuh"
@@ -91,10 +93,11 @@ struct PairUnit {
     uint32_t kt0, kt1;        // K tiles
     uint32_t part, rem_ix;    // split units: which part, and which of the rem tiles
     bool split;
+    bool last;                // no other unit follows on this pair
 };
 
 struct PairWork {
-    uint32_t m_tiles, n_tiles, num_tiles, k_tiles, pair, num_pairs, rounds, rem, ksplit, units;
+    uint32_t m_tiles, n_tiles, num_tiles, k_tiles, pair, num_pairs, rounds, rem, ksplit, units, split_at;
 
     __host__ __device__ __forceinline__ PairWork(const GemmParams& p, uint32_t pair_, uint32_t num_pairs_)
     {
@@ -109,18 +112,21 @@ struct PairWork {
         rounds = ksplit > 1u && num_tiles * ksplit == num_pairs ? 0u : num_tiles / num_pairs;
         rem = num_tiles - rounds * num_pairs;
         units = p.gemm_off ? 0u : rounds + (pair < rem * ksplit ? 1u : 0u);
+        // the position of the unit from the incomplete round
+        split_at = units > rounds ? (ksplit > 1u && p.flags == nullptr ? 0u : rounds) : units;
     }
 
     __host__ __device__ __forceinline__ PairUnit unit(uint32_t i, const GemmParams& p) const
     {
         PairUnit u;
-        uint32_t tile = pair + i * num_pairs;
+        uint32_t tile = pair + (i - (i > split_at ? 1u : 0u)) * num_pairs;
         u.part = 0;
         u.rem_ix = 0;
         u.kt0 = 0;
         u.kt1 = k_tiles;
-        u.split = i >= rounds && ksplit > 1u;
-        if (u.split) {
+        u.split = i == split_at && ksplit > 1u;
+        u.last = i + 1u == units;
+        if (i == split_at) {
             u.part = pair / rem;
             u.rem_ix = pair - u.part * rem;
             tile = rounds * num_pairs + u.rem_ix;
@@ -556,31 +562,46 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             }
             tcgen05_fence_after();
             if (u.split) {
-                // always the last unit: the operand stages are idle by now and receive the other parts' pieces
                 SplitExchange<OutT, kChunks> x;
                 const uint32_t slot = u.rem_ix * work.ksplit * 2u + cta;
                 x.ws = p.splitk_ws + (size_t)slot * (128u * kPairBlockN);
                 x.part_stride = (size_t)2u * 128u * kPairBlockN;
                 x.flags = p.splitk_flags + slot * 4u + q;
                 x.flag_stride = 8u;
-                x.red = smem + S::kOffA + q * kSplitRedBytes;
-                x.bar = &red_bar[q];
-                alive = x.run(p, c, lane_base + d_col, u.part, work.ksplit, q, lane, row0, u.n0, u.rem_ix, bar_ns);
+                if (u.last) {
+                    // the operand stages are idle by now and receive the other parts' pieces
+                    x.red = smem + S::kOffA + q * kSplitRedBytes;
+                    x.bar = &red_bar[q];
+                    alive = x.run(p, c, lane_base + d_col, u.part, work.ksplit, q, lane, row0, u.n0, u.rem_ix, bar_ns);
+                } else {
+                    x.put(p, lane_base + d_col, u.part, q, lane, row0, u.n0);
+                    tcgen05_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive_cluster(map_to_cta(smem_u32(&overlap_free[acc]), 0));
+                        mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[acc]), 0));
+                    }
+                    alive = x.take(p, c, u.part, work.ksplit, q, lane, row0, u.n0, u.rem_ix);
+                }
                 continue;
             }
-            // the half that holds the columns shared with the other accumulator goes first, columns 128..255 of
-            // accumulator 0, 0..127 of accumulator 1
+            // The half that holds the columns shared with the other accumulator goes first, columns 128..255 of
+            // accumulator 0, 0..127 of accumulator 1.  A half is pulled into registers as a whole and its columns are given
+            // back before anything is converted or stored: the next tile's products wait for them.
+            constexpr uint32_t kPull = FUSED_QUANT ? 2 : 4;  // 32-column chunks (the fused kernel's threads have 80 registers)
             for (uint32_t hi = 0; hi < 2; ++hi) {
                 const uint32_t col0 = (acc == 0u ? 1u - hi : hi) * 128u;
                 const bool inside = row0 < p.Mg && u.n0 + col0 < p.N;
                 uint32_t scale_word = 0;
 #pragma unroll
-                for (uint32_t g = 0; g < 2; ++g) {
-                    uint32_t r0[32], r1[32];
-                    tmem_ld_32x32(lane_base + d_col + col0 + g * 64u, r0);
-                    tmem_ld_32x32(lane_base + d_col + col0 + g * 64u + 32u, r1);
+                for (uint32_t g0 = 0; g0 < 4; g0 += kPull) {
+                    uint32_t r[kPull][32];
+#pragma unroll
+                    for (uint32_t i = 0; i < kPull; ++i) {
+                        tmem_ld_32x32(lane_base + d_col + col0 + (g0 + i) * 32u, r[i]);
+                    }
                     tmem_ld_wait();
-                    if (g == 1u) {
+                    if (g0 + kPull == 4u) {
                         tcgen05_fence_before();
                         __syncwarp();
                         if (lane == 0) {
@@ -588,29 +609,33 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                             mbar_arrive_cluster(map_to_cta(smem_u32(b), 0));
                         }
                     }
-                    const uint32_t col = u.n0 + col0 + g * 64u;
-                    if constexpr (std::is_same<OutT, ScatterOut>::value) {
-                        store_c_chunk<OutT>(c, p, row, col, r0);
-                        store_c_chunk<OutT>(c, p, row, col + 32u, r1);
-                    } else if constexpr (std::is_same<OutT, MxOut>::value) {
-                        if (g == 0u) {
+#pragma unroll
+                    for (uint32_t i = 0; i < kPull; i += 2) {
+                        const uint32_t g = g0 + i;  // chunks g and g + 1: 64 columns
+                        const uint32_t col = u.n0 + col0 + g * 32u;
+                        if constexpr (std::is_same<OutT, ScatterOut>::value) {
+                            store_c_chunk<OutT>(c, p, row, col, r[i]);
+                            store_c_chunk<OutT>(c, p, row, col + 32u, r[i + 1]);
+                        } else if constexpr (std::is_same<OutT, MxOut>::value) {
+                            if (g == 0u) {
+                                out_stage_free(lane);
+                            }
+                            uint32_t o[8], byte0, byte1;
+                            mx_quantise_chunk(p, r[i], o, byte0);
+                            out_stage_put(stage_out, lane, g * 2u, o);
+                            mx_quantise_chunk(p, r[i + 1], o, byte1);
+                            out_stage_put(stage_out, lane, g * 2u + 2u, o);
+                            scale_word |= (byte0 | (byte1 << 8)) << (8u * g);
+                            if (g == 2u) {
+                                out_stage_send(stage_out, &tmap_c, lane, inside, u.n0 + col0, row0);
+                                store_scale_word(p, row, u.n0 + col0, scale_word);
+                            }
+                        } else {
                             out_stage_free(lane);
+                            out_stage_put_chunk<OutT>(stage_out, lane, 0u, r[i]);
+                            out_stage_put_chunk<OutT>(stage_out, lane, 4u, r[i + 1]);
+                            out_stage_send(stage_out, &tmap_c, lane, inside && col < p.N, col, row0);
                         }
-                        uint32_t o[8], byte0, byte1;
-                        mx_quantise_chunk(p, r0, o, byte0);
-                        out_stage_put(stage_out, lane, g * 4u, o);
-                        mx_quantise_chunk(p, r1, o, byte1);
-                        out_stage_put(stage_out, lane, g * 4u + 2u, o);
-                        scale_word |= (byte0 | (byte1 << 8)) << (16u * g);
-                        if (g == 1u) {
-                            out_stage_send(stage_out, &tmap_c, lane, inside, u.n0 + col0, row0);
-                            store_scale_word(p, row, u.n0 + col0, scale_word);
-                        }
-                    } else {
-                        out_stage_free(lane);
-                        out_stage_put_chunk<OutT>(stage_out, lane, 0u, r0);
-                        out_stage_put_chunk<OutT>(stage_out, lane, 4u, r1);
-                        out_stage_send(stage_out, &tmap_c, lane, inside && col < p.N, col, row0);
                     }
                 }
             }

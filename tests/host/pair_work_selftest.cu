@@ -9,10 +9,13 @@
 
 using namespace catccos;
 
-static int check(uint32_t m, uint32_t n, uint32_t k, uint32_t max_pairs, uint32_t parts)
+static int check(uint32_t m, uint32_t n, uint32_t k, uint32_t max_pairs, uint32_t parts, bool gated)
 {
     GemmParams p;
     memset(&p, 0, sizeof(p));
+    uint32_t word = 0;
+    p.flags = gated ? &word : nullptr;
+    p.world = 1;
     p.Mg = m;
     p.N = n;
     p.K = k;
@@ -32,7 +35,7 @@ static int check(uint32_t m, uint32_t n, uint32_t k, uint32_t max_pairs, uint32_
             const PairUnit u = w.unit(i, p);
             const uint32_t tile = u.m0 / 256 * w.n_tiles + u.n_tile;
             if (tile >= tiles || u.kt0 >= u.kt1 || u.kt1 > k / 128 || u.n0 != u.n_tile * 256) return 1;
-            if (u.split && i + 1 != w.units) return 2;  // a split unit is a pair's last
+            if (u.last != (i + 1 == w.units) || (u.split && (gated ? !u.last : i != 0))) return 2;  // a split unit comes first, in a gated launch last
             if (u.split) {
                 const uint32_t slot = u.rem_ix * w.ksplit + u.part;
                 if (slot >= max_pairs || slots[slot]++ != 0) return 3;
@@ -51,7 +54,7 @@ int main()
             for (uint32_t n : {16u, 256u, 272u, 2304u, 7168u})
                 for (uint32_t k : {128u, 384u, 2304u, 7168u})
                     for (uint32_t parts = 1; parts <= kSplitKMax; ++parts)
-                        if (int rc = check(m, n, k, pairs, parts)) {
+                        if (int rc = check(m, n, k, pairs, parts, false) + 10 * check(m, n, k, pairs, parts, true)) {
                             printf("m %u n %u k %u pairs %u parts %u: %d\n", m, n, k, pairs, parts, rc);
                             return 1;
                         }
