@@ -812,14 +812,24 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                         CATCCOS_TR_ADD(p.trace, kTrProdFlagWaitNs, CATCCOS_TR_NOW() - t0);
                     }
                 }
-                if (lane == 0 && alive) {
-                    const uint32_t s = it % kStages;
-                    const uint32_t ph = (it / kStages) & 1u;
-                    if (it >= early) {
-                        const unsigned long long t1 = CATCCOS_TR_NOW();
-                        (void)t1;
-                        alive = mbar_wait(&empty[s], ph ^ 1u, p.status, 100, s, bar_ns);
+                if (!alive) {
+                    break;
+                }
+                // as in the MMA issuer the warp stays together and one elected lane issues
+                const uint32_t s = it % kStages;
+                if (it >= early) {
+                    const unsigned long long t1 = CATCCOS_TR_NOW();
+                    (void)t1;
+                    alive = mbar_wait_warp(&empty[s], ((it / kStages) & 1u) ^ 1u, p.status, 100, s, bar_ns);
+                    if (lane == 0) {
                         CATCCOS_TR_ADD(p.trace, kTrProdEmptyWaitNs, CATCCOS_TR_NOW() - t1);
+                    }
+                    if (!alive) {
+                        break;
+                    }
+                }
+                if (elect_one()) {
+                    if (it >= early) {
                         mbar_arrive_expect_tx(&full[s], tx_bytes);
                     }
                     if (kt == kt0 && ti < kTraceTiles) {
@@ -833,7 +843,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     }
                     CATCCOS_TR_STAMP(p.trace, kTrProdLastTma);
                 }
-                alive = __all_sync(0xFFFFFFFFu, alive);
+                __syncwarp();
             }
         }
     } else if (warp == 5) {
@@ -1024,13 +1034,11 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             }
             fence_proxy_async_shared();
             __syncwarp();
-            if (lane == 0) {
-                // Copy the atoms into tensor memory from here, not from the MMA issuer: one thread gets a tcgen05
-                // instruction out only every ~70 cycles, and four MMAs, three copies and a commit per K tile kept
-                // the issuer behind the tensor pipe.  Every stage has its own scale set in tensor memory, so the
-                // wait for the stage (above) also covers the set; the commit below stands in for this warp's
-                // arrival on the full barrier: the issuer sees the stage only when its scales are in place.
-                tcgen05_fence_after();
+            tcgen05_fence_after();
+            if (elect_one()) {
+                // Copy the atoms into tensor memory from here, not from the MMA issuer.  Every stage has its own scale set
+                // in tensor memory, so the wait for the stage (above) also covers the set; the commit below stands in for
+                // this warp's arrival on the full barrier: the issuer sees the stage only when its scales are in place.
                 const uint32_t hi_sf = (uint32_t)(make_smem_desc(0, 0, 128, 0) >> 32);  // 32 rows x 16 bytes, no swizzle
                 const uint32_t sf_t = tmem_base + S::kSfCol + s * S::kSfSetCols;
                 tcgen05_cp_sf_lohi(sf_t, smem_u32(sfa) >> 4, hi_sf);

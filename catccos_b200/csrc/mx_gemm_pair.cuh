@@ -260,14 +260,25 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                         CATCCOS_TR_ADD(p.trace, kTrProdFlagWaitNs, CATCCOS_TR_NOW() - t0);
                     }
                 }
-                if (lane == 0 && alive) {
-                    const uint32_t s = it % kStages;
-                    const uint32_t leader_bar = map_to_cta(smem_u32(&full[s]), 0);
-                    if (it >= early) {
-                        const unsigned long long t1 = CATCCOS_TR_NOW();
-                        (void)t1;
-                        alive = mbar_wait_cluster(&empty[s], ((it / kStages) & 1u) ^ 1u, p.status, 200, s, bar_ns);
+                if (!alive) {
+                    break;
+                }
+                // as in the MMA issuer the warp stays together and one elected lane issues
+                const uint32_t s = it % kStages;
+                const uint32_t leader_bar = map_to_cta(smem_u32(&full[s]), 0);
+                if (it >= early) {
+                    const unsigned long long t1 = CATCCOS_TR_NOW();
+                    (void)t1;
+                    alive = mbar_wait_warp(&empty[s], ((it / kStages) & 1u) ^ 1u, p.status, 200, s, bar_ns);
+                    if (lane == 0) {
                         CATCCOS_TR_ADD(p.trace, kTrProdEmptyWaitNs, CATCCOS_TR_NOW() - t1);
+                    }
+                    if (!alive) {
+                        break;
+                    }
+                }
+                if (elect_one()) {
+                    if (it >= early) {
                         mbar_arrive_expect_tx_cluster(leader_bar, tx_bytes);
                     }
                     if (kt == u.kt0 && ui < kTraceTiles) {
@@ -281,7 +292,7 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                     }
                     CATCCOS_TR_STAMP(p.trace, kTrProdLastTma);
                 }
-                alive = __all_sync(0xFFFFFFFFu, alive);
+                __syncwarp();
             }
         }
     } else if (warp == 5) {
@@ -509,14 +520,16 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             }
             fence_proxy_async_shared();
             __syncwarp();
+            // All loader warps of both CTAs report their atoms to the leader; the leader's warp j then copies K tile
+            // j's atoms of both CTAs into both CTAs' tensor memory (one cta_group::2 copy does the same offsets in
+            // the two).
             if (lane == 0) {
-                // All loader warps of both CTAs report their atoms to the leader; the leader's warp j then copies K tile
-                // j's atoms of both CTAs into both CTAs' tensor memory (one cta_group::2 copy does the same offsets in
-                // the two).
                 mbar_arrive_cluster(map_to_cta(smem_u32(&atoms[buf]), 0));
-                if (cta == 0) {
-                    alive = mbar_wait_cluster(&atoms[buf], ph, p.status, 208, buf, bar_ns) && alive;
-                    tcgen05_fence_after();
+            }
+            if (cta == 0) {
+                alive = mbar_wait_warp(&atoms[buf], ph, p.status, 208, buf, bar_ns) && alive;
+                tcgen05_fence_after();
+                if (elect_one()) {
                     if (real) {
                         const uint32_t hi_sf = (uint32_t)(make_smem_desc(0, 0, 128, 0) >> 32);
                         const uint32_t sf_t = tmem_base + S::kSfCol + buf * S::kSfGroupCols + j * S::kSfSetCols;
@@ -528,8 +541,8 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                     }
                     tcgen05_commit_pair(&sf_full[buf], 1);
                 }
+                __syncwarp();
             }
-            alive = __all_sync(0xFFFFFFFFu, alive);
             ++group;
             cur_a = nxt_a;
 #pragma unroll

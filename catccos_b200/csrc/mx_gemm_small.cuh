@@ -214,17 +214,21 @@ mx_gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             }
         }
         grid_dep_wait();
-        if (lane == 0) {
-            if (p.clear != nullptr && blockIdx.x == 0) {
-                *p.clear = StatusBlock{};
+        if (lane == 0 && p.clear != nullptr && blockIdx.x == 0) {
+            *p.clear = StatusBlock{};
+        }
+        __syncwarp();
+        // the warp stays together and one elected lane issues (mx_gemm.cuh)
+        for (uint32_t it = 0; it < n_it; ++it) {
+            const uint32_t s = it % kStages;
+            if (it >= early) {
+                alive = mbar_wait_warp(&empty[s], ((it / kStages) & 1u) ^ 1u, p.status, 300, s, bar_ns);
+                if (!alive) {
+                    break;
+                }
             }
-            for (uint32_t it = 0; alive && it < n_it; ++it) {
-                const uint32_t s = it % kStages;
+            if (elect_one()) {
                 if (it >= early) {
-                    alive = mbar_wait(&empty[s], ((it / kStages) & 1u) ^ 1u, p.status, 300, s, bar_ns);
-                    if (!alive) {
-                        break;
-                    }
                     load_w(it);
                 }
                 if (!QUANT) {
@@ -232,8 +236,8 @@ mx_gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                                 (int32_t)m0);
                 }
             }
+            __syncwarp();
         }
-        alive = __all_sync(0xFFFFFFFFu, alive);
     } else if (warp == 5) {
         // ------------------------------- MMA issuer ---------------------------------------
         const bool wk = p.w_kmajor != 0u;
