@@ -497,7 +497,8 @@ int encode_map_2d_uncached(CUtensorMap* map, const void* base, uint64_t inner, u
     const CUtensorMapDataType dt = fp4 ? CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B
                                        : (elem == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8);
     CU_TRY(g.drv.TensorMapEncodeTiled(map, dt, 2, const_cast<void*>(base), dims, strides, box,
-                                      estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                      estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                      !fp4 && box_inner * elem == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
                                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
     return 0;
 }
@@ -616,9 +617,9 @@ int launch_gemm_pair_inst(uint32_t max_pairs, uint32_t tiles, uint32_t parts, cu
 // What the tilings cost, in microseconds measured on B200 (kernel alone, back to back): a launch of one K tile, each
 // further K tile of a round with every SM busy, and what splitting K adds (partial tiles written, flagged, read, added;
 // more where more of them cross).  Used only to pick one.
-constexpr double kBasePair = 4.7, kBaseSingle256 = 4.0, kBaseSingle128 = 2.9;
-constexpr double kPeriodPair = 0.37, kPeriodSingle256 = 0.43, kPeriodSingle128 = 0.39;
-constexpr double kSplitCost = 3.5, kSplitCostPerCta = 0.012;
+constexpr double kBasePair = 4.7, kBaseSingle256 = 4.0, kBaseSingle128 = 2.9, kBaseSingle64 = 2.9;
+constexpr double kPeriodPair = 0.35, kPeriodSingle256 = 0.41, kPeriodSingle128 = 0.36, kPeriodSingle64 = 0.30;
+constexpr double kSplitCost = 4.3, kSplitCostPerCta = 0.012;
 // with whole tiles to follow, beside which the exchange passes (but the partial tiles' traffic does not)
 constexpr double kSplitFirstCost = 3.0, kSplitFirstCostPerCta = 0.024;
 
@@ -629,14 +630,15 @@ struct GemmPlan {
 };
 
 // Tiling of one GEMM launch: CTA pairs or single CTAs, tile width, and the number of K parts.
-GemmPlan plan_gemm(const RankCtx& rc, uint32_t Mg, uint32_t N, uint32_t K, bool no_split = false)
+// whole_tiles: K stays in one piece; wide: only the tile widths every variant of the kernel has (128 and more).
+GemmPlan plan_gemm(const RankCtx& rc, uint32_t Mg, uint32_t N, uint32_t K, bool whole_tiles = false, bool wide = false)
 {
     const uint32_t m128 = (Mg + 127) / 128, m256 = (Mg + 255) / 256;
-    const uint32_t n128 = (N + 127) / 128, n256 = (N + 255) / 256;
+    const uint32_t n256 = (N + 255) / 256;
     const uint32_t sms = (uint32_t)rc.num_sms, max_pairs = sms / 2;
     const uint32_t k_tiles = K / kGemmBlockK;
     // Splitting needs the scratch (the allocation-free entry point has none).
-    const bool may_split = rc.splitk_ws != nullptr && g.split_k != 1 && !no_split;
+    const bool may_split = rc.splitk_ws != nullptr && g.split_k != 1 && !whole_tiles;
     const uint32_t cap = may_split ? (g.split_k >= 2 ? (uint32_t)g.split_k : kSplitKMax) : 1u;
     const bool forced_split = g.split_k >= 2;
     auto split_cost = [](uint32_t ctas) { return kSplitCost + kSplitCostPerCta * ctas; };
@@ -658,8 +660,9 @@ GemmPlan plan_gemm(const RankCtx& rc, uint32_t Mg, uint32_t N, uint32_t K, bool 
     // single CTAs: rounds of whole tiles, or, when the tiles leave at least half of the SMs idle, every (tile, K part) on
     // its own CTA (a power of two that divides the K tiles, at least four K tiles per part, one part per 32 columns)
     auto single = [&](uint32_t bn, uint32_t* parts) {
-        const uint32_t t1 = m128 * (bn == 128 ? n128 : n256);
-        const double base = bn == 128 ? kBaseSingle128 : kBaseSingle256, period = bn == 128 ? kPeriodSingle128 : kPeriodSingle256;
+        const uint32_t t1 = m128 * ((N + bn - 1) / bn);
+        const double base = bn == 256 ? kBaseSingle256 : (bn == 128 ? kBaseSingle128 : kBaseSingle64);
+        const double period = bn == 256 ? kPeriodSingle256 : (bn == 128 ? kPeriodSingle128 : kPeriodSingle64);
         double best = base + (double)((t1 + sms - 1) / sms) * k_tiles * period;
         *parts = 1;
         for (uint32_t s = 2; s <= std::min(std::min(cap, sms / t1), bn / 32u); s *= 2) {
@@ -674,19 +677,28 @@ GemmPlan plan_gemm(const RankCtx& rc, uint32_t Mg, uint32_t N, uint32_t K, bool 
         }
         return best;
     };
-    uint32_t parts128 = 1, parts256 = 1;
-    const double t_128 = single(128, &parts128);
-    const double t_256 = single(256, &parts256);
-    uint32_t bn = (uint32_t)g.block_n;
-    if (bn != 128 && bn != 256) {
-        bn = (N > 128 && t_256 <= t_128) ? 256 : 128;
+    const uint32_t widths[3] = {256, 128, 64};
+    const uint32_t asked = wide && g.block_n == 64 ? 0u : (uint32_t)g.block_n;
+    uint32_t bn = 0, parts = 1;
+    double t_single = 0.0;
+    for (uint32_t w : widths) {
+        if (asked != 0 ? w != asked : ((w == 64 && wide) || (w == 256 && N <= 128))) {
+            continue;
+        }
+        uint32_t s = 1;
+        const double t = single(w, &s);
+        if (bn == 0 || t < t_single) {
+            bn = w;
+            parts = s;
+            t_single = t;
+        }
     }
 
     GemmPlan plan;
-    plan.use_pair = g.cta_pair == 1 || (g.cta_pair == 0 && g.block_n == 0 && t_pair < (bn == 256 ? t_256 : t_128));
+    plan.use_pair = g.cta_pair == 1 || (g.cta_pair == 0 && g.block_n == 0 && t_pair < t_single);
     plan.block_n = plan.use_pair ? kPairBlockN : bn;
-    plan.ksplit = plan.use_pair ? pair_parts : (bn == 256 ? parts256 : parts128);
-    plan.time = plan.use_pair ? t_pair : (bn == 256 ? t_256 : t_128);
+    plan.ksplit = plan.use_pair ? pair_parts : parts;
+    plan.time = plan.use_pair ? t_pair : t_single;
     return plan;
 }
 
@@ -732,7 +744,8 @@ SmallPlan plan_small(const RankCtx& rc, uint32_t M, uint32_t N, uint32_t K, bool
             if (quant) {
                 period = (s.mt == 16 ? kSmallQuant16 : kSmallQuant32) * (tiles * parts > sms ? kSmallQuantShared : 1.0);
             }
-            double t = rounds * kSmallBase + std::max(((k_tiles + parts - 1) / parts) * period * rounds, stream);
+            const double loop = ((k_tiles + parts - 1) / parts) * period * rounds;
+            double t = rounds * kSmallBase + std::max(loop, stream) + 0.2 * std::min(loop, stream);
             if (parts > 1) {
                 t += s.mt == 16 ? kSmallExchange16 : kSmallExchange32 + kSmallExchange32PerRow * (s.mt / parts);
             }
@@ -899,7 +912,7 @@ int launch_gemm(RankCtx& rc, cudaStream_t st, const void* a, const void* b, Gemm
             return launch_small(rc, st, small, a, b, sp, mx_out);
         }
     }
-    const GemmPlan plan = plan_gemm(rc, p.Mg, p.N, p.K, scatter);  // scatter: the owner adds whole tiles, K stays in one piece
+    const GemmPlan plan = plan_gemm(rc, p.Mg, p.N, p.K, scatter, scatter || fused_quant || p.flags != nullptr);  // scatter: the owner adds whole tiles, K stays in one piece
     const bool use_pair = plan.use_pair;
     const uint32_t bn = plan.block_n, ksplit = plan.ksplit;
     const uint32_t m256 = (p.Mg + 255) / 256;
@@ -943,7 +956,8 @@ int launch_gemm(RankCtx& rc, cudaStream_t st, const void* a, const void* b, Gemm
     CUtensorMap ta, tb;
     int rcode = encode_map_2d(&ta, a, p.K, p.Mg, kGemmBlockK, kGemmBlockM, a_fp4);
     if (rcode != 0) return rcode;
-    rcode = b_fp4 ? encode_map_2d(&tb, b, p.K, p.N, kGemmBlockK, bn, true) : encode_map_2d(&tb, b, p.N, p.K, 128, kGemmBlockK, false);
+    rcode = b_fp4 ? encode_map_2d(&tb, b, p.K, p.N, kGemmBlockK, bn, true)
+                  : encode_map_2d(&tb, b, p.N, p.K, std::min(bn, 128u), kGemmBlockK, false);
     if (rcode != 0) return rcode;
     const uint32_t tiles = ((p.Mg + kGemmBlockM - 1) / kGemmBlockM) * ((p.N + bn - 1) / bn);
     int grid = (int)(tiles < (uint32_t)rc.num_sms ? tiles : (uint32_t)rc.num_sms);
@@ -972,6 +986,13 @@ int launch_gemm(RankCtx& rc, cudaStream_t st, const void* a, const void* b, Gemm
     CATCCOS_GEMM_CASE(256)
     CATCCOS_GEMM_CASE(128)
 #undef CATCCOS_GEMM_CASE
+    if (bn == 64) {
+        if (mx_out) {
+            return launch_gemm_inst<64, MxOut, false>(grid, st, ta, tb, p, overlap_predecessor);
+        }
+        return f16 ? launch_gemm_inst<64, __half, false>(grid, st, ta, tb, p, overlap_predecessor)
+                   : launch_gemm_inst<64, __nv_bfloat16, false>(grid, st, ta, tb, p, overlap_predecessor);
+    }
     return CATCCOS_B200_EINVAL;
 }
 
@@ -1116,7 +1137,7 @@ int allgather_matmul(void* stream, const void* a, const void* a_scale, bool preq
     {
         // a split-K GEMM on this rank wants the first K segment of each of its K parts first, then the second
         // of each, ... (every rank takes the same decision)
-        const GemmPlan plan = plan_gemm(rc, W * M, N, K);
+        const GemmPlan plan = plan_gemm(rc, W * M, N, K, false, true);
         const uint32_t segs = seg.segs_per_chunk;
         if (plan.ksplit > 1 && segs <= 32 && segs > 1) {
             const uint32_t kper = K / kGemmBlockK / plan.ksplit, seg_ktiles = seg.seg_cols / kGemmBlockK;
@@ -1897,7 +1918,7 @@ int catccos_b200_mx_gemm_quant_out(void* stream, const void* a, const void* a_sc
 // Matmul + ReduceScatter: what plan_gemm will choose for the N tile (the reducer walks the same tiles)
 static uint32_t scatter_block_n(const RankCtx& rc, uint32_t M, uint32_t N, uint32_t K)
 {
-    return plan_gemm(rc, M, N, K, true).block_n;
+    return plan_gemm(rc, M, N, K, true, true).block_n;
 }
 
 int catccos_b200_mxfp8_matmul_reduce_scatter(void* stream, const void* a, const void* b, const void* a_scale,
@@ -2050,7 +2071,7 @@ int catccos_b200_set_option(const char* key, int64_t value)
         g.b_dtype = (int)value;
     } else if (k == "timeout_ms" && value > 0 && value <= 600000) {
         g.timeout_ns = (uint64_t)value * 1000000ull;
-    } else if (k == CATCCOS_B200_OPT_BLOCK_N && (value == 0 || value == 128 || value == 256)) {
+    } else if (k == CATCCOS_B200_OPT_BLOCK_N && (value == 0 || value == 64 || value == 128 || value == 256)) {
         g.block_n = (int)value;
     } else if (k == CATCCOS_B200_OPT_PHASE_MASK && value >= 1 && value <= 3) {
         g.phase_mask = (int)value;

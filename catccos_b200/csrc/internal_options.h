@@ -3,7 +3,7 @@
 // kernel variant through the same C ABI the operators use; a caller never needs them.
 #pragma once
 
-// 0 = automatic, 128 or 256: width of the single-CTA GEMM tile
+// 0 = automatic, 64, 128 or 256: width of the single-CTA GEMM tile
 #define CATCCOS_B200_OPT_BLOCK_N "block_n"
 // bit 0 = launch the producer half, bit 1 = launch the consumer half (default 3).  The harness that hosts
 // several ranks on ONE GPU runs every rank's producer before any consumer, because kernels of different

@@ -11,7 +11,7 @@
 //   SFB    E8M0 bytes in the reference's file layout [K/64, N, 2]
 //   C      bf16 or fp16, row-major [Mg, N]
 //
-// One CTA per 128 x BLOCK_N output tile, persistent over tiles, 320 threads:
+// One CTA per 128 x BLOCK_N output tile (256, 128 or 64 columns), persistent over tiles, 320 threads:
 //   warps 0-3 epilogue: tcgen05.ld of the fp32 accumulator, convert, 16-byte global stores
 //   warp 4    TMA producer: A and B tiles (128-byte swizzle) into a ring of shared-memory stages
 //   warp 5    MMA issuer: four tcgen05.mma.kind::mxf8f6f4.block_scale (K = 32 each) and one
@@ -103,9 +103,10 @@ struct GemmParams {
 
 template <uint32_t BLOCK_N>
 struct GemmSmem {
-    static constexpr uint32_t kStages = (BLOCK_N == 256) ? 4 : 6;
+    static constexpr uint32_t kStages = BLOCK_N == 256 ? 4 : (BLOCK_N == 128 ? 6 : 8);
     static constexpr uint32_t kABytes = kGemmBlockM * kGemmBlockK;
     static constexpr uint32_t kBBytes = BLOCK_N * kGemmBlockK;
+    static constexpr uint32_t kBRow = BLOCK_N < 128 ? BLOCK_N : 128;  // bytes of a K row in shared memory: one swizzle row
     static constexpr uint32_t kSfaBytes = 512;
     static constexpr uint32_t kSfbAtoms = (BLOCK_N + 127) / 128;
     static constexpr uint32_t kSfbBytes = kSfbAtoms * 512;
@@ -120,7 +121,7 @@ struct GemmSmem {
     static constexpr uint32_t kOffTmemPtr = kOffBar + kNumBars * 8;
     static constexpr uint32_t kOffGate = kOffTmemPtr + 8;  // K-tile iterations whose rows the producer has seen ready
     static constexpr uint32_t kBytes = kOffTmemPtr + 16;
-    static_assert(4 * 49152 <= kOffSfa, "the split-K pieces land in the idle operand stages");
+    static_assert(kOffSfa >= 4 * 12 * 4096, "the split-K pieces land in the idle operand stages");
     static constexpr uint32_t kDynamicBytes = kBytes + 1024;  // slack to align the base to 1024 bytes
     // Tensor memory: two 128 x BLOCK_N fp32 accumulators and one set of scale factors per stage (12 columns:
     // SFA 4, then SFB 4 per 128 columns of N).  For BLOCK_N = 256 the accumulators overlap by 64 columns
@@ -695,7 +696,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 {
     using S = GemmSmem<BLOCK_N>;
     constexpr uint32_t kStages = S::kStages;
-    static_assert(BLOCK_N == 128 || BLOCK_N == 256, "tile widths wired up: 128 and 256");
+    static_assert(BLOCK_N == 64 || BLOCK_N == 128 || BLOCK_N == 256, "tile widths wired up: 64, 128 and 256");
     static_assert(kSfWarps <= kStages, "a scale loader would take a stale phase of a stage for the one it waits for");
 
     grid_dep_launch();  // what follows on the stream may be set up meanwhile; it waits for this kernel before it reads
@@ -768,8 +769,8 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 // the transposed copy [N, K]: box = 128 (K, contiguous) x BLOCK_N rows
                 tma_load_2d(smem + S::kOffB + s * S::kBBytes, &tmap_b, &full[s], (int32_t)(kt * kGemmBlockK), (int32_t)n0);
             } else {
-                // B is [K, N] row-major: box = 128 (N, contiguous) x 128 (K); one box per 128 columns
-                for (uint32_t h = 0; h < BLOCK_N / 128; ++h) {
+                // B is [K, N] row-major: box = 128 (N, contiguous; or the tile's 64) x 128 (K); one box per 128 columns
+                for (uint32_t h = 0; h < BLOCK_N / S::kBRow; ++h) {
                     tma_load_2d(smem + S::kOffB + s * S::kBBytes + h * 16384u, &tmap_b, &full[s], (int32_t)(n0 + h * 128u),
                                 (int32_t)(kt * kGemmBlockK));
                 }
@@ -864,11 +865,13 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         // B: MN-major, 128-byte swizzle: 128 columns contiguous, K rows 128 bytes apart, 8-row K groups
         // 1024 bytes apart (SBO), 128-column groups 16 KiB apart (LBO).
         const uint32_t hi_a = (uint32_t)(make_smem_desc(0, 16, 1024, 2) >> 32);
-        const uint32_t hi_b = bk ? hi_a : (uint32_t)(make_smem_desc(0, 16384, 1024, 2) >> 32);
+        // (64-column tiles: rows of 64 bytes, 64-byte swizzle, 8-row K groups 512 bytes apart)
+        const uint64_t desc_b = bk ? make_smem_desc(0, 16, 1024, 2) : make_smem_desc(0, 16384, 8 * S::kBRow, S::kBRow == 64 ? 4 : 2);
+        const uint32_t hi_b = (uint32_t)(desc_b >> 32);
         const uint32_t a_lo0 = (uint32_t)make_smem_desc(0, 16, 1024, 2) | (smem_u32(smem + S::kOffA) >> 4);
-        const uint32_t b_lo0 = (uint32_t)make_smem_desc(0, bk ? 16 : 16384, 1024, 2) | (smem_u32(smem + S::kOffB) >> 4);
-        constexpr uint32_t kKbStepA = 32u >> 4;                // 32 bytes along K
-        const uint32_t kKbStepB = (bk ? 32u : 4096u) >> 4;     // 32 bytes along K, or 32 K rows of 128 bytes
+        const uint32_t b_lo0 = (uint32_t)desc_b | (smem_u32(smem + S::kOffB) >> 4);
+        constexpr uint32_t kKbStepA = 32u >> 4;                        // 32 bytes along K
+        const uint32_t kKbStepB = (bk ? 32u : 32u * S::kBRow) >> 4;    // 32 bytes along K, or 32 K rows
         uint32_t s = 0, ph = 0;
         for (uint32_t ti = 0; alive && ti < my_units; ++ti) {
             const uint32_t acc = ti & 1u;
@@ -941,7 +944,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         // lane, four A-scale words (rows lane, lane + 32, ...: exactly the 16 bytes of atom row `lane`)
         // and for every 128 columns of B four pairs of 16-bit halves (the file layout keeps the two
         // scales of a 64-deep K group together), and stores them as 16-byte atom rows.
-        constexpr uint32_t kNB = BLOCK_N / 32;  // B words per lane
+        constexpr uint32_t kNB = S::kSfbAtoms * 4;  // B words per lane
         const uint32_t j = warp - 6;
         if (p.flags == nullptr) {
             grid_dep_wait();  // the A scales are the output of the kernel launched just before (or: see the flags)
@@ -996,7 +999,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 const uint32_t n = n0 + i * 32 + lane;
                 rlo[i] = 0x7F7Fu;
                 rhi[i] = 0x7F7Fu;
-                if (n < p.N) {
+                if (i * 32u < BLOCK_N && n < p.N) {
                     rlo[i] = __ldg(reinterpret_cast<const uint16_t*>(p.b_scales + ((size_t)(2 * kt) * p.N + n) * 2));
                     rhi[i] = __ldg(reinterpret_cast<const uint16_t*>(p.b_scales + ((size_t)(2 * kt + 1) * p.N + n) * 2));
                 }
