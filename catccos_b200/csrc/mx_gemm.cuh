@@ -853,8 +853,8 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         // instruction cannot stay in uniform registers, and each then takes about 70 cycles to get out.  The issuer
         // issues what nobody else can (the MMAs, and the commit that releases the stage) and nothing more.
         const bool bk = p.b_kmajor != 0u;
-        const uint32_t idesc = make_idesc_mxf8(kGemmBlockM, BLOCK_N, !bk) | ((p.a_fmt & 7u) << 7) |
-                               ((p.b_fmt & 7u) << 10);  // operand formats: E4M3 = 0, E5M2 = 1, E2M1 = 5
+        const uint32_t idesc0 = make_idesc_mxf8(kGemmBlockM, 0, !bk) | ((p.a_fmt & 7u) << 7) |
+                                ((p.b_fmt & 7u) << 10);  // operand formats: E4M3 = 0, E5M2 = 1, E2M1 = 5
         const uint32_t ksplit = p.ksplit > 1u ? p.ksplit : 1u;
         const uint32_t kper = k_tiles / ksplit;  // K tiles per work unit (the host only splits evenly)
         const uint32_t num_units = num_tiles * ksplit;
@@ -886,6 +886,11 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             if (lane == 0) {
                 CATCCOS_TR_ADD(p.trace, kTrMmaAccWaitNs, CATCCOS_TR_NOW() - t0);
             }
+            // a ragged last column of tiles is multiplied as wide as it is (a multiple of 16)
+            const uint32_t unit = blockIdx.x + ti * gridDim.x;
+            const uint32_t left = p.N - tile_coord(unit % num_tiles, n_tiles, m_tiles, p).n_tile * BLOCK_N;
+            const uint32_t width = left < BLOCK_N ? (left + 15u) / 16u * 16u : BLOCK_N;
+            const uint32_t idesc = idesc0 | ((width >> 3) << 17);
             for (uint32_t kt = 0; alive && kt < kper; ++kt) {
                 const unsigned long long t1 = CATCCOS_TR_NOW();
                 (void)t1;

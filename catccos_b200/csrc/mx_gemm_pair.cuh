@@ -2,7 +2,8 @@
 //
 // Same operator, operands, layouts and flag gating as mx_gemm.cuh; what changes is the tile: a pair of
 // CTAs owns a 256 x 256 output tile.  CTA r of the pair loads A rows [m0 + 128 r, +128) and B columns
-// [n0 + 128 r, +128) of every K tile (32 KB per K tile per SM instead of 48 KB), the leader CTA (r = 0)
+// [n0 + 128 r, +128) of every K tile (32 KB per K tile per SM instead of 48 KB; a ragged last column of tiles is split
+// in two halves of what it has), the leader CTA (r = 0)
 // issues one tcgen05.mma.cta_group::2 (M = 256, N = 256, K = 32) that reads both CTAs' shared memory, and
 // each CTA ends up with the accumulator of its own 128 rows x 256 columns in its own tensor memory.
 // Every CTA loads its own tiles with plain TMA (no cluster multicast anywhere); what crosses the pair is
@@ -90,6 +91,7 @@ __host__ __device__ __forceinline__ TileCoord pair_tile_coord(uint32_t idx, uint
 // One work unit of a pair: a whole tile, or one K part of a tile of the last round.
 struct PairUnit {
     uint32_t m0, n0, n_tile;  // first row and column of the pair's tile
+    uint32_t width;           // columns that are multiplied: 256, or what a ragged last tile has, rounded up to 32
     uint32_t kt0, kt1;        // K tiles
     uint32_t part, rem_ix;    // split units: which part, and which of the rem tiles
     bool split;
@@ -137,6 +139,8 @@ struct PairWork {
         u.m0 = tc.m_tile * kPairBlockM;
         u.n0 = tc.n_tile * kPairBlockN;
         u.n_tile = tc.n_tile;
+        const uint32_t left = p.N - u.n0;
+        u.width = left < kPairBlockN ? (left + 31u) / 32u * 32u : kPairBlockN;
         return u;
     }
 };
@@ -219,7 +223,7 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         // packed 4-bit operands arrive as half the bytes they occupy in shared memory (the gaps are not written)
         const uint32_t tx_bytes = (p.a_fmt == 5u ? S::kABytes / 2u : S::kABytes) + (p.b_fmt == 5u ? S::kBBytes / 2u : S::kBBytes);
         auto load_b = [&](const PairUnit& u, uint32_t kt, uint32_t s, uint32_t leader_bar) {
-            const int32_t n = (int32_t)(u.n0 + cta * 128u), k = (int32_t)(kt * kGemmBlockK);
+            const int32_t n = (int32_t)(u.n0 + cta * (u.width / 2u)), k = (int32_t)(kt * kGemmBlockK);
             if (p.b_kmajor) {  // the transposed copy [N, K]: this CTA's columns are rows of it
                 tma_load_2d_pair(smem + S::kOffB + s * S::kBBytes, &tmap_b, leader_bar, k, n);
             } else {
@@ -302,8 +306,8 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         // issues the MMAs and the commits, nothing else.
         if (cta == 0) {
             const bool bk = p.b_kmajor != 0u;
-            const uint32_t idesc = make_idesc_mxf8(kPairBlockM, kPairBlockN, !bk) | ((p.a_fmt & 7u) << 7) |
-                                   ((p.b_fmt & 7u) << 10);  // operand formats: E4M3 = 0, E5M2 = 1, E2M1 = 5
+            const uint32_t idesc0 = make_idesc_mxf8(kPairBlockM, 0, !bk) | ((p.a_fmt & 7u) << 7) |
+                                    ((p.b_fmt & 7u) << 10);  // operand formats: E4M3 = 0, E5M2 = 1, E2M1 = 5
             const uint32_t hi_a = (uint32_t)(make_smem_desc(0, 16, 1024, 2) >> 32);
             // B, MN-major: each CTA's 128 columns are one 128-byte swizzle row per K row
             const uint64_t desc_b = bk ? make_smem_desc(0, 16, 1024, 2) : make_smem_desc(0, 16384, 1024, 2);
@@ -328,6 +332,7 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                     CATCCOS_TR_ADD(p.trace, kTrMmaAccWaitNs, CATCCOS_TR_NOW() - t0);
                 }
                 const uint32_t n_it = u.kt1 - u.kt0;
+                const uint32_t idesc = idesc0 | ((u.width >> 3) << 17);
                 for (uint32_t i = 0; alive && i < n_it; ++i) {
                     const uint32_t buf = group & 1u;
                     const unsigned long long t1 = CATCCOS_TR_NOW();

@@ -35,6 +35,7 @@ static int check(uint32_t m, uint32_t n, uint32_t k, uint32_t max_pairs, uint32_
             const PairUnit u = w.unit(i, p);
             const uint32_t tile = u.m0 / 256 * w.n_tiles + u.n_tile;
             if (tile >= tiles || u.kt0 >= u.kt1 || u.kt1 > k / 128 || u.n0 != u.n_tile * 256) return 1;
+            if (u.width % 32 != 0 || u.width > 256 || u.n0 + u.width < (n < u.n0 + 256 ? n : u.n0 + 256)) return 5;
             if (u.last != (i + 1 == w.units) || (u.split && (gated ? !u.last : i != 0))) return 2;  // a split unit comes first, in a gated launch last
             if (u.split) {
                 const uint32_t slot = u.rem_ix * w.ksplit + u.part;
