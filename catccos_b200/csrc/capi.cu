@@ -708,16 +708,23 @@ struct SmallPlan {
     uint32_t mt, parts;
 };
 
-// What it costs, as above: a launch of one K tile; each further K tile of a CTA while loads are latency-bound (with the
-// quantisation inside, four warps' work, more so with two CTAs on an SM); or, if that is longer, streaming every tile's
-// weights (rows of N bytes that are no multiple of 128 straddle two lines each); and the exchange of the parts.  CTAs
-// beyond two per SM start when others end and pay their start again, so splitting stops there.  A
-// quantiser in front costs a launch and a dependency, more in front of the kernels that need a whole SM's shared memory.
-constexpr double kSmallBase = 2.9, kSmallPeriod = 0.24, kSmallQuant16 = 0.40, kSmallQuant32 = 0.85, kSmallQuantShared = 1.5;
-constexpr double kSmallBytesPerUs = 6.0e6, kSmallBytesPerUsRagged = 3.3e6;
-constexpr double kSmallExchange16 = 0.8, kSmallExchange32 = 1.1, kSmallExchange32PerRow = 0.06;
+// What it costs, in microseconds, as a launch of one K tile; each further K tile of a CTA while loads are latency-bound
+// (with the quantisation inside, four warps' work); or, if that is longer, streaming every tile's weights (rows of N
+// bytes that are no multiple of 128 straddle two lines each); and the exchange of the parts.  A quantiser in front costs
+// a launch and a dependency.  The constants are fitted to 54 sizes x 4 to 8 variants measured on B200 (1 <= M <= 256,
+// 1024 <= N <= 7168, 1024 <= K <= 7168): estimates are off by 8 %, and the variant they choose by 0.7 % from the fastest.
+constexpr double kSmallBase = 2.9, kSmallPeriod16 = 0.23, kSmallPeriod32 = 0.24, kSmallQuant16 = 0.37, kSmallQuant32 = 0.79;
+constexpr double kSmallQuantShared = 1.45;  // two CTAs on an SM
+constexpr double kSmallBytesPerUs = 7.4e6, kSmallBytesPerUsRagged = 5.1e6, kSmallHidden = 0.73;
+constexpr double kSmallExchange16 = 0.6, kSmallExchange32 = 1.5, kSmallExchange32PerRow = 0.03;
 constexpr double kSmallMxOutPerRow = 0.08;  // a warp takes the block maximum of one row at a time
-constexpr double kQuantiserSmall = 1.6, kQuantiserLarge = 2.5;
+constexpr double kQuantiserSmall = 1.6, kQuantiserLarge = 1.8;
+
+// Clusters of `parts` CTAs that are resident at once, two CTAs on an SM (148, 71 and 33 of 2, 4 and 8 on 148 SMs).
+uint32_t small_clusters(uint32_t sms, uint32_t parts)
+{
+    return parts == 1 ? 2 * sms : (parts == 2 ? sms : (parts == 4 ? sms * 71 / 148 : sms * 33 / 148));
+}
 
 SmallPlan plan_small(const RankCtx& rc, uint32_t M, uint32_t N, uint32_t K, bool bf16_in, bool mx_out = false)
 {
@@ -729,23 +736,25 @@ SmallPlan plan_small(const RankCtx& rc, uint32_t M, uint32_t N, uint32_t K, bool
     const uint32_t tiles = ((M + s.mt - 1) / s.mt) * ((N + kSmallBlockN - 1) / kSmallBlockN), k_tiles = K / kGemmBlockK;
     const uint32_t cap = std::min(g.split_k >= 1 ? (uint32_t)g.split_k : kSmallMaxParts, k_tiles);
     const uint32_t sms = (uint32_t)rc.num_sms;
-    const double stream = (double)tiles * k_tiles * (kSmallBlockN * kGemmBlockK) / (N % 128u == 0u ? kSmallBytesPerUs : kSmallBytesPerUsRagged);
+    const double stream = (double)tiles * k_tiles * (kSmallBlockN * kGemmBlockK) /
+                          (N % 128u == 0u ? kSmallBytesPerUs : kSmallBytesPerUsRagged);
     double best = 0.0;
     for (uint32_t quant = 0; quant <= (bf16_in ? 1u : 0u); ++quant) {
         if (bf16_in && g.small_quant != 0 && (quant != 0) != (g.small_quant == 1)) {
             continue;
         }
         for (uint32_t parts = 1; parts <= cap; parts *= 2) {
-            if (parts > 1 && tiles * parts > 2 * sms && g.split_k <= 1) {
-                break;
+            const uint32_t resident = small_clusters(sms, parts);
+            if (parts > 1 && tiles > resident && g.split_k <= 1) {
+                break;  // clusters that wait for a place pay their start again
             }
-            const double rounds = (double)((tiles * parts + 2 * sms - 1) / (2 * sms));
-            double period = kSmallPeriod;
+            const double rounds = (double)((tiles + resident - 1) / resident);
+            double period = s.mt == 16 ? kSmallPeriod16 : kSmallPeriod32;
             if (quant) {
                 period = (s.mt == 16 ? kSmallQuant16 : kSmallQuant32) * (tiles * parts > sms ? kSmallQuantShared : 1.0);
             }
             const double loop = ((k_tiles + parts - 1) / parts) * period * rounds;
-            double t = rounds * kSmallBase + std::max(loop, stream) + 0.2 * std::min(loop, stream);
+            double t = rounds * kSmallBase + std::max(loop, stream) + (1.0 - kSmallHidden) * std::min(loop, stream);
             if (parts > 1) {
                 t += s.mt == 16 ? kSmallExchange16 : kSmallExchange32 + kSmallExchange32PerRow * (s.mt / parts);
             }
