@@ -165,6 +165,7 @@ struct State {
     int a_dtype = 0;         // element type of the A codes (what the quantiser writes, what the GEMM reads): 0 = E4M3, 1 = E5M2
     int b_dtype = 0;         // element type of the B codes the caller passes
     int split_k = 0;         // 0 = automatic, 1 = never split K, 2..8 = split K in that many parts when it fits
+    int b_lsu = 0;           // 0 = automatic, 1 = B through the load/store units, 2 = through TMA
     int small_tile = 0;      // 0 = automatic, 1 = always the small-tile kernel where it can run, 2 = never
     int small_quant = 0;     // 0 = automatic, 1 = the small-tile kernel quantises a fused call itself, 2 = never
     int tile_order = -1;     // gated GEMM: -1 = automatic, 1 = own shard first, 0 = slice by slice over all ranks
@@ -518,7 +519,7 @@ int launch_gemm_inst(int grid, cudaStream_t st, const CUtensorMap& ta, const CUt
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(FUSED ? kGemmFusedThreads : kGemmThreads);
+    cfg.blockDim = dim3(FUSED ? kGemmFusedThreads : kGemmThreads + (p.b_lsu ? kBLoadWarps * 32 : 0));
     cfg.dynamicSmemBytes = GemmSmem<BLOCK_N>::kDynamicBytes;
     cfg.stream = st;
     cudaLaunchAttribute attr;
@@ -619,6 +620,7 @@ int launch_gemm_pair_inst(uint32_t max_pairs, uint32_t tiles, uint32_t parts, cu
 // more where more of them cross).  Used only to pick one.
 constexpr double kBasePair = 4.7, kBaseSingle256 = 4.0, kBaseSingle128 = 2.9, kBaseSingle64 = 2.9;
 constexpr double kPeriodPair = 0.35, kPeriodSingle256 = 0.41, kPeriodSingle128 = 0.36, kPeriodSingle64 = 0.30;
+constexpr double kRagged = 1.2, kRagged64 = 1.12;  // N no multiple of 32: every other K row of B starts inside a sector
 constexpr double kSplitCost = 4.3, kSplitCostPerCta = 0.012;
 // with whole tiles to follow, beside which the exchange passes (but the partial tiles' traffic does not)
 constexpr double kSplitFirstCost = 3.0, kSplitFirstCostPerCta = 0.024;
@@ -641,28 +643,30 @@ GemmPlan plan_gemm(const RankCtx& rc, uint32_t Mg, uint32_t N, uint32_t K, bool 
     const bool may_split = rc.splitk_ws != nullptr && g.split_k != 1 && !whole_tiles;
     const uint32_t cap = may_split ? (g.split_k >= 2 ? (uint32_t)g.split_k : kSplitKMax) : 1u;
     const bool forced_split = g.split_k >= 2;
+    const double ragged = N % 32u != 0u ? kRagged : 1.0, ragged64 = N % 32u != 0u ? kRagged64 : 1.0;
+    const double pair_period = kPeriodPair * ragged;
     auto split_cost = [](uint32_t ctas) { return kSplitCost + kSplitCostPerCta * ctas; };
 
     // CTA pairs: whole rounds, and a last round whose tiles are cut in as many parts as shorten it
     const uint32_t tiles = m256 * n256, rem = tiles % max_pairs;
     uint32_t pair_parts = 1;
-    double last = rem != 0 ? k_tiles * kPeriodPair : 0.0;
+    double last = rem != 0 ? k_tiles * pair_period : 0.0;
     for (uint32_t s = 2; rem != 0 && s <= std::min(std::min(cap, max_pairs / rem), k_tiles); ++s) {
         const double cost = tiles >= max_pairs ? kSplitFirstCost + kSplitFirstCostPerCta * 2 * rem * s : split_cost(2 * rem * s);
-        const double t = ((k_tiles + s - 1) / s) * kPeriodPair + cost;
+        const double t = ((k_tiles + s - 1) / s) * pair_period + cost;
         if (t < last) {
             last = t;
             pair_parts = s;
         }
     }
-    const double t_pair = kBasePair + (tiles / max_pairs) * k_tiles * kPeriodPair + last;
+    const double t_pair = kBasePair + (tiles / max_pairs) * k_tiles * pair_period + last;
 
     // single CTAs: rounds of whole tiles, or, when the tiles leave at least half of the SMs idle, every (tile, K part) on
     // its own CTA (a power of two that divides the K tiles, at least four K tiles per part, one part per 32 columns)
     auto single = [&](uint32_t bn, uint32_t* parts) {
         const uint32_t t1 = m128 * ((N + bn - 1) / bn);
         const double base = bn == 256 ? kBaseSingle256 : (bn == 128 ? kBaseSingle128 : kBaseSingle64);
-        const double period = bn == 256 ? kPeriodSingle256 : (bn == 128 ? kPeriodSingle128 : kPeriodSingle64);
+        const double period = bn == 256 ? kPeriodSingle256 * ragged : (bn == 128 ? kPeriodSingle128 * ragged : kPeriodSingle64 * ragged64);
         double best = base + (double)((t1 + sms - 1) / sms) * k_tiles * period;
         *parts = 1;
         for (uint32_t s = 2; s <= std::min(std::min(cap, sms / t1), bn / 32u); s *= 2) {
@@ -971,6 +975,8 @@ int launch_gemm(RankCtx& rc, cudaStream_t st, const void* a, const void* b, Gemm
     const uint32_t tiles = ((p.Mg + kGemmBlockM - 1) / kGemmBlockM) * ((p.N + bn - 1) / bn);
     int grid = (int)(tiles < (uint32_t)rc.num_sms ? tiles : (uint32_t)rc.num_sms);
     p.ksplit = ksplit;
+    p.b = static_cast<const uint8_t*>(b);
+    p.b_lsu = bn == 64 && !b_fp4 && (g.b_lsu == 0 ? p.N % 32u != 0u : g.b_lsu == 1) ? 1u : 0u;
     if (ksplit > 1) {
         grid = (int)(tiles * ksplit);  // <= SMs by construction: all units are resident at once
     }
@@ -2090,6 +2096,8 @@ int catccos_b200_set_option(const char* key, int64_t value)
         g.fuse_mode = (int)value;
     } else if (k == CATCCOS_B200_OPT_SPLIT_K && value >= 0 && value <= 8) {
         g.split_k = (int)value;
+    } else if (k == CATCCOS_B200_OPT_B_LSU && value >= 0 && value <= 2) {
+        g.b_lsu = (int)value;
     } else if (k == CATCCOS_B200_OPT_SMALL_TILE && value >= 0 && value <= 2) {
         g.small_tile = (int)value;
     } else if (k == CATCCOS_B200_OPT_SMALL_QUANT && value >= 0 && value <= 2) {

@@ -252,6 +252,23 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, ui
         : "memory");
 }
 
+// 16-byte copy global -> shared by the load/store units; zeros when !inside (then nothing is read).
+__device__ __forceinline__ void cp_async_16(uint32_t smem_dst, const void* gsrc, bool inside)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_dst), "l"(gsrc), "r"(inside ? 16u : 0u) : "memory");
+}
+
+__device__ __forceinline__ void cp_async_commit()
+{
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+template <int kPending>
+__device__ __forceinline__ void cp_async_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
+}
+
 // Tiled store shared -> global (the async proxy reads shared memory: fence_proxy_async_shared() first).  Elements outside
 // the tensor are not written.
 __device__ __forceinline__ void tma_store_2d(const void* tmap, const void* smem_src, int32_t x, int32_t y)

@@ -22,6 +22,8 @@
 // 0 = automatic (K is cut in up to eight parts when the output tiles would leave half of the SMs idle),
 // 1 = never, 2..8 = at most that many parts
 #define CATCCOS_B200_OPT_SPLIT_K "split_k"
+// 8-bit weights of a GEMM: 0 = automatic, 1 = loaded by the load/store units, 2 = by TMA
+#define CATCCOS_B200_OPT_B_LSU "b_lsu"
 // small-tile kernel (one GPU, no flags): 0 = automatic, 1 = always where it can run, 2 = never
 #define CATCCOS_B200_OPT_SMALL_TILE "small_tile"
 // a fused call on the small-tile kernel: 0 = automatic, 1 = it quantises the activations itself, 2 = quantiser first

@@ -50,6 +50,13 @@ namespace catccos {
 constexpr uint32_t kGemmBlockM = 128;
 constexpr uint32_t kGemmBlockK = 128;   // bytes == elements (8-bit codes): one 128-byte swizzle row
 constexpr uint32_t kGemmThreads = 320;
+constexpr uint32_t kBLoadWarps = 4;     // in launches whose B comes through the load/store units (GemmParams::b_lsu)
+// Tiles whose kernel has those warps.  At 128 and 256 columns the copies themselves become the limit (509 x 2320 x 3968:
+// 17.0 and 33.9 us against 16.5 and 20.6 by TMA; at 64 columns 14.7 against 16.4).
+template <uint32_t BLOCK_N, bool FUSED_QUANT>
+constexpr bool kHasBLoad = BLOCK_N == 64 && !FUSED_QUANT;
+template <uint32_t BLOCK_N, bool FUSED_QUANT>
+constexpr uint32_t kGemmMaxThreads = FUSED_QUANT ? 320 + 256 + 192 : (kHasBLoad<BLOCK_N, FUSED_QUANT> ? 320 + kBLoadWarps * 32 : 320);
 constexpr uint32_t kPushWarps = 6;
 constexpr uint32_t kGemmFusedThreads = kGemmThreads + kQuantThreads + kPushWarps * 32;  // + eight quantise warps + six pushers
 constexpr uint32_t kSfWarps = 4;
@@ -58,6 +65,7 @@ constexpr uint32_t kTmemCols = 512;
 
 struct GemmParams {
     const uint8_t* a_scales;  // [Mg, K/32]
+    const uint8_t* b;         // [K, N]: the codes, for launches that do not read them through a tensor map (b_lsu)
     const uint8_t* b_scales;  // [K/64, N, 2]
     void* c;                  // [Mg, N]: bf16 / fp16, or E4M3 codes when the epilogue quantises (MxOut)
     uint8_t* c_scales;        // MxOut only: E8M0 [Mg, N/32], one scale per 32 output columns of a row
@@ -81,6 +89,7 @@ struct GemmParams {
     uint32_t world, rank, m_local, epoch;
     uint32_t b_early;         // 1: B and its scales were in place before the kernel launched just before this one (the
                               // quantiser of the same call): they are loaded while that kernel drains
+    uint32_t b_lsu;           // 1: B is loaded by four more warps instead of TMA (rows that start inside a sector)
     uint32_t gemm_off;        // 1: the GEMM warps stay idle (the producer half of a call, run apart)
     uint32_t own_first;       // tile order of a gated launch: 1 = this rank's whole shard first (it is there before any
                               // peer's rows), 0 = slice by slice over ALL ranks, own slice leading (every rank's
@@ -690,7 +699,7 @@ __global__ void __launch_bounds__(256) mx_reduce_scatter_kernel(const float* __r
 }
 
 template <uint32_t BLOCK_N, typename OutT, bool FUSED_QUANT>
-__global__ void __launch_bounds__(FUSED_QUANT ? kGemmFusedThreads : kGemmThreads, 1)
+__global__ void __launch_bounds__(kGemmMaxThreads<BLOCK_N, FUSED_QUANT>, 1)
 mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                const __grid_constant__ GemmParams p)
 {
@@ -725,7 +734,8 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     if (threadIdx.x == 0) {
         CATCCOS_TR_STAMP(p.trace, kTrCtaStart);
         for (uint32_t s = 0; s < kStages; ++s) {
-            mbar_init(&full[s], 2);  // the producer's expect_tx arrival and one scale-loader warp
+            // the producer's expect_tx arrival, one scale-loader warp, and the B loader warps where there are any
+            mbar_init(&full[s], 2 + (kHasBLoad<BLOCK_N, FUSED_QUANT> && p.b_lsu ? kBLoadWarps : 0u));
             mbar_init(&empty[s], 1);
         }
         for (uint32_t a = 0; a < 2; ++a) {
@@ -763,7 +773,9 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         const uint32_t num_units = num_tiles * ksplit;
         uint32_t it = 0, ti = 0;
         // packed 4-bit operands arrive as half the bytes they occupy in shared memory (the gaps are not written)
-        const uint32_t tx_bytes = (p.a_fmt == 5u ? S::kABytes / 2u : S::kABytes) + (p.b_fmt == 5u ? S::kBBytes / 2u : S::kBBytes);
+        const bool b_tma = !kHasBLoad<BLOCK_N, FUSED_QUANT> || p.b_lsu == 0u;
+        const uint32_t tx_bytes = (p.a_fmt == 5u ? S::kABytes / 2u : S::kABytes) +
+                                  (b_tma ? (p.b_fmt == 5u ? S::kBBytes / 2u : S::kBBytes) : 0u);
         auto load_b = [&](uint32_t n0, uint32_t kt, uint32_t s) {
             if (p.b_kmajor) {
                 // the transposed copy [N, K]: box = 128 (K, contiguous) x BLOCK_N rows
@@ -777,7 +789,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             }
         };
         if (p.flags == nullptr) {
-            if (p.b_early && blockIdx.x < num_units) {
+            if (p.b_early && b_tma && blockIdx.x < num_units) {
                 // the weights do not come from the kernel launched just before: fill the ring's B half meanwhile
                 const uint32_t ks = blockIdx.x / num_tiles;
                 const uint32_t n0 = tile_coord(blockIdx.x - ks * num_tiles, n_tiles, m_tiles, p).n_tile * BLOCK_N;
@@ -839,7 +851,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     CATCCOS_TR_STAMP_FIRST(p.trace, kTrProdFirstTma);
                     tma_load_2d(smem + S::kOffA + s * S::kABytes, &tmap_a, &full[s], (int32_t)(kt * kGemmBlockK),
                                 (int32_t)m0);
-                    if (it >= early) {
+                    if (it >= early && b_tma) {
                         load_b(n0, kt, s);
                     }
                     CATCCOS_TR_STAMP(p.trace, kTrProdLastTma);
@@ -942,6 +954,59 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             // pusher pw of CTA b is worker pw * grid + b: a short item list spreads over all SMs instead of
             // filling the first CTAs' six pushers
             push_worker(p.push, lane, pw * gridDim.x + blockIdx.x, gridDim.x * kPushWarps, pw, gridDim.x, push_turn);
+        }
+    } else if (kHasBLoad<BLOCK_N, FUSED_QUANT> && warp >= 10) {
+        // ------------------------------- B through the load/store units -------------------
+        // A weight whose rows are a multiple of 16 bytes but not of 32 has every other K row start inside a 32-byte sector.
+        // TMA takes about 5 cycles for such a row of 128 bytes against 1.6 for an aligned one; 16-byte asynchronous copies
+        // only pay for the fifth sector.  Each of four warps copies 32 K rows of a stage into the layout TMA would have
+        // written, three stages in flight.
+        constexpr uint32_t kRowChunks = BLOCK_N / 16, kInFlight = 3;
+        const uint32_t lw = warp - 10;
+        if (p.flags == nullptr && !p.b_early) {
+            grid_dep_wait();
+        }
+        const uint32_t ksplit = p.ksplit > 1u ? p.ksplit : 1u;
+        const uint32_t kper = k_tiles / ksplit;
+        const uint32_t num_units = num_tiles * ksplit;
+        uint32_t it = 0;
+        auto landed = [&](uint32_t done) {
+            fence_proxy_async_shared();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&full[done % kStages]);
+            }
+        };
+        for (uint32_t unit = blockIdx.x; alive && unit < num_units; unit += gridDim.x) {
+            const uint32_t ks = unit / num_tiles;
+            const uint32_t n0 = tile_coord(unit - ks * num_tiles, n_tiles, m_tiles, p).n_tile * BLOCK_N;
+            for (uint32_t kt = ks * kper; alive && kt < ks * kper + kper; ++kt, ++it) {
+                const uint32_t s = it % kStages;
+                alive = mbar_wait_warp(&empty[s], ((it / kStages) & 1u) ^ 1u, p.status, 109, s, bar_ns);
+                if (!alive) {
+                    break;
+                }
+                const uint32_t stage = smem_u32(smem + S::kOffB + s * S::kBBytes);
+#pragma unroll
+                for (uint32_t i = 0; i < kRowChunks; ++i) {
+                    const uint32_t e = i * 32u + lane;
+                    const uint32_t row = lw * 32u + e / kRowChunks, c = e % kRowChunks;
+                    const uint32_t swizzled = c ^ ((row >> 1) & 3u);  // rows of 64 bytes, 64-byte swizzle
+                    const uint32_t n = n0 + c * 16u;
+                    const bool inside = n < p.N;
+                    cp_async_16(stage + row * S::kBRow + (swizzled << 4),
+                                p.b + (size_t)(kt * kGemmBlockK + row) * p.N + (inside ? n : 0u), inside);
+                }
+                cp_async_commit();
+                if (it >= kInFlight) {
+                    cp_async_wait<kInFlight>();
+                    landed(it - kInFlight);
+                }
+            }
+        }
+        cp_async_wait<0>();
+        for (uint32_t done = it < kInFlight ? 0u : it - kInFlight; alive && done < it; ++done) {
+            landed(done);
         }
     } else if (warp >= 6) {
         // ------------------------------- scale loaders ------------------------------------

@@ -15,7 +15,7 @@ def tile64(capi, cuda):
     capi.set_option("cta_pair", 2)
     capi.set_option("block_n", 64)
     yield capi
-    for key in ("small_tile", "cta_pair", "block_n", "split_k", "c_dtype", "a_dtype"):
+    for key in ("small_tile", "cta_pair", "block_n", "split_k", "c_dtype", "a_dtype", "b_lsu"):
         capi.set_option(key, 0)
 
 
@@ -26,13 +26,15 @@ def _problem(oracle, m, n, k):
     return x, (*oracle.quantize_rows(x), *oracle.quantize_weight(w))
 
 
+@pytest.mark.parametrize("b_lsu", [1, 2])  # the weight by the load/store units, or by TMA
 @pytest.mark.parametrize("split_k", [1, 2])
 @pytest.mark.parametrize("m,n,k", [(1, 16, 128), (128, 64, 1024), (129, 80, 1152), (300, 272, 2048), (509, 528, 3968), (2000, 1040, 256)])
-def test_shapes(tile64, cuda, oracle, m, n, k, split_k):
+def test_shapes(tile64, cuda, oracle, m, n, k, split_k, b_lsu):
     _, ops = _problem(oracle, m, n, k)
     gold = oracle.allgather_matmul([ops[0]], [ops[1]], ops[2], ops[3])
     dev = [cuda.from_numpy(v).cuda() for v in ops]
     tile64.set_option("split_k", split_k)
+    tile64.set_option("b_lsu", b_lsu)
     out = tile64.mx_gemm(*dev)
     bad, most = oracle.check_close(out.float().cpu().numpy(), gold, 1e-2, 1e-3)
     assert bad == 0, (bad, most)
