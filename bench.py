@@ -35,9 +35,9 @@ METRIC = "mxfp8_allgather_matmul_tflops"
 UNIT = "TFLOP/s"
 FP8_NOMINAL_TFLOPS = 4500.0
 NVLINK_NOMINAL_GBS = 900.0
-# dram__bytes_read.sum + dram__bytes_write.sum of one launch of the dominant kernel at N = 1 (the split-K GEMM
+# dram__bytes_read.sum + dram__bytes_write.sum of one launch of the dominant kernel at N = 1 (the CTA-pair GEMM
 # on 1024 x 2304 x 7168), from an ncu capture of `bench.py --kernel gemm --m 1024 --n 2304 --k 7168`
-GEMM_DRAM_TRAFFIC_BYTES_N1 = 24.69e6
+GEMM_DRAM_TRAFFIC_BYTES_N1 = 24.70e6
 PARITY_ROWS_PER_RANK = 32
 
 
@@ -584,7 +584,7 @@ def run_gpu(args) -> None:
         "roofline": {
             "bound": "tensor", "achieved": gemm_tflops, "peak": fp8_peak, "unit": UNIT, "frac": gemm_tflops / fp8_peak,
             "traffic": GEMM_DRAM_TRAFFIC_BYTES_N1 if world == 1 else None,
-            "kernel": "mx_gemm_kernel (tcgen05.mma kind::mxf8f6f4.block_scale)",
+            "kernel": "mx_gemm_pair_kernel (tcgen05.mma cta_group::2 kind::mxf8f6f4.block_scale)",
             "kernel_ms": gemm_ms,
             "peak_source": f"2 x cuBLAS bf16 burst of {peaks['source']} ({peaks['bf16_tflops']} TFLOP/s); "
                            "the peaks file holds no fp8 figure, fp8 issues at twice the bf16 rate",

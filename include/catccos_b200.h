@@ -197,9 +197,9 @@ int catccos_b200_last_status(uint32_t out[4]);
  *   "timeout_ms"      limit of device-side waits on peers (default 2000)
  * Any other key is rejected with CATCCOS_B200_EINVAL, except the test hooks that
  * catccos_b200/csrc/internal_options.h lists (they force kernel variants and are not part of this boundary).
- * The kernels choose their own tiling: CTA pairs (256 x 256 tiles) for more than one wave of work, K cut in
- * up to eight parts when the tiles would leave half of the SMs idle (the partial tiles meet in a per-rank
- * scratch allocated when the rank is set up; because of it, and of the symmetric buffer's epochs, the operator
+ * The kernels choose their own tiling by size (CTA pairs, single CTAs, small tiles), with K cut in up to eight parts
+ * when the tiles would leave SMs idle (the partial tiles meet in a per-rank scratch allocated when the rank is set up,
+ * or in the shared memory of a cluster; because of it, and of the symmetric buffer's epochs, the operator
  * calls of one rank must not overlap on the GPU). */
 int catccos_b200_set_option(const char* key, int64_t value);
 
