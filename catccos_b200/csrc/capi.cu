@@ -615,15 +615,20 @@ int launch_gemm_pair_inst(uint32_t max_pairs, uint32_t tiles, uint32_t parts, cu
     return 0;
 }
 
-// What the tilings cost, in microseconds measured on B200 (kernel alone, back to back): a launch of one K tile, each
-// further K tile of a round with every SM busy, and what splitting K adds (partial tiles written, flagged, read, added;
-// more where more of them cross).  Used only to pick one.
-constexpr double kBasePair = 4.7, kBaseSingle256 = 4.0, kBaseSingle128 = 2.9, kBaseSingle64 = 2.9;
-constexpr double kPeriodPair = 0.35, kPeriodSingle256 = 0.41, kPeriodSingle128 = 0.36, kPeriodSingle64 = 0.30;
-constexpr double kRagged = 1.2, kRagged64 = 1.12;  // N no multiple of 32: every other K row of B starts inside a sector
-constexpr double kSplitCost = 4.3, kSplitCostPerCta = 0.012;
-// with whole tiles to follow, beside which the exchange passes (but the partial tiles' traffic does not)
-constexpr double kSplitFirstCost = 3.0, kSplitFirstCostPerCta = 0.024;
+// What the tilings cost, in microseconds (kernel alone, back to back): a launch, each K tile of a round, and what splitting
+// K adds (partial tiles written, flagged, read, added; more where more of them cross).  Used only to pick one.  The
+// constants are fitted to 390 sizes x up to 17 variants measured on B200 (64 <= M <= 4096, N and K to 8192): estimates are
+// off by 6 %.  In 150 sizes left out of the fit the tiling they choose is 0.4 % from the fastest (mean; 8 % at worst).
+constexpr double kBasePair = 5.42, kBaseSingle256 = 4.05, kBaseSingle128 = 3.4, kBaseSingle64 = 3.13;
+constexpr double kOutput = 0.223e-6;  // per output element
+// with few SMs busy; the loads of a full GPU take kBusy more (pairs 0.30 to 0.36 us, 128 columns 0.30 to 0.34)
+constexpr double kPeriodPair = 0.291, kPeriodSingle256 = 0.378, kPeriodSingle128 = 0.276, kPeriodSingle64 = 0.255, kBusy = 0.2;
+constexpr double kRagged = 1.11;  // N no multiple of 32: every other K row of B starts inside a sector
+constexpr double kSplitCostPair = 3.16, kSplitCostPairPerCta = 0.0216;
+// single CTAs: the bytes that cross go with the tile's width, and each part adds a piece to wait for
+constexpr double kSplitCost = 1.75, kSplitCostPerCta256 = 0.0314, kSplitCostPerPart = 0.353;
+// pairs with whole tiles to follow, beside which the exchange passes (but the partial tiles' traffic does not)
+constexpr double kSplitFirstCost = 2.32, kSplitFirstCostPerCta = 0.019;
 
 struct GemmPlan {
     bool use_pair;
@@ -643,37 +648,39 @@ GemmPlan plan_gemm(const RankCtx& rc, uint32_t Mg, uint32_t N, uint32_t K, bool 
     const bool may_split = rc.splitk_ws != nullptr && g.split_k != 1 && !whole_tiles;
     const uint32_t cap = may_split ? (g.split_k >= 2 ? (uint32_t)g.split_k : kSplitKMax) : 1u;
     const bool forced_split = g.split_k >= 2;
-    const double ragged = N % 32u != 0u ? kRagged : 1.0, ragged64 = N % 32u != 0u ? kRagged64 : 1.0;
-    const double pair_period = kPeriodPair * ragged;
-    auto split_cost = [](uint32_t ctas) { return kSplitCost + kSplitCostPerCta * ctas; };
+    const double ragged = N % 32u != 0u ? kRagged : 1.0;
+    auto busy = [&](uint32_t ctas) { return ragged * (1.0 + kBusy * std::min(1.0, (double)ctas / sms)); };
 
     // CTA pairs: whole rounds, and a last round whose tiles are cut in as many parts as shorten it
     const uint32_t tiles = m256 * n256, rem = tiles % max_pairs;
     uint32_t pair_parts = 1;
-    double last = rem != 0 ? k_tiles * pair_period : 0.0;
+    double last = rem != 0 ? k_tiles * kPeriodPair * busy(2 * tiles) : 0.0;
     for (uint32_t s = 2; rem != 0 && s <= std::min(std::min(cap, max_pairs / rem), k_tiles); ++s) {
-        const double cost = tiles >= max_pairs ? kSplitFirstCost + kSplitFirstCostPerCta * 2 * rem * s : split_cost(2 * rem * s);
-        const double t = ((k_tiles + s - 1) / s) * pair_period + cost;
+        const uint32_t ctas = 2 * rem * s;
+        const double cost = tiles >= max_pairs ? kSplitFirstCost + kSplitFirstCostPerCta * ctas
+                                               : kSplitCostPair + kSplitCostPairPerCta * ctas;
+        const double t = ((k_tiles + s - 1) / s) * kPeriodPair * busy(tiles >= max_pairs ? sms : ctas) + cost;
         if (t < last) {
             last = t;
             pair_parts = s;
         }
     }
-    const double t_pair = kBasePair + (tiles / max_pairs) * k_tiles * pair_period + last;
+    const double t_pair = kBasePair + (tiles / max_pairs) * k_tiles * kPeriodPair * busy(sms) + last;
 
     // single CTAs: rounds of whole tiles, or, when the tiles leave at least half of the SMs idle, every (tile, K part) on
     // its own CTA (a power of two that divides the K tiles, at least four K tiles per part, one part per 32 columns)
     auto single = [&](uint32_t bn, uint32_t* parts) {
         const uint32_t t1 = m128 * ((N + bn - 1) / bn);
         const double base = bn == 256 ? kBaseSingle256 : (bn == 128 ? kBaseSingle128 : kBaseSingle64);
-        const double period = bn == 256 ? kPeriodSingle256 * ragged : (bn == 128 ? kPeriodSingle128 * ragged : kPeriodSingle64 * ragged64);
-        double best = base + (double)((t1 + sms - 1) / sms) * k_tiles * period;
+        const double period = bn == 256 ? kPeriodSingle256 : (bn == 128 ? kPeriodSingle128 : kPeriodSingle64);
+        double best = base + (double)((t1 + sms - 1) / sms) * k_tiles * period * busy(t1);
         *parts = 1;
         for (uint32_t s = 2; s <= std::min(std::min(cap, sms / t1), bn / 32u); s *= 2) {
             if (k_tiles % s != 0 || k_tiles / s < 4) {
                 continue;
             }
-            const double t = base + k_tiles / s * period + split_cost(t1 * s);
+            const double t = base + k_tiles / s * period * busy(t1 * s) + kSplitCost + kSplitCostPerCta256 * t1 * s * bn / 256 +
+                             kSplitCostPerPart * s;
             if (t < best || forced_split) {
                 best = t;
                 *parts = s;
@@ -702,7 +709,7 @@ GemmPlan plan_gemm(const RankCtx& rc, uint32_t Mg, uint32_t N, uint32_t K, bool 
     plan.use_pair = g.cta_pair == 1 || (g.cta_pair == 0 && g.block_n == 0 && t_pair < t_single);
     plan.block_n = plan.use_pair ? kPairBlockN : bn;
     plan.ksplit = plan.use_pair ? pair_parts : parts;
-    plan.time = plan.use_pair ? t_pair : t_single;
+    plan.time = (plan.use_pair ? t_pair : t_single) + kOutput * Mg * N;
     return plan;
 }
 
@@ -721,6 +728,7 @@ constexpr double kSmallBase = 2.9, kSmallPeriod16 = 0.23, kSmallPeriod32 = 0.24,
 constexpr double kSmallQuantShared = 1.45;  // two CTAs on an SM
 constexpr double kSmallBytesPerUs = 7.4e6, kSmallBytesPerUsRagged = 5.1e6, kSmallHidden = 0.73;
 constexpr double kSmallExchange16 = 0.6, kSmallExchange32 = 1.5, kSmallExchange32PerRow = 0.03;
+constexpr double kSmallShortK = 0.5;  // 32-row tiles, up to four K tiles: 64 sizes read 0.2 to 0.4 above the estimate, others 0.2 below
 constexpr double kSmallMxOutPerRow = 0.08;  // a warp takes the block maximum of one row at a time
 constexpr double kQuantiserSmall = 1.6, kQuantiserLarge = 1.8;
 
@@ -771,6 +779,7 @@ SmallPlan plan_small(const RankCtx& rc, uint32_t M, uint32_t N, uint32_t K, bool
             }
         }
     }
+    best += s.mt == 32 && k_tiles <= 4 ? kSmallShortK : 0.0;
     s.use = g.small_tile == 1 || best < plan_gemm(rc, M, N, K).time + (bf16_in ? kQuantiserLarge : 0.0);
     return s;
 }
