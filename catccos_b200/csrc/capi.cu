@@ -1093,10 +1093,15 @@ int copy_engine_join(RankCtx& rc, cudaStream_t st, uint32_t W)
     return 0;
 }
 
-// Alignment a fused call needs; a call that lacks it takes the general path, which refuses it with a message.
-bool fused_operands_ok(const void* a, const void* b, const void* b_scale, const void* c)
+// Alignment that the quantisers' and TMA's 16-byte accesses, the output's whole sectors and the 16-bit reads of the weight
+// scales need.  Checked at the entry: the quantiser, which runs first, checks nothing.
+bool matmul_operands_ok(const char* op, const void* a, const void* b, const void* b_scale, const void* c)
 {
-    return (((uintptr_t)a | (uintptr_t)b) & 15u) == 0u && ((uintptr_t)c & 31u) == 0u && ((uintptr_t)b_scale & 1u) == 0u;
+    if ((((uintptr_t)a | (uintptr_t)b) & 15u) || ((uintptr_t)c & 31u) || ((uintptr_t)b_scale & 1u)) {
+        ERROR_LOG("%s: a and b must be 16-byte aligned, c 32-byte aligned, b_scale 2-byte aligned", op);
+        return false;
+    }
+    return true;
 }
 
 // Common part of the two AllGather-Matmul entry points.
@@ -1106,11 +1111,18 @@ int allgather_matmul(void* stream, const void* a, const void* a_scale, bool preq
     if (!t || !a || !b || !b_scale || !c || (prequant && !a_scale)) {
         return CATCCOS_B200_EINVAL;
     }
+    const uint32_t M = t->m, K = t->k, N = t->n, W = t->rankSize;
+    if (M == 0 || K == 0 || N == 0 || K % kGemmBlockK != 0 || N % 16 != 0) {
+        ERROR_LOG("allgather matmul: M=%u K=%u N=%u unsupported (K a multiple of 128, N of 16)", M, K, N);
+        return CATCCOS_B200_EINVAL;
+    }
+    if (!matmul_operands_ok("allgather matmul", a, b, b_scale, c)) {
+        return CATCCOS_B200_EINVAL;
+    }
     int rcode = ensure_init();
     if (rcode != 0) return rcode;
-    const uint32_t M = t->m, K = t->k, N = t->n, W = t->rankSize;
-    if (W != (uint32_t)g.world || M == 0 || K % kGemmBlockK != 0 || N % 16 != 0) {
-        ERROR_LOG("allgather matmul: rankSize %u (world %d), M=%u K=%u N=%u unsupported", W, g.world, M, K, N);
+    if (W != (uint32_t)g.world) {
+        ERROR_LOG("allgather matmul: rankSize %u (world %d)", W, g.world);
         return CATCCOS_B200_EINVAL;
     }
     SymmAlloc* sa = find_symm(symm);
@@ -1225,15 +1237,15 @@ int allgather_matmul(void* stream, const void* a, const void* a_scale, bool preq
     // transfer like everybody's: the tiles then follow the send groups, slice by slice over all ranks.
     p.own_first = g.tile_order >= 0 ? (uint32_t)g.tile_order : ((fuse_mode == 6 || fuse_mode == 7) ? 0u : 1u);
     if (produce && consume && fuse_mode == 3) {
-        if (prequant && ((uintptr_t)a & 15u) == 0u && ((uintptr_t)a_scale & 3u) == 0u) {
-            // nothing to quantise and nobody to send to: the GEMM reads the caller's operands in place (operands that are
-            // aligned for neither TMA nor word loads go through the stage)
+        if (prequant && ((uintptr_t)a_scale & 3u) == 0u) {
+            // nothing to quantise and nobody to send to: the GEMM reads the caller's operands in place (scales that are not
+            // aligned for its word loads go through the stage)
             p.a_scales = (const uint8_t*)a_scale;
             p.flags = nullptr;
             return launch_gemm(rc, st, a, b, p);
         }
         const SmallPlan small = plan_small(rc, M, N, K, !prequant);
-        if (!prequant && small.use && small.quant && g.b_dtype != 2 && fused_operands_ok(a, b, b_scale, c)) {
+        if (!prequant && small.use && small.quant && g.b_dtype != 2) {
             SmallParams sp = {};
             sp.x = a;
             sp.w_scales = (const uint8_t*)b_scale;
@@ -1801,10 +1813,14 @@ int catccos_b200_fp4_mx_allgather_matmul(void* stream, const void* a, const void
     if (!t || !a || !b || !a_scale || !b_scale || !c) {
         return CATCCOS_B200_EINVAL;
     }
+    const uint32_t M = t->m, K = t->k, N = t->n, W = t->rankSize;
+    if (M == 0 || K == 0 || N == 0) {
+        ERROR_LOG("fp4 allgather matmul: M=%u K=%u N=%u unsupported", M, K, N);
+        return CATCCOS_B200_EINVAL;
+    }
     int rcode = ensure_init();
     if (rcode != 0) return rcode;
-    const uint32_t M = t->m, K = t->k, N = t->n, W = t->rankSize;
-    if (W != (uint32_t)g.world || M == 0 || K % kGemmBlockK != 0 || N % 16 != 0) {
+    if (W != (uint32_t)g.world || K % kGemmBlockK != 0 || N % 16 != 0) {
         ERROR_LOG("fp4 allgather matmul: rankSize %u (world %d), M=%u K=%u N=%u unsupported", W, g.world, M, K, N);
         return CATCCOS_B200_EINVAL;
     }
@@ -1953,10 +1969,18 @@ int catccos_b200_mxfp8_matmul_reduce_scatter(void* stream, const void* a, const 
     if (!t || !a || !b || !a_scale || !b_scale || !d) {
         return CATCCOS_B200_EINVAL;
     }
+    const uint32_t M = t->m, K = t->k, N = t->n, W = t->rankSize;  // m is the whole M: every rank holds all rows of its K slice
+    if (M == 0 || K == 0 || N == 0) {
+        ERROR_LOG("matmul reduce scatter: M=%u K=%u N=%u unsupported", M, K, N);
+        return CATCCOS_B200_EINVAL;
+    }
+    if ((uintptr_t)d & 7u) {
+        ERROR_LOG("matmul reduce scatter: d must be 8-byte aligned (32-byte with one rank)");
+        return CATCCOS_B200_EINVAL;  // the reducer stores four 16-bit results at a time
+    }
     int rcode = ensure_init();
     if (rcode != 0) return rcode;
-    const uint32_t M = t->m, K = t->k, N = t->n, W = t->rankSize;  // m is the whole M: every rank holds all rows of its K slice
-    if (W != (uint32_t)g.world || M == 0 || K % kGemmBlockK != 0 || N % 16 != 0 || M % W != 0 || (M / W) % 32 != 0) {
+    if (W != (uint32_t)g.world || K % kGemmBlockK != 0 || N % 16 != 0 || M % W != 0 || (M / W) % 32 != 0) {
         ERROR_LOG("matmul reduce scatter: rankSize %u (world %d), M=%u K=%u N=%u unsupported (M / rankSize must be a "
                   "multiple of 32, K of 128, N of 16)", W, g.world, M, K, N);
         return CATCCOS_B200_EINVAL;
@@ -2162,8 +2186,7 @@ extern "C" int catccos_b200_mx_quant_matmul_static(void* stream, const void* a_b
         ERROR_LOG("mx_quant_matmul_static: k must be a multiple of 128 and n of 16 (got n=%u k=%u)", n, k);
         return CATCCOS_B200_EINVAL;
     }
-    if ((((uintptr_t)a_bf16 | (uintptr_t)b) & 15u) || ((uintptr_t)c & 31u) || ((uintptr_t)b_scale & 1u)) {
-        ERROR_LOG("mx_quant_matmul_static: a and b must be 16-byte aligned, c 32-byte aligned, b_scale 2-byte aligned");
+    if (!matmul_operands_ok("mx_quant_matmul_static", a_bf16, b, b_scale, c)) {
         return CATCCOS_B200_EINVAL;  // refused before the shared array or the stream is touched
     }
     if ((size_t)m * k > kStaticMaxElems) {

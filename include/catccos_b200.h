@@ -78,7 +78,9 @@ int catccos_b200_mx_quant_allgather(void* stream, const void* in_bf16, void* out
  * (include/catccos/dgemm/kernel/mx_allgather_matmul.hpp:121-135,
  * include/catccos/dgemm/device/device_dgemm.hpp:77,116): A already quantised.
  * a E4M3 [m, k]; a_scale E8M0 [m, k/32]; b E4M3 [k, n]; b_scale E8M0 [k/64, n, 2];
- * c [rankSize*m, n] (bf16 by default, fp16 with option "c_dtype" = 1). */
+ * c [rankSize*m, n] (bf16 by default, fp16 with option "c_dtype" = 1).
+ * k % 128 == 0, n % 16 == 0; a and b 16-byte aligned, c 32-byte, b_scale 2-byte: anything else is CATCCOS_B200_EINVAL,
+ * before a launch. */
 int catccos_b200_fp8_mx_allgather_matmul(void* stream, const void* a, const void* b, const void* a_scale,
                                          const void* b_scale, void* c, void* symm,
                                          const catccos_b200_tiling_t* tiling, uint32_t magic);
@@ -107,7 +109,8 @@ int catccos_b200_mx_quant_allgather_matmul(void* stream, const void* a_bf16, con
  * [r * m / rankSize, (r + 1) * m / rankSize) as d [m / rankSize, n] (bf16, or fp16 with "c_dtype" = 1).
  * tiling->m is the WHOLE m, as in the reference's Arguments.  The GEMM's epilogue sends fp32 partial rows straight to
  * the stage of the rank that owns them; that rank adds them in rank order (the result does not depend on timing).
- * symm: catccos_b200_symm_bytes_needed(tiling, 2) bytes.  m / rankSize % 32 == 0, k % 128 == 0, n % 16 == 0. */
+ * symm: catccos_b200_symm_bytes_needed(tiling, 2) bytes.  m / rankSize % 32 == 0, k % 128 == 0, n % 16 == 0; d 8-byte
+ * aligned (32-byte with one rank). */
 int catccos_b200_mxfp8_matmul_reduce_scatter(void* stream, const void* a, const void* b, const void* a_scale,
                                              const void* b_scale, void* d, void* symm,
                                              const catccos_b200_tiling_t* tiling, uint32_t magic);

@@ -59,3 +59,26 @@ def test_misaligned_scale_pointers_are_refused_before_any_launch(capi):
     # the allocation-free entry point refuses bad pointers before it touches its shared array
     assert L.catccos_b200_mx_quant_matmul_static(None, 0x10008, 0x20000, 0x30000, 0x40000, 8, 16, 128) == -1
     assert st[0] == 0
+
+
+def test_matmul_entry_points_refuse_bad_operands_before_any_launch(capi):
+    # The quantiser and TMA read 16 bytes at a time and the tiling divides by the number of tiles: a misaligned operand or an
+    # empty axis has to come back as EINVAL.  Made-up addresses: nothing is initialised, let alone launched.
+    L = capi.load()
+    ok = dict(a=0x10000, a_scale=0x18000, b=0x20000, b_scale=0x30000, c=0x40000)
+
+    def calls(m=8, k=128, n=16, **bad):
+        p, t = {**ok, **bad}, capi.make_tiling(m, k, n, 1)
+        t = ctypes.byref(t)
+        yield L.catccos_b200_mx_quant_allgather_matmul(None, p["a"], p["b"], p["b_scale"], p["c"], None, t, 0)
+        yield L.catccos_b200_fp8_mx_allgather_matmul(None, p["a"], p["b"], p["a_scale"], p["b_scale"], p["c"], None, t, 0)
+        if not bad:
+            yield L.catccos_b200_fp4_mx_allgather_matmul(None, p["a"], p["b"], p["a_scale"], p["b_scale"], p["c"], None, t, 0)
+            yield L.catccos_b200_mxfp8_matmul_reduce_scatter(None, p["a"], p["b"], p["a_scale"], p["b_scale"], p["c"], None, t, 0)
+
+    for bad in (dict(a=0x10002), dict(a=0x10008), dict(b=0x20008), dict(b_scale=0x30001), dict(c=0x40010)):
+        assert list(calls(**bad)) == [-1, -1], bad
+    for empty in (dict(m=0), dict(k=0), dict(n=0)):
+        assert list(calls(**empty)) == [-1] * 4, empty
+    t = capi.make_tiling(32, 128, 16, 1)
+    assert L.catccos_b200_mxfp8_matmul_reduce_scatter(None, 0x10000, 0x20000, 0x18000, 0x30000, 0x40004, None, ctypes.byref(t), 0) == -1
