@@ -1104,6 +1104,11 @@ bool matmul_operands_ok(const char* op, const void* a, const void* b, const void
     return true;
 }
 
+bool share_memory(const void* p, size_t p_bytes, const void* q, size_t q_bytes)
+{
+    return (uintptr_t)p < (uintptr_t)q + q_bytes && (uintptr_t)q < (uintptr_t)p + p_bytes;
+}
+
 // Common part of the two AllGather-Matmul entry points.
 int allgather_matmul(void* stream, const void* a, const void* a_scale, bool prequant, const void* b,
                      const void* b_scale, void* c, void* symm, const catccos_b200_tiling_t* t)
@@ -1237,7 +1242,11 @@ int allgather_matmul(void* stream, const void* a, const void* a_scale, bool preq
     // transfer like everybody's: the tiles then follow the send groups, slice by slice over all ranks.
     p.own_first = g.tile_order >= 0 ? (uint32_t)g.tile_order : ((fuse_mode == 6 || fuse_mode == 7) ? 0u : 1u);
     if (produce && consume && fuse_mode == 3) {
-        if (prequant && ((uintptr_t)a_scale & 3u) == 0u) {
+        // C may lie in A's memory (a caller's buffer used twice): A is then quantised or copied into the stage first.  A kernel
+        // that still reads A where it is while others of its CTAs store C needs the two apart.
+        const bool apart = !share_memory(c, (size_t)M * N * 2, a, (size_t)M * K * (prequant ? 1 : 2)) &&
+                           !(prequant && share_memory(c, (size_t)M * N * 2, a_scale, (size_t)M * (K / 32)));
+        if (prequant && apart && ((uintptr_t)a_scale & 3u) == 0u) {
             // nothing to quantise and nobody to send to: the GEMM reads the caller's operands in place (scales that are not
             // aligned for its word loads go through the stage)
             p.a_scales = (const uint8_t*)a_scale;
@@ -1245,7 +1254,7 @@ int allgather_matmul(void* stream, const void* a, const void* a_scale, bool preq
             return launch_gemm(rc, st, a, b, p);
         }
         const SmallPlan small = plan_small(rc, M, N, K, !prequant);
-        if (!prequant && small.use && small.quant && g.b_dtype != 2) {
+        if (!prequant && apart && small.use && small.quant && g.b_dtype != 2) {
             SmallParams sp = {};
             sp.x = a;
             sp.w_scales = (const uint8_t*)b_scale;

@@ -80,7 +80,8 @@ int catccos_b200_mx_quant_allgather(void* stream, const void* in_bf16, void* out
  * a E4M3 [m, k]; a_scale E8M0 [m, k/32]; b E4M3 [k, n]; b_scale E8M0 [k/64, n, 2];
  * c [rankSize*m, n] (bf16 by default, fp16 with option "c_dtype" = 1).
  * k % 128 == 0, n % 16 == 0; a and b 16-byte aligned, c 32-byte, b_scale 2-byte: anything else is CATCCOS_B200_EINVAL,
- * before a launch. */
+ * before a launch.  With one rank c may share memory with a and a_scale (a is then copied to symm first), never with b or
+ * b_scale. */
 int catccos_b200_fp8_mx_allgather_matmul(void* stream, const void* a, const void* b, const void* a_scale,
                                          const void* b_scale, void* c, void* symm,
                                          const catccos_b200_tiling_t* tiling, uint32_t magic);
