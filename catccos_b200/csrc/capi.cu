@@ -109,13 +109,12 @@ struct RankCtx {
     int device = 0;
     int num_sms = 0;
     StatusBlock* status = nullptr;  // device memory
-    // split-K scratch of this rank's GEMM launches: one fp32 partial tile and four flag words per SM, and the
-    // count of split launches so far (the flags are epochs).  Launches of one rank are stream-ordered.
     uint8_t* fp4_bt = nullptr;  // the transposed copy of a packed E2M1 weight, made on every call that gets one
     size_t fp4_bt_bytes = 0;
+    // split-K scratch of this rank's GEMM launches: one fp32 partial tile and four flag words per SM, then the two words
+    // that count the split launches (the flags are epochs, split_epoch).  Launches of one rank are stream-ordered.
     float* splitk_ws = nullptr;
     uint32_t* splitk_flags = nullptr;
-    uint32_t splitk_epoch = 0;
     // copy-engine allgather: one stream per peer (the transfers to the peers run side by side), an event that
     // marks "this rank's shard is quantised" and one per stream that marks "everything for that peer has left"
     cudaStream_t side = nullptr;  // the quantise-and-push kernel runs here, beside the GEMM on the caller's stream
@@ -190,9 +189,8 @@ int setup_rank_ctx(RankCtx& rc, int device)
     CUDA_TRY(cudaMalloc(&rc.fp4_bt, 1u << 20));
     rc.fp4_bt_bytes = 1u << 20;
     CUDA_TRY(cudaMalloc(&rc.splitk_ws, (size_t)rc.num_sms * kSplitKTileBytes));
-    CUDA_TRY(cudaMalloc(&rc.splitk_flags, (size_t)rc.num_sms * 4 * sizeof(uint32_t)));
-    CUDA_TRY(cudaMemset(rc.splitk_flags, 0, (size_t)rc.num_sms * 4 * sizeof(uint32_t)));
-    rc.splitk_epoch = 0;
+    CUDA_TRY(cudaMalloc(&rc.splitk_flags, ((size_t)rc.num_sms * 4 + 2) * sizeof(uint32_t)));
+    CUDA_TRY(cudaMemset(rc.splitk_flags, 0, ((size_t)rc.num_sms * 4 + 2) * sizeof(uint32_t)));
     {
         int lo = 0, hi = 0;
         CUDA_TRY(cudaDeviceGetStreamPriorityRange(&lo, &hi));
@@ -942,7 +940,7 @@ int launch_gemm(RankCtx& rc, cudaStream_t st, const void* a, const void* b, Gemm
     if (ksplit > 1) {
         p.splitk_ws = rc.splitk_ws;
         p.splitk_flags = rc.splitk_flags;
-        p.splitk_epoch = ++rc.splitk_epoch;
+        p.splitk_state = rc.splitk_flags + (size_t)rc.num_sms * 4;
     }
     if (use_pair) {
         CUtensorMap pa, pb, pc;

@@ -107,7 +107,7 @@ struct GemmParams {
     uint32_t ksplit;
     float* splitk_ws;        // [tiles][ksplit][BLOCK_N / 32][128][32]
     uint32_t* splitk_flags;  // [tiles][ksplit][4] epoch words, one per epilogue warp
-    uint32_t splitk_epoch;
+    uint32_t* splitk_state;  // see split_epoch
 };
 
 template <uint32_t BLOCK_N>
@@ -474,8 +474,30 @@ constexpr uint32_t kSplitKMax = 8;
 constexpr uint32_t kSplitPieceBytes = 32u * 32u * 4u;           // 32 rows x 32 floats
 constexpr uint32_t kSplitRedBytes = 12u * kSplitPieceBytes;     // most pieces a warp takes in: two chunks from six parts
 
+// The epoch that a launch's flags carry, for one of `readers` warps (each of the launch calls this once, whatever becomes of
+// it later).  state[0] counts the split launches that have used this scratch, state[1] the warps of the present one that have
+// read it; the last one advances it for the next launch.  The count lives in device memory because a launch's parameters
+// stay the same when a CUDA graph replays it: with the epoch among them a second replay would take the first one's flags
+// for its own and add partial tiles that are not there yet.  Call it once the predecessor has finished (grid_dep_wait);
+// it is off the critical path, the accumulator takes longer.
+__device__ __forceinline__ uint32_t split_epoch(uint32_t* state, uint32_t readers, uint32_t lane)
+{
+    uint32_t epoch = 0;
+    if (lane == 0) {
+        epoch = ld_acquire_gpu(state) + 1u;
+        uint32_t before;
+        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(state + 1) : "memory");
+        if (before + 1u == readers) {
+            state[1] = 0u;
+            state[0] = epoch;
+        }
+    }
+    return __shfl_sync(0xFFFFFFFFu, epoch, 0);
+}
+
 template <typename OutT, uint32_t kChunks>
 struct SplitExchange {
+    uint32_t epoch;       // of this launch (split_epoch)
     float* ws;            // part 0's partial tile
     size_t part_stride;   // floats between the parts' partial tiles
     uint32_t* flags;      // this warp's flag word of part 0
@@ -518,7 +540,7 @@ struct SplitExchange {
         }
         __syncwarp();  // every lane's partial stores are ordered before lane 0's release
         if (lane == 0) {
-            st_release_gpu(flags + part * flag_stride, p.splitk_epoch);
+            st_release_gpu(flags + part * flag_stride, epoch);
         }
         // chunks right of the matrix were not written by anybody
         const uint32_t own_end = n0 >= p.N ? own0 : max(own0, min(own1, (p.N - n0 + 31u) / 32u));
@@ -528,8 +550,8 @@ struct SplitExchange {
         // lanes 0 .. parts-1 each watch one part's flag (the polls overlap instead of queueing up)
         bool ok = true;
         if (lane < parts && lane != part &&
-            !wait_flag_ge_gpu(flags + lane * flag_stride, p.splitk_epoch, p.timeout_ns, p.status)) {
-            report_status(p.status, kStatusFlagTimeout, 0x100u + lane, id, p.splitk_epoch);
+            !wait_flag_ge_gpu(flags + lane * flag_stride, epoch, p.timeout_ns, p.status)) {
+            report_status(p.status, kStatusFlagTimeout, 0x100u + lane, id, epoch);
             ok = false;
         }
         if (!__all_sync(0xFFFFFFFFu, ok)) {
@@ -610,12 +632,12 @@ struct SplitExchange {
         }
         __syncwarp();  // every lane's partial stores are ordered before lane 0's release
         if (lane == 0) {
-            st_release_gpu(flags + part * flag_stride, p.splitk_epoch);
+            st_release_gpu(flags + part * flag_stride, epoch);
         }
         bool ok = true;
         if (lane < parts && lane != part &&
-            !wait_flag_ge_gpu(flags + lane * flag_stride, p.splitk_epoch, p.timeout_ns, p.status)) {
-            report_status(p.status, kStatusFlagTimeout, 0x100u + lane, id, p.splitk_epoch);
+            !wait_flag_ge_gpu(flags + lane * flag_stride, epoch, p.timeout_ns, p.status)) {
+            report_status(p.status, kStatusFlagTimeout, 0x100u + lane, id, epoch);
             ok = false;
         }
         if (!__all_sync(0xFFFFFFFFu, ok)) {
@@ -1138,9 +1160,13 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             const uint32_t ks = blockIdx.x / num_tiles;
             const uint32_t tile = blockIdx.x - ks * num_tiles;
             TileCoord tc = tile_coord(tile, n_tiles, m_tiles, p);
+            SplitExchange<OutT, kChunks> x;
+            if (p.flags == nullptr) {
+                grid_dep_wait();  // a gated launch's quantiser has waited for the launch before it
+            }
+            x.epoch = split_epoch(p.splitk_state, num_units * 4u, lane);
             alive = mbar_wait_warp(&tmem_full[0], 0, p.status, 106, 0, bar_ns);
             tcgen05_fence_after();
-            SplitExchange<OutT, kChunks> x;
             x.part_stride = (size_t)kGemmBlockM * BLOCK_N;
             x.ws = p.splitk_ws + (size_t)tile * ksplit * x.part_stride;
             x.flags = p.splitk_flags + (size_t)tile * ksplit * 4u + q;

@@ -119,6 +119,9 @@ struct PairWork {
         split_at = units > rounds ? (ksplit > 1u && p.flags == nullptr ? 0u : rounds) : units;
     }
 
+    // pairs that have a split unit
+    __host__ __device__ __forceinline__ uint32_t split_units() const { return ksplit > 1u && units > 0u ? rem * ksplit : 0u; }
+
     __host__ __device__ __forceinline__ PairUnit unit(uint32_t i, const GemmParams& p) const
     {
         PairUnit u;
@@ -564,6 +567,13 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         constexpr uint32_t kChunks = kPairBlockN / 32;
         const uint32_t lane_base = tmem_base + ((q * 32u) << 16);
         uint8_t* stage_out = smem + S::kOffOut + q * kOutStageBytes;
+        uint32_t split_ep = 0;
+        if (work.split_units() > work.pair) {
+            if (p.flags == nullptr) {
+                grid_dep_wait();  // a gated launch's quantiser has waited for the launch before it
+            }
+            split_ep = split_epoch(p.splitk_state, work.split_units() * 8u, lane);
+        }
         for (uint32_t ui = 0; alive && ui < work.units; ++ui) {
             const PairUnit u = work.unit(ui, p);
             const uint32_t row0 = u.m0 + cta * 128u + q * 32u;  // this warp's first row
@@ -582,6 +592,7 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             tcgen05_fence_after();
             if (u.split) {
                 SplitExchange<OutT, kChunks> x;
+                x.epoch = split_ep;
                 const uint32_t slot = u.rem_ix * work.ksplit * 2u + cta;
                 x.ws = p.splitk_ws + (size_t)slot * (128u * kPairBlockN);
                 x.part_stride = (size_t)2u * 128u * kPairBlockN;
