@@ -369,7 +369,7 @@ void choose_segments(uint32_t M, uint32_t K, int num_sms, QuantPushParams& p, ui
 }
 
 // bf16 [M, K] -> codes and scales in one place, nobody waiting on flags: the flat quantiser.
-// `reset` (or nullptr): a wait record that starts anew with this call.
+// `reset` (or nullptr): the wait records of the allocation-free entry point, cleared for this call.
 int launch_quant_flat(cudaStream_t st, const void* in, uint32_t M, uint32_t K, uint8_t* codes, uint8_t* scales,
                       StatusBlock* reset = nullptr)
 {
@@ -814,7 +814,7 @@ int launch_small_inst(cudaStream_t st, const CUtensorMap& tw, const CUtensorMap&
     return 0;
 }
 
-// p: x or x_scales, w_scales, c, c_scales, M, N, K, w_early, w_kmajor, clear filled in.
+// p: x or x_scales, w_scales, c, c_scales, M, N, K, w_early, w_kmajor, records filled in.
 int launch_small(RankCtx& rc, cudaStream_t st, const SmallPlan& plan, const void* x_codes, const void* w, SmallParams p,
                  bool mx_out)
 {
@@ -2176,7 +2176,7 @@ static __device__ __align__(256) uint8_t g_static_scratch[kStaticBytes];
 struct StaticDeviceState {
     uint8_t* ptr = nullptr;  // device address of g_static_scratch on this device
     int num_sms = 0;
-    uint32_t record = 0;  // which of the two wait records the last call uses; the other one is clear
+    WaitRecordTurn turn;
 };
 StaticDeviceState g_static_dev[kMaxRanks * 2];
 std::mutex g_static_mu;
@@ -2226,7 +2226,10 @@ extern "C" int catccos_b200_mx_quant_matmul_static(void* stream, const void* a_b
     rc.device = dev;
     rc.num_sms = sd.num_sms;
     StatusBlock* records = reinterpret_cast<StatusBlock*>(sd.ptr + kStaticStatusOff);
-    rc.status = records + sd.record;
+    cudaStream_t st = (cudaStream_t)stream;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CUDA_TRY(cudaStreamIsCapturing(st, &capture));
+    const bool captured = capture != cudaStreamCaptureStatusNone;
 
     QuantPushParams seg = {};
     choose_segments(m, k, rc.num_sms, seg);
@@ -2241,7 +2244,11 @@ extern "C" int catccos_b200_mx_quant_matmul_static(void* stream, const void* a_b
     }
     const SmallPlan small = plan_small(rc, m, n, k, true);
     if (small.use && small.quant) {
-        // one launch; it takes the clear record, and clears the last call's once that call has finished
+        // one launch (wait_records.hpp: how it comes by a clear record)
+        rc.status = records + sd.turn.one_launch(captured);
+        if (captured) {
+            CUDA_TRY(cudaMemsetAsync(rc.status, 0, sizeof(StatusBlock), st));
+        }
         SmallParams sp = {};
         sp.x = a_bf16;
         sp.w_scales = (const uint8_t*)b_scale;
@@ -2249,18 +2256,16 @@ extern "C" int catccos_b200_mx_quant_matmul_static(void* stream, const void* a_b
         sp.M = m;
         sp.N = n;
         sp.K = k;
-        sp.clear = records + sd.record;
-        sd.record ^= 1u;
-        rc.status = records + sd.record;
-        return launch_small(rc, (cudaStream_t)stream, small, nullptr, b, sp, false);
+        sp.records = records;
+        return launch_small(rc, st, small, nullptr, b, sp, false);
     }
     // Two launches on the caller's stream, as catccos_b200_mx_quant_allgather_matmul at one rank: the quantiser on every
     // SM, then the GEMM (K in one piece: the array has no room for partial tiles).  One kernel that does both measured
     // 36 us on 509 x 2320 x 3968.
-    cudaStream_t st = (cudaStream_t)stream;
+    rc.status = records + sd.turn.two_launches(captured);
     uint8_t* codes = sd.ptr + kStaticCodesOff;
     uint8_t* scales = sd.ptr + kStaticScalesOff;
-    int rcode = launch_quant_flat(st, a_bf16, m, k, codes, scales, rc.status);
+    int rcode = launch_quant_flat(st, a_bf16, m, k, codes, scales, records);
     if (rcode != 0) return rcode;
     GemmParams p = {};
     p.a_scales = scales;
@@ -2333,8 +2338,14 @@ extern "C" int catccos_b200_mx_quant_matmul_static_status(uint32_t out[4])
         return CATCCOS_B200_ESTATE;  // no call has been made on this device yet
     }
     CUDA_TRY(cudaDeviceSynchronize());
-    StatusBlock sb;
-    CUDA_TRY(cudaMemcpy(&sb, sd.ptr + kStaticStatusOff + sd.record * sizeof(sb), sizeof(sb), cudaMemcpyDeviceToHost));
+    StatusBlock records[kWaitRecords];
+    CUDA_TRY(cudaMemcpy(records, sd.ptr + kStaticStatusOff, sizeof(records), cudaMemcpyDeviceToHost));
+    StatusBlock sb = records[0];
+    for (const StatusBlock& r : records) {
+        if (sb.code == 0) {
+            sb = r;  // a call clears the records it does not use: at most one is set
+        }
+    }
     out[0] = sb.code;
     out[1] = sb.rank;
     out[2] = sb.chunk;

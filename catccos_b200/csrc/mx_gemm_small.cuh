@@ -42,7 +42,7 @@ struct SmallParams {
     uint32_t device_tiny;     // QUANT, MxOut: tiny blocks follow the reference device kernel
     uint64_t bar_timeout_ns;
     StatusBlock* status;
-    StatusBlock* clear;       // another wait record, no longer in use, to be cleared (or nullptr)
+    StatusBlock* records;     // kWaitRecords wait records of which all but `status` are to be cleared (or nullptr)
 };
 
 template <uint32_t MT>
@@ -214,8 +214,8 @@ mx_gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             }
         }
         grid_dep_wait();
-        if (lane == 0 && p.clear != nullptr && blockIdx.x == 0) {
-            *p.clear = StatusBlock{};
+        if (p.records != nullptr && blockIdx.x == 0 && lane < kWaitRecords && p.records + lane != p.status) {
+            p.records[lane] = StatusBlock{};  // what the call before left: it has finished
         }
         __syncwarp();
         // the warp stays together and one elected lane issues (mx_gemm.cuh)

@@ -17,6 +17,7 @@
 #include <cuda_fp4.h>
 
 #include "common.cuh"
+#include "wait_records.hpp"
 #include "trace.cuh"
 
 namespace catccos {
@@ -339,8 +340,8 @@ __global__ void __launch_bounds__(kQuantThreads) mx_quant_flat_kernel(const uint
                                                                       uint32_t device_tiny, StatusBlock* reset)
 {
     grid_dep_wait();
-    if (reset != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
-        *reset = StatusBlock{};
+    if (reset != nullptr && blockIdx.x == 0 && threadIdx.x < kWaitRecords) {
+        reset[threadIdx.x] = StatusBlock{};
         __threadfence();  // before the GEMM behind this kernel may look at it
     }
     grid_dep_launch();

@@ -171,7 +171,7 @@ int catccos_b200_mx_quant_scatter_packed(void* stream, const void* in_bf16, cons
  * call's contents: calls are correct back to back on one stream, but two calls whose kernels overlap
  * on the GPU (different streams, no dependency) race on it.  The kernels that the first call of a new shape
  * class (tile width, output type) launches are configured on that first launch as well, so make one call per
- * shape class before capture.  Device-side wait records of this path are kept in the same array and read with
+ * shape class before capture.  A captured call may be replayed any number of times, with direct calls in between.  Device-side wait records of this path are kept in the same array and read with
  * catccos_b200_mx_quant_matmul_static_status, not with catccos_b200_last_status. */
 int catccos_b200_mx_quant_matmul_static(void* stream, const void* a_bf16, const void* b, const void* b_scale, void* c,
                                         uint32_t m, uint32_t n, uint32_t k);

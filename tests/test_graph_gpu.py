@@ -68,3 +68,37 @@ def test_replays(capi, cuda, oracle, m, n, k, options):
         for key in OPTIONS:
             capi.set_option(key, 0)
         capi.symm_free(symm)
+
+
+@pytest.mark.parametrize("small_tile", [1, 2])  # one launch, two launches
+def test_replays_of_the_allocation_free_call(capi, cuda, small_tile):
+    torch = cuda
+    m, n, k = 48, 272, 1024
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    xs = [torch.randn((m, k), generator=gen, device="cuda").to(torch.bfloat16) for _ in range(3)]
+    codes, scales = capi.mx_quant((torch.randn((n, k), generator=gen, device="cuda") * 0.02).to(torch.bfloat16))
+    b, b_scales = codes.t().contiguous(), scales.view(n, k // 64, 2).permute(1, 0, 2).contiguous()
+    capi.set_option("small_tile", small_tile)
+    capi.set_option("small_quant", small_tile)
+    try:
+        want = []
+        for x in xs:
+            want.append(torch.empty((m, n), dtype=torch.bfloat16, device="cuda"))
+            capi.mx_quant_matmul_static(x, b, b_scales, want[-1])
+        x, c = xs[0].clone(), torch.empty_like(want[0])
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            capi.mx_quant_matmul_static(x, b, b_scales, c)
+            capi.mx_quant_matmul_static(x, b, b_scales, c)
+        for i in (0, 1, 2, 1):
+            x.copy_(xs[i])
+            c.fill_(float("nan"))
+            graph.replay()
+            other = torch.empty_like(c)
+            capi.mx_quant_matmul_static(xs[0], b, b_scales, other)
+            assert torch.equal(c, want[i]) and torch.equal(other, want[0])
+            assert capi.static_status()[0] == 0
+    finally:
+        capi.set_option("small_tile", 0)
+        capi.set_option("small_quant", 0)
