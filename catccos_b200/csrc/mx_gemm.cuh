@@ -248,7 +248,9 @@ __device__ __forceinline__ uint32_t wait_rows_ready(const GemmParams& p, uint32_
         ready = min(ready, cnt);
     }
     ready = __reduce_min_sync(0xFFFFFFFFu, ready);
-    return __all_sync(0xFFFFFFFFu, ok) ? ready : 0u;
+    ok = __all_sync(0xFFFFFFFFu, ok);
+    __syncwarp();  // each chunk's flag was acquired by one lane; a vote orders no memory
+    return ok ? ready : 0u;
 }
 
 __device__ __forceinline__ void st_release_cta_shared(uint32_t* p, uint32_t v)
@@ -557,6 +559,7 @@ struct SplitExchange {
         if (!__all_sync(0xFFFFFFFFu, ok)) {
             return false;
         }
+        __syncwarp();  // each part's flag was acquired by one lane; a vote orders no memory
         if (lane == 0) {
             mbar_arrive_expect_tx(bar, (parts - 1u) * (own_end - own0) * kSplitPieceBytes);
             fence_proxy_async_all();  // the other parts' generic-proxy stores before this thread's bulk copies
@@ -643,6 +646,7 @@ struct SplitExchange {
         if (!__all_sync(0xFFFFFFFFu, ok)) {
             return false;
         }
+        __syncwarp();  // each part's flag was acquired by one lane; a vote orders no memory
         const uint32_t own0 = (part * kChunks + parts - 1u) / parts, own1 = ((part + 1u) * kChunks + parts - 1u) / parts;
         for (uint32_t chunk = own0; chunk < own1 && n0 + chunk * 32u < p.N; ++chunk) {
             uint32_t r[32];
@@ -1059,6 +1063,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 // one lane reads the word for the warp: the producer may be updating it, and the branch below holds
                 // warp-wide operations, so every lane has to take the same side
                 const uint32_t g = __shfl_sync(0xFFFFFFFFu, ld_acquire_cta_shared(gate), 0);
+                __syncwarp();  // lane 0 acquired it
                 if (g > it) {
                     known_end = g;
                 } else {

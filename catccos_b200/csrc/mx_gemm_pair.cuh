@@ -446,6 +446,7 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 // one lane reads the word for the warp: the producer may be updating it, and the branch below holds
                 // warp-wide operations, so every lane has to take the same side
                 const uint32_t g = __shfl_sync(0xFFFFFFFFu, ld_acquire_cta_shared(gate), 0);
+                __syncwarp();  // lane 0 acquired it
                 if (g >= c.it + (last - c.kt)) {
                     known_end = g;
                 } else {

@@ -418,6 +418,7 @@ __device__ __forceinline__ void push_worker(const PushParams& p, uint32_t lane, 
             if (!__all_sync(0xFFFFFFFFu, ok)) {
                 return;  // the quantise warps of this launch will not deliver: nothing sensible left to push
             }
+            __syncwarp();  // lane 0 acquired the flag; a vote orders no memory
             if (lane == 0) {
                 CATCCOS_TR_ADD(p.trace, kTrPushFlagWaitNs + pw, CATCCOS_TR_NOW() - t0);
             }
