@@ -6,6 +6,7 @@
 //
 // The C ABI's functions are not linked but bound by address (bind()), so that they are those of the library that capi.py
 // has loaded.  Every function returns the C ABI's code (alone, or first in a tuple with the outputs).
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <ATen/ATen.h>
@@ -120,14 +121,21 @@ catccos_b200_tiling_t tiling(uint32_t m, uint32_t k, uint32_t n, uint32_t world)
     return t;
 }
 
-// Launches may wait for room in the stream's queue: other Python threads run meanwhile.
+// Launches may wait for room in the stream's queue: other Python threads run meanwhile.  The lock is back before an
+// exception leaves.
+struct Unlocked {
+    PyThreadState* state = PyEval_SaveThread();
+    ~Unlocked() { PyEval_RestoreThread(state); }
+};
+
 template <typename F>
 PyObject* released(F&& call)
 {
     int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = call();
-    Py_END_ALLOW_THREADS
+    {
+        Unlocked unlocked;
+        rc = call();
+    }
     return PyLong_FromLong(rc);
 }
 
@@ -155,8 +163,8 @@ PyObject* guarded(const char* name, Py_ssize_t want, Py_ssize_t n, bool bound, F
         return body();
     } catch (const Error&) {
         return nullptr;
-    } catch (const std::exception& e) {
-        PyErr_SetString(PyExc_RuntimeError, e.what());
+    } catch (...) {
+        torch::translate_exception_to_python(std::current_exception());  // torch.OutOfMemoryError and the like
         return nullptr;
     }
 }
