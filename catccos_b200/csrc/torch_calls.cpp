@@ -72,12 +72,27 @@ uint32_t product_columns(PyObject* b_scales)
 
 void* pointer(PyObject* tensor_object) { return tensor(tensor_object).data_ptr(); }
 
-void* address(PyObject* number)
+// An address as ctypes takes one: a number, None, or a pointer object with a `value` (ctypes.c_void_p).
+void* address(PyObject* o)
 {
-    if (number == Py_None) {
+    if (o == Py_None) {
         return nullptr;
     }
-    void* p = PyLong_AsVoidPtr(number);
+    if (PyLong_Check(o)) {
+        void* p = PyLong_AsVoidPtr(o);
+        if (p == nullptr && PyErr_Occurred()) {
+            throw Error{};
+        }
+        return p;
+    }
+    PyObject* value = PyObject_GetAttrString(o, "value");
+    if (value == nullptr || !(value == Py_None || PyLong_Check(value))) {
+        Py_XDECREF(value);
+        PyErr_Format(PyExc_TypeError, "expected an address, got %s", Py_TYPE(o)->tp_name);
+        throw Error{};
+    }
+    void* p = value == Py_None ? nullptr : PyLong_AsVoidPtr(value);
+    Py_DECREF(value);
     if (p == nullptr && PyErr_Occurred()) {
         throw Error{};
     }
