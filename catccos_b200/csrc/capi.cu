@@ -742,6 +742,11 @@ SmallPlan plan_small(const RankCtx& rc, uint32_t M, uint32_t N, uint32_t K, bool
     if (g.small_tile == 2 || g.cta_pair != 0 || g.block_n != 0) {
         return s;  // another tiling is asked for
     }
+#ifdef CATCCOS_TRACE
+    if (g.trace_armed && rc.trace != nullptr) {
+        return s;  // this kernel keeps no timeline: the call is recorded on the general ones
+    }
+#endif
     s.mt = M <= 16 ? 16 : 32;
     const uint32_t tiles = ((M + s.mt - 1) / s.mt) * ((N + kSmallBlockN - 1) / kSmallBlockN), k_tiles = K / kGemmBlockK;
     const uint32_t cap = std::min(g.split_k >= 1 ? (uint32_t)g.split_k : kSmallMaxParts, k_tiles);
@@ -883,12 +888,6 @@ int launch_gemm(RankCtx& rc, cudaStream_t st, const void* a, const void* b, Gemm
     p.timeout_ns = g.timeout_ns;
     // a barrier inside the kernel may have to wait for as long as the flag wait it depends on
     p.bar_timeout_ns = 2 * g.timeout_ns + 1000000000ull;
-#ifdef CATCCOS_TRACE
-    if (g.trace_armed && rc.trace != nullptr) {
-        g.trace_armed = false;
-        p.trace = p.q.trace = p.push.trace = rc.trace;
-    }
-#endif
     p.a_fmt = g.a_dtype == 2 ? 5u : (g.a_dtype == 1 ? 1u : 0u);
     p.b_fmt = g.b_dtype == 2 ? 5u : (g.b_dtype == 1 ? 1u : 0u);
     const bool a_fp4 = g.a_dtype == 2, b_fp4 = g.b_dtype == 2;
@@ -932,6 +931,12 @@ int launch_gemm(RankCtx& rc, cudaStream_t st, const void* a, const void* b, Gemm
             return launch_small(rc, st, small, a, b, sp, mx_out);
         }
     }
+#ifdef CATCCOS_TRACE
+    if (g.trace_armed && rc.trace != nullptr) {
+        g.trace_armed = false;
+        p.trace = p.q.trace = p.push.trace = rc.trace;
+    }
+#endif
     const GemmPlan plan = plan_gemm(rc, p.Mg, p.N, p.K, scatter, scatter || fused_quant || p.flags != nullptr);  // scatter: the owner adds whole tiles, K stays in one piece
     const bool use_pair = plan.use_pair;
     const uint32_t bn = plan.block_n, ksplit = plan.ksplit;

@@ -8,6 +8,7 @@ Every rank warms the step up, arms the timeline for one launch (L2 flushed, rank
 all-reduce, as in bench.py), reads the per-CTA stamps back and reduces them; rank 0 prints one table per rank.
 Times are microseconds since the first CTA of that rank started (each GPU has its own %globaltimer; ranks are
 not compared with each other).  "min / med / max" run over the CTAs (or pushers) that wrote the slot.
+The small-tile kernel keeps no timeline: on one GPU a step that would take it is recorded on the general kernels instead.
 """
 from __future__ import annotations
 
