@@ -572,21 +572,6 @@ int resident_pairs(uint32_t max_pairs, uint32_t* pairs)
     return 0;
 }
 
-// Whole rounds of tiles, then the rest cut along K (mx_gemm_pair.cuh).  `parts` <= 1: the rest stays whole.
-struct PairGrid {
-    uint32_t pairs, ksplit;
-};
-
-PairGrid pair_grid(uint32_t tiles, uint32_t pairs, uint32_t parts)
-{
-    const uint32_t rem = tiles % pairs;
-    if (rem == 0 || parts <= 1) {
-        return {std::min(tiles, pairs), 1};
-    }
-    parts = std::min(parts, pairs / rem);
-    return {tiles < pairs ? rem * parts : pairs, parts};
-}
-
 template <typename OutT, bool FUSED>
 int launch_gemm_pair_inst(uint32_t max_pairs, uint32_t tiles, uint32_t parts, cudaStream_t st, const CUtensorMap& ta,
                           const CUtensorMap& tb, const CUtensorMap& tc, GemmParams& p, bool overlap_predecessor)

@@ -89,6 +89,22 @@ __host__ __device__ __forceinline__ TileCoord pair_tile_coord(uint32_t idx, uint
     return t;
 }
 
+// The launch of `tiles` tiles on at most `pairs` resident pairs: whole rounds, then the rest cut along K in at most `parts` parts
+// each (<= 1: it stays whole).
+struct PairGrid {
+    uint32_t pairs, ksplit;
+};
+
+inline PairGrid pair_grid(uint32_t tiles, uint32_t pairs, uint32_t parts)
+{
+    const uint32_t rem = tiles % pairs;
+    if (rem == 0 || parts <= 1) {
+        return {tiles < pairs ? tiles : pairs, 1};
+    }
+    parts = parts < pairs / rem ? parts : pairs / rem;
+    return {tiles < pairs ? rem * parts : pairs, parts};
+}
+
 // One work unit of a pair: a whole tile, or one K part of a tile of the last round.
 struct PairUnit {
     uint32_t m0, n0, n_tile;  // first row and column of the pair's tile

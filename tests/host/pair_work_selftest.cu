@@ -19,18 +19,19 @@ static int check(uint32_t m, uint32_t n, uint32_t k, uint32_t max_pairs, uint32_
     p.Mg = m;
     p.N = n;
     p.K = k;
-    const uint32_t tiles = ((m + 255) / 256) * ((n + 255) / 256), rem = tiles % max_pairs;
-    uint32_t pairs = tiles < max_pairs ? tiles : max_pairs;
-    p.ksplit = 1;
-    if (rem != 0 && parts > 1) {
-        p.ksplit = parts < max_pairs / rem ? parts : max_pairs / rem;
-        pairs = tiles < max_pairs ? rem * p.ksplit : max_pairs;
-    }
-    if (p.ksplit > k / 128) return 0;
+    const uint32_t tiles = ((m + 255) / 256) * ((n + 255) / 256);
+    const PairGrid grid = pair_grid(tiles, max_pairs, parts);
+    const uint32_t pairs = grid.pairs;
+    p.ksplit = grid.ksplit;
+    if (p.ksplit > k / 128) return 0;  // no part without a K tile is asked for
+    if (pairs == 0 || pairs > max_pairs || p.ksplit < 1 || p.ksplit > (parts > 1 ? parts : 1)) return 6;
     std::vector<std::vector<int>> seen(tiles, std::vector<int>(k / 128, 0));
     std::vector<int> slots(max_pairs, 0);
+    uint32_t readers = 0, split_units = 0;
     for (uint32_t pair = 0; pair < pairs; ++pair) {
         const PairWork w(p, pair, pairs);
+        readers += pair < w.split_units() ? 1 : 0;
+        split_units = w.split_units();
         for (uint32_t i = 0; i < w.units; ++i) {
             const PairUnit u = w.unit(i, p);
             const uint32_t tile = u.m0 / 256 * w.n_tiles + u.n_tile;
@@ -45,6 +46,8 @@ static int check(uint32_t m, uint32_t n, uint32_t k, uint32_t max_pairs, uint32_
         }
     }
     for (auto& t : seen) for (int c : t) if (c != 1) return 4;
+    if (readers != split_units) return 7;  // the pairs that read the launch's epoch are as many as it is counted for
+    for (uint32_t i = 0; i < max_pairs; ++i) if ((i < split_units) != (slots[i] == 1)) return 8;
     return 0;
 }
 
