@@ -83,10 +83,15 @@ def test_types(small, cuda, oracle, m):
     small.set_option("a_dtype", 1)
     small.set_option("c_dtype", 1)
     codes, scales = small.mx_quant(x_d)
+    small.set_option("split_k", 2)  # the same order of summation whoever quantises
     want = small.mx_gemm(codes, scales, b_d, bs_d, out_dtype=torch.float16)
-    got = torch.empty_like(want)
-    small.mx_quant_matmul_static(x_d, b_d, bs_d, got)
-    assert torch.equal(got, want)
+    for quant in (1, 2):
+        small.set_option("small_quant", quant)
+        got = torch.empty_like(want)
+        small.mx_quant_matmul_static(x_d, b_d, bs_d, got)
+        assert torch.equal(got, want), quant
+    small.set_option("small_quant", 0)
+    small.set_option("split_k", 0)
     small.set_option("small_tile", 2)
     other = small.mx_gemm(codes, scales, b_d, bs_d, out_dtype=torch.float16)
     # two fp32 summation orders, each rounded once to 11 bits: one unit in the last place of the larger
@@ -107,7 +112,35 @@ def test_types(small, cuda, oracle, m):
     assert torch.all((out[0].float() - out[1].float()).abs() <= 2.0 ** -7 * out[1].float().abs().clamp_min(1.0))
 
 
-def test_nonfinite_and_tiny_blocks(small, cuda, oracle, golden):
+@pytest.mark.parametrize("split_k", [1, 4])
+@pytest.mark.parametrize("m", [12, 40])
+def test_nonfinite_blocks(small, cuda, oracle, m, split_k):
+    # an infinity or a NaN makes its block NaN (code 0x7F, scale 0xFF), and with it exactly its row of the product
+    torch = cuda
+    n, k = 160, 2048
+    x, (bc, bsc) = _problem(oracle, m, n, k)
+    bad = {3: (5, 0x7F80), 6: (1024, 0xFF80), 11: (2047, 0x7FC0)}  # row: column, +inf, -inf, NaN
+    rows = np.array([r for r in range(m) if r not in bad])
+    ac, asc = oracle.quantize_rows(np.ascontiguousarray(x[rows]))
+    gold = oracle.allgather_matmul([ac], [asc], bc, bsc)
+    for r, (col, bits) in bad.items():
+        x[r, col] = bits
+    x_d, b_d, bs_d = to_dev_bf16(torch, x), torch.from_numpy(bc).cuda(), torch.from_numpy(bsc).cuda()
+    keep, gone = torch.from_numpy(rows).cuda(), torch.tensor(sorted(bad), device="cuda")
+    small.set_option("split_k", split_k)
+    for quant in (1, 2):
+        small.set_option("small_quant", quant)
+        c = torch.zeros((m, n), dtype=torch.bfloat16, device="cuda")
+        small.mx_quant_matmul_static(x_d, b_d, bs_d, c)
+        assert bool(c[gone].isnan().all())
+        _check(oracle, c[keep], gold)
+    codes, scales = small.mx_gemm_quant_out(*small.mx_quant(x_d), b_d, bs_d)
+    assert bool((codes[gone] == 0x7F).all()) and bool((scales[gone] == 0xFF).all())
+    want = oracle.quantize_rows(c.view(torch.int16).cpu().numpy().view(np.uint16)[rows])
+    assert np.array_equal(codes[keep].cpu().numpy(), want[0]) and np.array_equal(scales[keep].cpu().numpy(), want[1])
+
+
+def test_tiny_blocks(small, cuda, oracle, golden):
     # the edge fixture's zeros, subnormals, ties and tiny blocks through the quantisation inside the kernel, both rules
     torch = cuda
     x = np.ascontiguousarray(golden("quant_edges")["x"].reshape(-1)[: 128 * 24].reshape(24, 128))
