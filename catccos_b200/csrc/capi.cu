@@ -1659,7 +1659,7 @@ int catccos_b200_mx_quant(void* stream, const void* in_bf16, uint32_t rows, uint
         return CATCCOS_B200_EINVAL;
     }
     if (k % 128 == 0 && ((uintptr_t)scales & 3u)) {
-        return CATCCOS_B200_EINVAL;  // four scale bytes go out as one 32-bit store when a row holds a multiple of four
+        return CATCCOS_B200_EINVAL;  // a row of whole words: the GEMMs, which take such rows, read the scales as 32-bit words
     }
     int rcode = ensure_init();
     if (rcode != 0) return rcode;
@@ -1702,7 +1702,7 @@ int catccos_b200_mx_quant_allgather(void* stream, const void* in_bf16, void* out
         return CATCCOS_B200_EINVAL;
     }
     if (K % 128 == 0 && ((uintptr_t)out_scales & 3u)) {
-        return CATCCOS_B200_EINVAL;  // scales are stored and copied as 32-bit words when a row holds a multiple of four
+        return CATCCOS_B200_EINVAL;  // several ranks copy such rows as 32-bit words, and the GEMMs read them so
     }
     RankCtx& rc = cur();
     CUDA_TRY(cudaSetDevice(rc.device));
@@ -2154,7 +2154,6 @@ namespace {
 // this file-scope device array instead of a buffer from catccos_b200_symm_alloc.  Every GPU that
 // loads the library carries it (about 8.3 MiB) until the process exits.
 constexpr size_t kStaticMaxElems = size_t(8) << 20;  // m * k may not exceed this
-constexpr uint32_t kStaticMaxItems = 8192;           // (16-row chunks) x (K segments) may not exceed this
 constexpr size_t kStaticStatusOff = 0;
 constexpr size_t kStaticScalesOff = kStaticStatusOff + 1024;
 constexpr size_t kStaticCodesOff = kStaticScalesOff + kStaticMaxElems / 32;
@@ -2221,14 +2220,6 @@ extern "C" int catccos_b200_mx_quant_matmul_static(void* stream, const void* a_b
     CUDA_TRY(cudaStreamIsCapturing(st, &capture));
     const bool captured = capture != cudaStreamCaptureStatusNone;
 
-    QuantPushParams seg = {};
-    choose_segments(m, k, rc.num_sms, seg);
-    const uint32_t chunks = (m + kRowsPerChunk - 1) / kRowsPerChunk;
-    if ((size_t)chunks * seg.segs_per_chunk > kStaticMaxItems) {
-        ERROR_LOG("mx_quant_matmul_static: %u row chunks x %u K segments exceed the limit of %u", chunks, seg.segs_per_chunk,
-                  kStaticMaxItems);
-        return CATCCOS_B200_ENOMEM;
-    }
     if (g.b_dtype == 2) {
         return CATCCOS_B200_ESTATE;  // packed weights need a transposed copy, and this path has no scratch for it
     }

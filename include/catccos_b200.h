@@ -164,8 +164,7 @@ int catccos_b200_mx_quant_scatter_packed(void* stream, const void* in_bf16, cons
  * loops where an allocation would serialise the device.  The call itself makes no cudaMalloc, cudaFree
  * or other allocating call; inputs and the output are the caller's.
  *
- * Limits: m * k <= 8 Mi elements (8 388 608) and at most 8192 (16-row chunk, K segment) pairs, else
- * CATCCOS_B200_ENOMEM with an [ERROR] line; k % 128 == 0, n % 16 == 0.  The first call on each device
+ * Limits: m * k <= 8 Mi elements (8 388 608), else CATCCOS_B200_ENOMEM with an [ERROR] line; k % 128 == 0, n % 16 == 0.  The first call on each device
  * looks up the array's device address (that device must be current) and should therefore be made
  * before any stream capture begins.  All calls on a device share the one array, which keeps the last
  * call's contents: calls are correct back to back on one stream, but two calls whose kernels overlap

@@ -47,8 +47,8 @@ def test_set_option_rejects_unknown(capi):
 
 
 def test_misaligned_scale_pointers_are_refused_before_any_launch(capi):
-    # With k % 128 == 0 a row's scale bytes are written four at a time: a scales pointer carved from a byte
-    # pool at an odd offset must come back as EINVAL, not as a misaligned-address fault on the device.
+    # With k % 128 == 0 a row of scales is whole words, which the GEMMs (and the copies between ranks) read as such: a
+    # scales pointer carved from a byte pool at an odd offset must come back as EINVAL, where it is made.
     # The checks run before the library touches CUDA, so made-up addresses do.
     L = capi.load()
     assert L.catccos_b200_mx_quant(None, 0x10000, 8, 128, 0x20000, 0x30001) == -1
