@@ -602,6 +602,7 @@ int launch_gemm_pair_inst(uint32_t max_pairs, uint32_t tiles, uint32_t parts, cu
 // K adds (partial tiles written, flagged, read, added; more where more of them cross).  Used only to pick one.  The
 // constants are fitted to 390 sizes x up to 17 variants measured on B200 (64 <= M <= 4096, N and K to 8192): estimates are
 // off by 6 %.  In 150 sizes left out of the fit the tiling they choose is 0.4 % from the fastest (mean; 8 % at worst).
+// Larger M (to 32768) is not in the fit: such launches are many rounds of pairs whatever the constants say.
 constexpr double kBasePair = 5.42, kBaseSingle256 = 4.05, kBaseSingle128 = 3.4, kBaseSingle64 = 3.13;
 constexpr double kOutput = 0.223e-6;  // per output element
 // with few SMs busy; the loads of a full GPU take kBusy more (pairs 0.30 to 0.36 us, 128 columns 0.30 to 0.34)
@@ -706,7 +707,8 @@ struct SmallPlan {
 // (with the quantisation inside, four warps' work); or, if that is longer, streaming every tile's weights (rows of N
 // bytes that are no multiple of 128 straddle two lines each); and the exchange of the parts.  A quantiser in front costs
 // a launch and a dependency.  The constants are fitted to 54 sizes x 4 to 8 variants measured on B200 (1 <= M <= 256,
-// 1024 <= N <= 7168, 1024 <= K <= 7168): estimates are off by 8 %, and the variant they choose by 0.7 % from the fastest.
+// 1024 <= N <= 7168, 1024 <= K <= 7168; above 16 rows with tiles of 32 only, so tiles of 16 are not considered there):
+// estimates are off by 8 %, and the variant they choose by 0.7 % from the fastest.
 constexpr double kSmallBase = 2.9, kSmallPeriod16 = 0.23, kSmallPeriod32 = 0.24, kSmallQuant16 = 0.37, kSmallQuant32 = 0.79;
 constexpr double kSmallQuantShared = 1.45;  // two CTAs on an SM
 constexpr double kSmallBytesPerUs = 7.4e6, kSmallBytesPerUsRagged = 5.1e6, kSmallHidden = 0.73;

@@ -12,14 +12,14 @@
 //   C      bf16 or fp16, row-major [Mg, N]
 //
 // One CTA per 128 x BLOCK_N output tile (256, 128 or 64 columns), persistent over tiles, 320 threads:
-//   warps 0-3 epilogue: tcgen05.ld of the fp32 accumulator, convert, 16-byte global stores
+//   warps 0-3 epilogue: tcgen05.ld of the fp32 accumulator, convert, 32-byte global stores (whole sectors)
 //   warp 4    TMA producer: A and B tiles (128-byte swizzle) into a ring of shared-memory stages
 //   warp 5    MMA issuer: four tcgen05.mma.kind::mxf8f6f4.block_scale (K = 32 each) and one
 //             tcgen05.commit per stage, nothing else (see the scale loaders)
 //   warps 6-9 scale loaders: warp j serves every fourth K tile; plain global loads of the E8M0
 //             bytes (the next K tile's loads are in flight while the current one is stored),
 //             written to shared memory in the 32x16-byte atom layout tcgen05.cp expects, copied into
-//             the stage's scale set in tensor memory by lane 0 (tcgen05.cp), whose tcgen05.commit on the
+//             the stage's scale set in tensor memory by an elected lane (tcgen05.cp), whose tcgen05.commit on the
 //             stage's full barrier is the warp's arrival
 //
 // With FUSED_QUANT the CTA carries fourteen more warps (10-23): eight run the quantise producer (mx_quant.cuh)

@@ -13,18 +13,22 @@
 //   tmem_empty[a], overlap_free[a]  live in the leader; the epilogue warps of both CTAs arrive there
 //   atoms[b], sf_full[b]        live in the leader, sf_empty[b] in each CTA: see below
 //
-// Two rings.  The round trip of a stage (commit, empty, TMA, full, MMA) takes about 3000 cycles on a loaded GPU
-// against 512 cycles of MMA per K tile, so the operand ring is as deep as shared memory allows and carries
-// nothing but TMA.  The scale factors have a ring of their own that moves in groups of four K tiles: the scale-loader
-// warps load the E8M0 bytes one group ahead into registers, write the atoms, and the leader's lane 0 of every warp
-// copies one K tile's atoms of both CTAs into tensor memory; two groups are in flight.
+// Two rings.  The operand ring carries nothing but TMA and is as deep as shared memory allows.  The scale factors have a
+// ring of their own that moves in groups of four K tiles: the scale-loader warps load the E8M0 bytes one group ahead into
+// registers, write the atoms, and an elected lane of each of the leader's warps copies one K tile's atoms of both CTAs
+// into tensor memory; two groups are in flight.
 //
-// What bounds it: a K tile moves 32 KB into and 32 KB out of each SM's shared memory (500 of the 512 MMA cycles) and
-// 64 B per cycle and SM out of L2, so both are close to their limits when the tensor pipe is; long launches are held by
-// the power cap instead.  Pairs on 256 x 128 tiles (48 KB per 256 MMA cycles) were measured 1.4 to 1.6 times slower.
-// Measured (B200, 3 operand sets in turn, kernel alone): 1024 x 2304 x 7168 25.7 -> 21.2 us, 3001 x 2064 x 5120
-// 41.3 -> 33.3, 4096 x 3456 x 5120 66.5 -> 58.9, 8192 x 2304 x 7168 105 -> 99, 32768 x 3456 x 5120 450 -> 428 us
-// against one ring of five stages that also carried the scales, no split, and stores straight from registers.
+// What bounds it: about 600 SM cycles per K tile against 512 of MMA (slope over K, whole tiles; 8192 x 2304 and
+// 16384 x 3456 at 1.46 GHz under the power cap, 1024 x 2304 at 1.965 GHz: 601, 587, 601 cycles).  It is not the ring's
+// depth: five stages take 616, 580, 611, four 625, 601, 751.  Which of the rest it is has not been shown: a K tile moves
+// 32 KB into and 32 KB out of each SM's shared memory (500 cycles at 128 bytes), and 51 bytes per cycle and SM leave L2.
+// The cycles are the same under the power cap, which lowers the clock.  Pairs on 256 x 128 tiles (48 KB per 256 MMA
+// cycles) were measured 1.4 to 1.6 times slower.
+// Measured (B200, kernel alone, three operand sets in turn, 40 calls queued behind an idle GPU, so near the full clock; in
+// brackets a second without a pause, at 1.3 to 1.8 GHz), against one ring of five stages that also carried the scales, no split
+// behind whole tiles, and stores straight from registers: 1024 x 2304 x 7168 27.0 -> 21.5 us (26.7 -> 22.3), 3001 x 2064 x
+// 5120 42.3 -> 32.3 (44.6 -> 37.9), 4096 x 3456 x 5120 68.0 -> 57.2 (77.0 -> 67.8), 8192 x 2304 x 7168 103.5 -> 96.0
+// (122 -> 113), 32768 x 3456 x 5120 440 -> 414 (515 -> 488).
 //
 // Work units.  num_tiles = rounds * pairs + rem: the rem tiles that would leave pairs idle in a round of their own are
 // cut into ksplit parts along K, one (tile, part) per pair, and every pair takes `rounds` whole tiles.  The parts

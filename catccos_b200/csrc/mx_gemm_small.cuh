@@ -14,8 +14,9 @@
 //     operand ring (every CTA for itself): a fused call is one launch and has no quantised copy of X anywhere.
 //
 // Tiles of 64 and 128 rows were measured too: no faster than mx_gemm.cuh's tiles at the sizes that fill them.
-// Measured (B200, device time back to back): fused 16 x 4096 x 7168 13.7 -> 8.8 us, 1 x 2432 x 2432 10.3 -> 4.6,
-// 8 x 1024 x 7168 11.7 -> 6.2, 64 x 1024 x 1024 7.3 -> 5.4; the matmul alone 16 x 4096 x 7168 12.9 -> 8.6.
+// Measured (B200, 200 calls queued in the stream, against a quantise kernel and mx_gemm.cuh's tiles without programmatic
+// launches): fused 16 x 4096 x 7168 18.5 to 20.3 -> 8.6 us, 1 x 2432 x 2432 12.3 -> 4.5, 8 x 1024 x 7168 14.5 -> 6.2, 12 x
+// 3008 x 4992 18.5 -> 6.2, 64 x 1024 x 1024 13.8 -> 5.4; the matmul alone 16 x 4096 x 7168 14.4 -> 8.6.
 //
 // 320 threads: warps 0-3 X scales (or, QUANT, X codes and scales), then the epilogue; warp 4 TMA; warp 5 MMA issuer, which
 // also copies the stage's scale factors into tensor memory; warps 6-9 W scales, warp j every fourth K tile.

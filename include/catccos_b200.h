@@ -203,7 +203,8 @@ int catccos_b200_last_status(uint32_t out[4]);
  * The kernels choose their own tiling by size (CTA pairs, single CTAs, small tiles), with K cut in up to eight parts
  * when the tiles would leave SMs idle (the partial tiles meet in a per-rank scratch allocated when the rank is set up,
  * or in the shared memory of a cluster; because of it, and of the symmetric buffer's epochs, the operator
- * calls of one rank must not overlap on the GPU). */
+ * calls of one rank must not overlap on the GPU).  Calls at rankSize 1 may be captured in a CUDA graph, after one direct
+ * call of the same kind, and replayed any number of times; calls of several ranks may not, their epochs are counted by the host. */
 int catccos_b200_set_option(const char* key, int64_t value);
 
 /* Number of kernels this library has launched since it was loaded. */
