@@ -111,8 +111,8 @@ struct RankCtx {
     StatusBlock* status = nullptr;  // device memory
     uint8_t* fp4_bt = nullptr;  // the transposed copy of a packed E2M1 weight, made on every call that gets one
     size_t fp4_bt_bytes = 0;
-    // split-K scratch of this rank's GEMM launches: one fp32 partial tile and four flag words per SM, then the two words
-    // that count the split launches (the flags are epochs, split_epoch).  Launches of one rank are stream-ordered.
+    // split-K scratch of this rank's GEMM launches: one fp32 partial tile and four flag words per SM, then the 64-bit
+    // word that counts the split launches (the flags are epochs, split_epoch).  Launches of one rank are stream-ordered.
     float* splitk_ws = nullptr;
     uint32_t* splitk_flags = nullptr;
     // copy-engine allgather: one stream per peer (the transfers to the peers run side by side), an event that
@@ -932,7 +932,7 @@ int launch_gemm(RankCtx& rc, cudaStream_t st, const void* a, const void* b, Gemm
     if (ksplit > 1) {
         p.splitk_ws = rc.splitk_ws;
         p.splitk_flags = rc.splitk_flags;
-        p.splitk_state = rc.splitk_flags + (size_t)rc.num_sms * 4;
+        p.splitk_state = reinterpret_cast<unsigned long long*>(rc.splitk_flags + (size_t)rc.num_sms * 4);
     }
     if (use_pair) {
         CUtensorMap pa, pb, pc;

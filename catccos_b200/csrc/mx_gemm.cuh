@@ -107,7 +107,7 @@ struct GemmParams {
     uint32_t ksplit;
     float* splitk_ws;        // [tiles][ksplit][BLOCK_N / 32][128][32]
     uint32_t* splitk_flags;  // [tiles][ksplit][4] epoch words, one per epilogue warp
-    uint32_t* splitk_state;  // see split_epoch
+    unsigned long long* splitk_state;  // see split_epoch
 };
 
 template <uint32_t BLOCK_N>
@@ -477,21 +477,19 @@ constexpr uint32_t kSplitPieceBytes = 32u * 32u * 4u;           // 32 rows x 32 
 constexpr uint32_t kSplitRedBytes = 12u * kSplitPieceBytes;     // most pieces a warp takes in: two chunks from six parts
 
 // The epoch that a launch's flags carry, for one of `readers` warps (each of the launch calls this once, whatever becomes of
-// it later).  state[0] counts the split launches that have used this scratch, state[1] the warps of the present one that have
-// read it; the last one advances it for the next launch.  The count lives in device memory because a launch's parameters
-// stay the same when a CUDA graph replays it: with the epoch among them a second replay would take the first one's flags
-// for its own and add partial tiles that are not there yet.  Call it once the predecessor has finished (grid_dep_wait);
-// it is off the critical path, the accumulator takes longer.
-__device__ __forceinline__ uint32_t split_epoch(uint32_t* state, uint32_t readers, uint32_t lane)
+// it later).  The high half of the word counts the split launches that have used this scratch, the low half the warps of the
+// present one that have read it, in one atomic operation; the last one advances the count for the next launch.  The word
+// lives in device memory because a launch's parameters stay the same when a CUDA graph replays it: with the epoch among
+// them a second replay would take the first one's flags for its own and add partial tiles that are not there yet.  Call it
+// once the predecessor has finished (grid_dep_wait); it is off the critical path, the accumulator takes longer.
+__device__ __forceinline__ uint32_t split_epoch(unsigned long long* state, uint32_t readers, uint32_t lane)
 {
     uint32_t epoch = 0;
     if (lane == 0) {
-        epoch = ld_acquire_gpu(state) + 1u;
-        uint32_t before;
-        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(state + 1) : "memory");
-        if (before + 1u == readers) {
-            state[1] = 0u;
-            state[0] = epoch;
+        const unsigned long long before = atomicAdd(state, 1ull);
+        epoch = (uint32_t)(before >> 32) + 1u;
+        if ((uint32_t)before + 1u == readers) {
+            atomicExch(state, (unsigned long long)epoch << 32);
         }
     }
     return __shfl_sync(0xFFFFFFFFu, epoch, 0);
